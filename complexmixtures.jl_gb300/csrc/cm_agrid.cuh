@@ -49,6 +49,8 @@ constexpr int kAgridBuckets = 8;       // each list ordered by bucket of the ato
 constexpr int kAgridStage = 3072;      // stencil atoms staged in shared memory at a time (48 KB, dynamic)
 constexpr int kAgridRound = 4;         // stencil atoms each thread loads per staging round
 constexpr int kAgridBuildThreads = 256;
+constexpr int kAgridRecThreads = 32;   // k_agrid_records: a few records per SM,
+constexpr int kAgridRecLanes = 4;      // each on a group of lanes
 
 // The fine cells of a search cell: edge vectors and bounds, FP32.
 // Largest distance from p to a point of the fine cell centred at c: squared
@@ -456,29 +458,51 @@ __device__ __forceinline__ AgridCell agrid_cell(const Bufs &B, const FrameGeom &
 // by more than `band` holds no atom that can be the minimum, be within the
 // guard band of it or lower the reference row, and neither do the buckets
 // after it.
-__device__ __forceinline__ void agrid_query(const Bufs &B, const FrameGeom &G, const FrameScratch &F, int f, int packed,
+// GL lanes (gl = 0 .. GL - 1) split the list; each ends with its own entries' values.
+template <int GL>
+__device__ __forceinline__ void agrid_query(int gl, const Bufs &B, const FrameGeom &G, const FrameScratch &F, int f, int packed,
                                             float4 q, int b, bool isref, float band, Top2 &T, long long &evals) {
     const AgridCell c = agrid_cell(B, G, F, f, packed, q);
     const float4 *e = B.gent + (int64_t)f * B.gcap;
-    int i = c.st[0];
+    int i = c.st[0], next = c.st[1];
+    const int last = c.st[kAgridBuckets];
+    if (i >= last) return;
+    int k = 0;
 #pragma unroll 1
-    for (int k = 0; k < kAgridBuckets; ++k) {
+    for (;;) {
+        while (i >= next) {  // the bucket of entry i
+            ++k;
+            next = c.st[k + 1];
+        }
         const float thr = fmaxf(sqrtf(T.m1), isref ? sqrtf(T.r1) : 0.f) + band;
         if (fmaf(c.w, (float)k, c.lo) > thr) break;
-        const int end = c.st[k + 1];
-        evals += end - i;
-        for (; i < end; ++i) {
-            const float4 a = e[i];
-            const float ex = a.x - q.x, ey = a.y - q.y, ez = a.z - q.z;
-            const float d2 = fmaf(ez, ez, fmaf(ey, ey, ex * ex));
+        // four entries in flight: past the end the last one again, as infinity
+        float4 a[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a[j] = e[min(i + GL * j + gl, last - 1)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float ex = a[j].x - q.x, ey = a[j].y - q.y, ez = a[j].z - q.z;
+            float d2 = fmaf(ez, ez, fmaf(ey, ey, ex * ex));
+            if (GL > 1 || j > 0) d2 = i + GL * j + gl < last ? d2 : INFINITY;
             T.m2 = fminf(T.m2, fmaxf(T.m1, d2));
             const bool lt = d2 < T.m1;
-            T.p1 = lt ? __float_as_int(a.w) : T.p1;
+            T.p1 = lt ? __float_as_int(a[j].w) : T.p1;
             T.b1 = lt ? b : T.b1;
             T.m1 = fminf(T.m1, d2);
             if (isref) T.r1 = fminf(T.r1, d2);
         }
+        if (GL == 1) evals += min(4, last - i);
+        else evals += gl == 0 ? min(4 * GL, last - i) : 0;
+        i += 4 * GL;
+        if (i >= last) break;
     }
+}
+
+// The lanes of the calling lane's group of G.
+template <int G>
+__device__ __forceinline__ unsigned agrid_group_mask() {
+    return G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
 }
 
 // Exact scan of a slot's or molecule's sites over their lists: every list
@@ -489,8 +513,9 @@ __device__ __forceinline__ void agrid_query(const Bufs &B, const FrameGeom &G, c
 // 2 delta, so each such atom lies within (nearest distance + 3 delta) of its
 // site, which the list's margin covers, and the buckets past sqrt(thr) + band
 // hold none of them.
-__device__ __noinline__ void agrid_exact(const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F, int f,
-                                         ExactMol &X, const int *vc, const float4 *vq, float band, float thr_arg,
+template <int GL>
+__device__ __noinline__ void agrid_exact(int gl, const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F,
+                                         int f, ExactMol &X, const int *vc, const float4 *vq, float band, float thr_arg,
                                          float thr_r1, Best64 &Bst, double &rr1, long long &evals) {
     best_init(Bst);
     rr1 = INFINITY;
@@ -505,20 +530,27 @@ __device__ __noinline__ void agrid_exact(const DevSys &S, const Bufs &B, const F
         const float lim = sqrtf(thr) + band;
         double yb[3];
         bool have_y = false;
-        int i = c.st[0];
-        for (int k = 0; k < kAgridBuckets; ++k) {
-            if (fmaf(c.w, (float)k, c.lo) > lim) break;
-            const int end = c.st[k + 1];
-            for (; i < end; ++i) {
-                const float4 a = e[i];
-                const float ex = a.x - q.x, ey = a.y - q.y, ez = a.z - q.z;
+        const int i0 = c.st[0];
+        int last = i0;  // the end of the buckets that can hold such an atom
+        for (int k = 0; k < kAgridBuckets && fmaf(c.w, (float)k, c.lo) <= lim; ++k) last = c.st[k + 1];
+        for (int i = i0; i < last; i += 4 * GL) {
+            float4 a[4];
+            unsigned need = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) a[j] = e[min(i + GL * j + gl, last - 1)];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float ex = a[j].x - q.x, ey = a[j].y - q.y, ez = a[j].z - q.z;
                 const float d2f = fmaf(ez, ez, fmaf(ey, ey, ex * ex));
-                if (!(d2f <= thr_arg || (isref && d2f <= thr_r1))) continue;
+                if (i + GL * j + gl < last && (d2f <= thr_arg || (isref && d2f <= thr_r1))) need |= 1u << j;
+            }
+            for (; need; need &= need - 1) {
+                const int j = __ffs(need) - 1;
                 if (!have_y) {
                     exact_solvent_atom(B, G, X, b, yb);
                     have_y = true;
                 }
-                const int ai = __float_as_int(a.w);
+                const int ai = __float_as_int(j == 0 ? a[0].w : j == 1 ? a[1].w : j == 2 ? a[2].w : a[3].w);
                 double xa[3];
                 exact_solute_atom(B, X, ai, xa);
                 const double d2 = exact_d2(G, xa, yb);
@@ -529,6 +561,25 @@ __device__ __noinline__ void agrid_exact(const DevSys &S, const Bufs &B, const F
                 }
             }
         }
+    }
+    if (GL > 1) {
+        // the group's smallest d = sqrt(d2), among equal d the larger (a, b); every lane ends with it
+        double d = Bst.d2 <= S.cut2 ? best_d(Bst) : INFINITY;
+        const unsigned mask = agrid_group_mask<GL>();
+#pragma unroll
+        for (int o = GL / 2; o > 0; o >>= 1) {
+            const double od = __shfl_xor_sync(mask, d, o), od2 = __shfl_xor_sync(mask, Bst.d2, o);
+            const int oa = __shfl_xor_sync(mask, Bst.a, o), ob = __shfl_xor_sync(mask, Bst.b, o);
+            if (od < d || (od == d && (oa > Bst.a || (oa == Bst.a && ob > Bst.b)))) {
+                if (od < d) Bst.d2 = od2;
+                d = od;
+                Bst.a = oa;
+                Bst.b = ob;
+            }
+            rr1 = fmin(rr1, __shfl_xor_sync(mask, rr1, o));
+            evals += __shfl_xor_sync(mask, evals, o);
+        }
+        Bst.d = d <= 1e300 ? d : -1.0;
     }
 }
 
@@ -560,8 +611,11 @@ __device__ __forceinline__ int agrid_decide(const DevSys &S, const Guard &g, con
 // The record of a query inside the band (agrid_decide's 2), decided by
 // atoms_decide's rules with the exact scans over the sites' lists (agrid_exact)
 // instead of the stencil walk: v the solvent molecule (sample < 0) or the
-// slot of sample `sample`, whose placement is drawn again in FP64.
-__device__ __noinline__ DirRec agrid_record(const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F,
+// slot of sample `sample`, whose placement is drawn again in FP64.  The GL
+// lanes of a group share the scans and return the same record; the first one
+// counts the statistics.
+template <int GL>
+__device__ __noinline__ DirRec agrid_record(int gl, const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F,
                                             int f, int v, int sample, const int *vc, const float4 *vq, const Top2 &T,
                                             LocalStats &st) {
     const Guard &g = F.g;
@@ -587,12 +641,14 @@ __device__ __noinline__ DirRec agrid_record(const DevSys &S, const Bufs &B, cons
         Best64 Bst;
         double rr1;
         long long ev;
-        agrid_exact(S, B, G, F, f, X, vc, vq, band, r_sq_ru(d1 + g.two_delta), thr1, Bst, rr1, ev);
-        st.guard++;
-        st.guard_pairs += ev;
+        agrid_exact<GL>(gl, S, B, G, F, f, X, vc, vq, band, r_sq_ru(d1 + g.two_delta), thr1, Bst, rr1, ev);
+        if (gl == 0) {
+            st.guard++;
+            st.guard_pairs += ev;
+        }
         if (Bst.d2 <= S.cut2) {
             const double d = best_d(Bst);
-            st.maxerr = fmax(st.maxerr, fabs((double)d1 - d));
+            if (gl == 0) st.maxerr = fmax(st.maxerr, fabs((double)d1 - d));
             r.within = 1;
             r.i_local = Bst.a;
             r.j = vb + Bst.b;
@@ -611,9 +667,11 @@ __device__ __noinline__ DirRec agrid_record(const DevSys &S, const Bufs &B, cons
     if (bin < 0 || (S.usecutoff && d1 >= g.dbulk_lo && d1 <= g.dbulk_hi)) {
         d64 = sqrt(exact_pair_d2(B, G, X, T.p1, T.b1));
         bin = setbin0(d64, S.binstep);
-        st.guard++;
-        st.guard_pairs++;
-        st.maxerr = fmax(st.maxerr, fabs((double)d1 - d64));
+        if (gl == 0) {
+            st.guard++;
+            st.guard_pairs++;
+            st.maxerr = fmax(st.maxerr, fabs((double)d1 - d64));
+        }
     }
     r.within = 1;
     r.i_local = T.p1;
@@ -629,9 +687,11 @@ __device__ __noinline__ DirRec agrid_record(const DevSys &S, const Bufs &B, cons
             Best64 Bst;
             double rr1;
             long long ev;
-            agrid_exact(S, B, G, F, f, X, vc, vq, band, -1.f, r_sq_ru(sqrtf(T.r1) + g.two_delta), Bst, rr1, ev);
-            st.guard++;
-            st.guard_pairs += ev;
+            agrid_exact<GL>(gl, S, B, G, F, f, X, vc, vq, band, -1.f, r_sq_ru(sqrtf(T.r1) + g.two_delta), Bst, rr1, ev);
+            if (gl == 0) {
+                st.guard++;
+                st.guard_pairs += ev;
+            }
             if (rr1 <= S.cut2) {
                 r.ref = 1;
                 r.rbin = setbin0(sqrt(rr1), S.binstep);
@@ -639,6 +699,46 @@ __device__ __noinline__ DirRec agrid_record(const DevSys &S, const Bufs &B, cons
         }
     }
     return r;
+}
+
+// Top-2 of a molecule's or slot's sites over their lists (vc, vq: its sites'
+// cells and positions); false when no listed atom was met.
+template <int GL>
+__device__ __forceinline__ bool agrid_top2(int gl, const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F, int f,
+                                           const int *vc, const float4 *vq, Top2 &T, long long &ev) {
+    top2_init(T);
+    ev = 0;
+    const float band = F.g.two_delta + 1e-3f * (1.0f + (float)S.cut);
+    for (int b = 0; b < S.apv; ++b) agrid_query<GL>(gl, B, G, F, f, vc[b], vq[b], b, b == S.iref, band, T, ev);
+    if (GL > 1) {
+        // the group's top-2; every lane ends with it
+        const unsigned mask = agrid_group_mask<GL>();
+#pragma unroll
+        for (int o = GL / 2; o > 0; o >>= 1) {
+            const float m1 = __shfl_xor_sync(mask, T.m1, o), m2 = __shfl_xor_sync(mask, T.m2, o);
+            const int p1 = __shfl_xor_sync(mask, T.p1, o), b1 = __shfl_xor_sync(mask, T.b1, o);
+            T.m2 = fminf(fmaxf(T.m1, m1), fminf(T.m2, m2));
+            if (m1 < T.m1 || (m1 == T.m1 && (p1 < T.p1 || (p1 == T.p1 && b1 < T.b1)))) {
+                T.p1 = p1;
+                T.b1 = b1;
+            }
+            T.m1 = fminf(T.m1, m1);
+            T.r1 = fminf(T.r1, __shfl_xor_sync(mask, T.r1, o));
+        }
+    }
+    return ev != 0;
+}
+
+// A query inside the band: listed for k_agrid_records (counters[9] entries in
+// adefer), false when there is no room for it.  About one query in a hundred
+// is inside the band, and decided on the spot it left its warp on one lane of
+// dependent FP64 operations in a third of the warp's rounds.
+__device__ __forceinline__ bool agrid_defer(const Bufs &B, int entry) {
+    if (B.adefer_cap == 0) return false;
+    const int at = atomicAdd(B.counters + 9, 1);
+    if (at >= B.adefer_cap) return false;
+    B.adefer[at] = entry;
+    return true;
 }
 
 // Real pass of a single solute molecule, one thread per (frame, solvent
@@ -651,10 +751,21 @@ __device__ __forceinline__ void k_agrid_real_body(const uint3 blockIdx, const di
     __syncthreads();
     const SHist h = shist_bind(S, hbase);
     LocalStats st;
-    const int apv = S.apv, iref = S.iref;
+    const int apv = S.apv;
     const int64_t n = (int64_t)B.nf * S.mv;
-    auto one_molecule = [&](int64_t it) {
-        const int f = (int)(it / S.mv), v = (int)(it - (int64_t)f * S.mv);
+    auto put = [&](const DirRec &r, int f, int v) {
+        st.molpairs++;
+        if (r.within) {
+            apply_hit(S, h, false, r.bin, r.i_local, r.j, r.ref, r.rbin);
+            st.hits++;
+            if (B.slot) {
+                const int sl = B.slot[(int64_t)f * B.ms];
+                if (sl >= 0) B.flags[((int64_t)f * B.ndist + sl) * S.mv + v] = flag_code(r);
+            }
+        }
+    };
+    auto one_molecule = [&](int it) {
+        const int f = it / S.mv, v = it - f * S.mv;
         const FrameScratch &F = B.FS[f];
         const FrameGeom &G = B.G[f];
         const int *vc = B.avcell + (int64_t)f * B.Nv + (int64_t)v * apv;
@@ -668,33 +779,26 @@ __device__ __forceinline__ void k_agrid_real_body(const uint3 blockIdx, const di
         }
         const float4 *vq = B.avq32 + (int64_t)f * B.Nv + (int64_t)v * apv;
         Top2 T;
-        top2_init(T);
-        long long ev = 0;
-        const float band = F.g.two_delta + 1e-3f * (1.0f + (float)S.cut);
-        for (int b = 0; b < apv; ++b) agrid_query(B, G, F, f, vc[b], vq[b], b, b == iref, band, T, ev);
-        if (ev == 0) return;
-        st.atompairs += (unsigned long long)ev;
+        long long ev;
+        if (!agrid_top2<1>(0, S, B, G, F, f, vc, vq, T, ev)) return;
         DirRec r;
-        if (agrid_decide(S, F.g, T, (int64_t)v * apv, r) == 2) r = agrid_record(S, B, G, F, f, v, -1, vc, vq, T, st);
-        st.molpairs++;
-        if (r.within) {
-            apply_hit(S, h, false, r.bin, r.i_local, r.j, r.ref, r.rbin);
-            st.hits++;
-            if (B.slot) {
-                const int sl = B.slot[(int64_t)f * B.ms];
-                if (sl >= 0) B.flags[((int64_t)f * B.ndist + sl) * S.mv + v] = flag_code(r);
-            }
+        if (agrid_decide(S, F.g, T, (int64_t)v * apv, r) == 2) {
+            if (agrid_defer(B, it)) return;
+            r = agrid_record<1>(0, S, B, G, F, f, v, -1, vc, vq, T, st);
         }
+        st.atompairs += (unsigned long long)ev;
+        put(r, f, v);
     };
     // warps take 32 molecules at a time from counters[6] (zeroed with the
-    // chunk's counters), as k_agrid_random takes its slots
+    // chunk's counters), as k_agrid_random takes its slots; nf mv < 2^31 (the
+    // fallback's queue holds every item of the chunk)
     const int lane = threadIdx.x & 31;
     for (;;) {
         long long at = 0;
         if (lane == 0) at = (long long)atomicAdd((unsigned long long *)(B.counters + 6), 32ull);
         at = __shfl_sync(0xffffffffu, at, 0);
         if (at >= n) break;
-        if (at + lane < n) one_molecule(at + lane);
+        if (at + lane < n) one_molecule((int)at + lane);
         __syncwarp();
     }
     stats_flush(S, st, false);
@@ -707,12 +811,20 @@ __global__ void __launch_bounds__(256, 4) k_agrid_real(DevSys S, Bufs B) {
     k_agrid_real_body(blockIdx, gridDim, S, B);
 }
 
-// Random insertion of a single solute molecule, third pass: one thread per
-// slot of the list k_slot_filter made, after k_atoms_place has placed them
-// into the placement buffers; persistent grid.  In a frame with a grid the
-// slot's sites are queried and the record is decided at once (agrid_record
-// inside the band); k_atoms_place has queued the near slots of the other
-// frames for k_atoms_eval.
+// Random insertion of a single solute molecule, last pass: one thread per
+// slot that k_atoms_place placed, in the order of the slots' fine cells;
+// persistent grid.  The slot's sites are queried and the record is decided
+// (agrid_record inside the band).  k_atoms_place has
+// queued the near slots of the frames without a grid for k_atoms_eval.
+//
+// The loads of the lists bound it: a 16-byte load of 32 lanes from 32 lists
+// takes about 11 cycles of the SM's L1 port, four times the arithmetic on it.
+// Slots of a fine cell read the same lists, so in fine-cell order a warp's
+// lanes share their lines and finish their lists together, and four entries
+// per lane in flight then pay.  On a 43,000-atom system (50 frames, 10
+// samples) the queries went from 2,850 to 1,980 us sorted and four wide, to
+// 1,250 us (978 here, 274 in k_agrid_records) with the records inside the
+// band apart and 4 M slots a launch instead of 32 samples.
 __device__ __forceinline__ void k_agrid_random_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B, int sample0, int ny) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned int *hbase = (unsigned int *)smem_raw;
@@ -720,44 +832,43 @@ __device__ __forceinline__ void k_agrid_random_body(const uint3 blockIdx, const 
     __syncthreads();
     const SHist h = shist_bind(S, hbase);
     LocalStats st;
-    const int apv = S.apv, iref = S.iref;
+    const int apv = S.apv;
     (void)ny;
-    const int n = min(B.counters[5], B.aslot_cap);
-    auto one_slot = [&](int it) {
-        const int e = B.aslot[it];
-        const int y = e / S.mv, k = e - y * S.mv;
-        const int f = B.samples[sample0 + y].pad;
-        const FrameScratch &F = B.FS[f];
-        if (!F.agrid) return;
-        const FrameGeom &G = B.G[f];
-        const int64_t base = (int64_t)y * B.Nv + (int64_t)k * apv;
-        Top2 T;
-        top2_init(T);
-        long long ev = 0;
-        const float band = F.g.two_delta + 1e-3f * (1.0f + (float)S.cut);
-        for (int b = 0; b < apv; ++b)
-            agrid_query(B, G, F, f, B.pcell[base + b], B.pq32[base + b], b, b == iref, band, T, ev);
-        if (ev == 0) return;
-        st.atompairs += (unsigned long long)ev;
-        DirRec r;
-        if (agrid_decide(S, F.g, T, (int64_t)k * apv, r) == 2)
-            r = agrid_record(S, B, G, F, f, k, sample0 + y, B.pcell + base, B.pq32 + base, T, st);
+    const int n = min(B.counters[8], B.aslot_cap);
+    auto put = [&](const DirRec &r) {
         st.molpairs++;
         if (r.within) {
             apply_hit(S, h, true, r.bin, r.i_local, r.j, r.ref, r.rbin);
             st.hits++;
         }
     };
-    // warps take 32 listed slots at a time from counters[6] (zeroed with the
-    // slot list): the slots' costs vary with their lists, and a fixed share per
-    // thread left the CTAs' warps waiting for their slowest one
+    auto one_slot = [&](int e) {
+        const int y = e / S.mv, k = e - y * S.mv;
+        const int f = B.samples[sample0 + y].pad;
+        const FrameScratch &F = B.FS[f];
+        const FrameGeom &G = B.G[f];
+        const int64_t base = (int64_t)y * B.Nv + (int64_t)k * apv;
+        Top2 T;
+        long long ev;
+        if (!agrid_top2<1>(0, S, B, G, F, f, B.pcell + base, B.pq32 + base, T, ev)) return;
+        DirRec r;
+        if (agrid_decide(S, F.g, T, (int64_t)k * apv, r) == 2) {
+            if (agrid_defer(B, e)) return;
+            r = agrid_record<1>(0, S, B, G, F, f, k, sample0 + y, B.pcell + base, B.pq32 + base, T, st);
+        }
+        st.atompairs += (unsigned long long)ev;
+        put(r);
+    };
+    // warps take 32 slots at a time from counters[6] (zeroed with the slot
+    // list): a fixed share per thread left the CTAs' warps waiting for their
+    // slowest one
     const int lane = threadIdx.x & 31;
     for (;;) {
         int at = 0;
         if (lane == 0) at = atomicAdd(B.counters + 6, 32);
         at = __shfl_sync(0xffffffffu, at, 0);
         if (at >= n) break;
-        if (at + lane < n) one_slot(at + lane);
+        if (at + lane < n) one_slot(B.sslot[at + lane]);
         __syncwarp();
     }
     stats_flush(S, st, true);
@@ -767,6 +878,58 @@ __device__ __forceinline__ void k_agrid_random_body(const uint3 blockIdx, const 
 
 __global__ void __launch_bounds__(256, 4) k_agrid_random(DevSys S, Bufs B, int sample0, int ny) {
     k_agrid_random_body(blockIdx, gridDim, S, B, sample0, ny);
+}
+
+// The listed queries inside the band, a group of lanes each: queried again and
+// decided by agrid_record.  RANDOM: entries y mv + slot of the piece from
+// sample sample0 on; else entries frame mv + molecule.  Its time is the
+// latency of one record's FP64 chain; the list holds a few per SM, so they run
+// side by side.
+template <bool RANDOM>
+__device__ __forceinline__ void k_agrid_records_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B, int sample0) {
+    const int n = min(B.counters[9], B.adefer_cap);
+    if ((int64_t)blockIdx.x * (blockDim.x / kAgridRecLanes) >= n) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned int *hbase = (unsigned int *)smem_raw;
+    shist_zero(S, hbase);
+    __syncthreads();
+    const SHist h = shist_bind(S, hbase);
+    LocalStats st;
+    const int gl = threadIdx.x % kAgridRecLanes;
+    const int per = blockDim.x / kAgridRecLanes;
+    for (int it = blockIdx.x * per + threadIdx.x / kAgridRecLanes; it < n; it += gridDim.x * per) {
+        const int e = B.adefer[it];
+        const int row = e / S.mv, v = e - row * S.mv;
+        const int f = RANDOM ? B.samples[sample0 + row].pad : row;
+        const FrameScratch &F = B.FS[f];
+        const FrameGeom &G = B.G[f];
+        const int64_t base = (int64_t)row * B.Nv + (int64_t)v * S.apv;
+        const int *vc = (RANDOM ? B.pcell : B.avcell) + base;
+        const float4 *vq = (RANDOM ? B.pq32 : B.avq32) + base;
+        Top2 T;
+        long long ev;
+        agrid_top2<kAgridRecLanes>(gl, S, B, G, F, f, vc, vq, T, ev);
+        const DirRec r = agrid_record<kAgridRecLanes>(gl, S, B, G, F, f, v, RANDOM ? sample0 + row : -1, vc, vq, T, st);
+        if (gl != 0) continue;
+        st.molpairs++;
+        st.atompairs += (unsigned long long)ev;
+        if (r.within) {
+            apply_hit(S, h, RANDOM, r.bin, r.i_local, r.j, r.ref, r.rbin);
+            st.hits++;
+            if (!RANDOM && B.slot) {
+                const int sl = B.slot[(int64_t)f * B.ms];
+                if (sl >= 0) B.flags[((int64_t)f * B.ndist + sl) * S.mv + v] = flag_code(r);
+            }
+        }
+    }
+    stats_flush(S, st, RANDOM);
+    __syncthreads();
+    shist_flush(S, h, RANDOM);
+}
+
+template <bool RANDOM>
+__global__ void __launch_bounds__(kAgridRecThreads) k_agrid_records(DevSys S, Bufs B, int sample0) {
+    k_agrid_records_body<RANDOM>(blockIdx, gridDim, S, B, sample0);
 }
 
 }  // namespace cmk

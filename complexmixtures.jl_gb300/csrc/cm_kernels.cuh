@@ -397,7 +397,8 @@ struct Bufs {
     int4 *eq;                       // edge queue: 3 int4 per entry (s, v, code, frame), (a | b << 8, rb1, rb2, bin), (d32 bits)
     int eq_cap;
     int *counters;                  // [0] guard queue, [1] random queue, [2] ATOMS queue, [3] edge queue,
-                                    // [4] the chunk's real pass is redone without queues (k_queue_check)
+                                    // [4] the chunk's real pass is redone without queues (k_queue_check),
+                                    // [5] slot list, [6..7] work claims, [8] sorted slots, [9] deferred queries
     // ATOMS
     int *akey;                      // [nf][Ns]
     float4 *atq32, *asq32;
@@ -418,6 +419,13 @@ struct Bufs {
     int aq_cap;
     int *aslot;                     // random-insertion slots that can reach the solute (y * mv + slot); count in counters[5]
     int aslot_cap;
+    // candidate grid: the listed slots in order of the fine cell of their
+    // centre (k_slot_filter counts, k_slot_scan, k_atoms_place scatters)
+    int2 *skey;                     // [aslot_cap]: fine cell of the slot's frame (-1: no grid), rank among that cell's slots
+    int *sslot;                     // [aslot_cap]: slots in fine-cell order; count in counters[8]
+    int *adefer;                    // queries inside the band (the slot list's memory, done with by then); count in counters[9]
+    int adefer_cap;
+    int *scount;                    // [nf][gfs]: slots of each fine cell, then the first position of each in sslot
     // ATOMS candidate grid (one solute molecule, FP32 search): each search
     // cell split into agk^3 fine cells, each with the list of solute atoms
     // that can be the closest (or within the guard band of it) to a point of
@@ -1922,8 +1930,11 @@ __device__ __forceinline__ bool placed_store32(const Bufs &B, const FrameScratch
 // (placed_maybe_near on a box widened to cover the FP32 rounding of the
 // centre's cell) can hold no pair within the cutoff and is dropped; the others
 // go to the slot list (y * mv + slot, count in counters[5]), so that the FP64
-// placement runs on full warps.
-__device__ __forceinline__ void k_slot_filter_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B, int sample0) {
+// placement runs on full warps.  With the candidate grid a listed slot also
+// counts itself at the fine cell of its centre (frames from frame0 on), for
+// the queries' order (k_slot_scan).
+__device__ __forceinline__ void k_slot_filter_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B, int sample0,
+                                                   int frame0) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= S.mv) return;
     const int y = blockIdx.y;
@@ -1938,11 +1949,13 @@ __device__ __forceinline__ void k_slot_filter_body(const uint3 blockIdx, const d
     const unsigned char *nm = B.anear + (int64_t)f * B.as + (int64_t)sm.s * G.ncell;
     const float rc = B.rc[(int64_t)f * B.mv + jmol];
     int lo[3], hi[3];
+    float gc[3];
     bool maybe = false;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         // U n in grid units from the grid's origin (FP32 of the exact product fk n 2^-53)
         const float g = cmfeed::u128_to_f32(0, fk[q] * (uint64_t)G.n[q]) * 0x1.0p-53f;
+        gc[q] = g;
         const float reach = rc / F.cw[q] + 2e-3f;
         lo[q] = (int)floorf(g - reach);
         hi[q] = (int)floorf(g + reach);
@@ -1954,21 +1967,87 @@ __device__ __forceinline__ void k_slot_filter_body(const uint3 blockIdx, const d
                 maybe = nm[(wrap_cell(dz, G.n[2]) * G.n[1] + wrap_cell(dy, G.n[1])) * G.n[0] + wrap_cell(dx, G.n[0])] != 0;
     if (!maybe) return;
     const int at = atomicAdd(B.counters + 5, 1);
-    if (at < B.aslot_cap) B.aslot[at] = y * S.mv + k;
-    else raise_err(S, ERR_QUEUE);
+    if (at >= B.aslot_cap) {
+        raise_err(S, ERR_QUEUE);
+        return;
+    }
+    B.aslot[at] = y * S.mv + k;
+    if (B.agk > 0) {
+        int2 kr = make_int2(-1, 0);
+        if (F.agrid) {
+            int c[3], u[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                c[q] = min(max((int)gc[q], 0), G.n[q] - 1);
+                u[q] = min(max((int)((gc[q] - (float)c[q]) * (float)B.agk), 0), B.agk - 1);
+            }
+            kr.x = cell_linear(G, c[0], c[1], c[2]) * (B.agk * B.agk * B.agk) + (u[2] * B.agk + u[1]) * B.agk + u[0];
+            kr.y = atomicAdd(B.scount + (int64_t)(f - frame0) * B.gfs + kr.x, 1);
+        }
+        B.skey[at] = kr;
+    }
 }
 
-__global__ void k_slot_filter(DevSys S, Bufs B, int sample0) {
-    k_slot_filter_body(blockIdx, gridDim, S, B, sample0);
+__global__ void k_slot_filter(DevSys S, Bufs B, int sample0, int frame0) {
+    k_slot_filter_body(blockIdx, gridDim, S, B, sample0, frame0);
+}
+
+// First position of each fine cell's slots in the sorted slot list: an
+// exclusive scan of a frame's counts by one CTA of 1024 threads (frame frame0
+// + block), from a base that the frame takes off counters[8] (the order of
+// the frames in the list does not matter).  A few microseconds; the sorted
+// order is what it buys (k_agrid_random).
+__device__ __forceinline__ void k_slot_scan_body(const uint3 blockIdx, const dim3 gridDim, const Bufs &B, int frame0) {
+    __shared__ int wsum[32];
+    __shared__ int s_base;
+    const int f = frame0 + blockIdx.x;
+    if (!B.FS[f].agrid) return;  // no slot of the frame was counted
+    int *c = B.scount + (int64_t)blockIdx.x * B.gfs;
+    const int n = B.G[f].ncell * B.agk * B.agk * B.agk;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int per = (n + 1023) / 1024;
+    const int lo = min(n, t * per), hi = min(n, lo + per);
+    int local = 0;
+    for (int i = lo; i < hi; ++i) local += c[i];
+    int incl = local;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+        int s = wsum[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += y;
+        }
+        wsum[lane] = s;
+        if (lane == 31) s_base = atomicAdd(B.counters + 8, s);
+    }
+    __syncthreads();
+    int at = s_base + incl - local + (w > 0 ? wsum[w - 1] : 0);
+    for (int i = lo; i < hi; ++i) {
+        const int v = c[i];
+        c[i] = at;
+        at += v;
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_slot_scan(Bufs B, int frame0) {
+    k_slot_scan_body(blockIdx, gridDim, B, frame0);
 }
 
 // Second pass: the listed slots placed (FP64, the same draws, on full warps),
 // written to the placement buffers, and -- in frames without a candidate grid
 // -- queued for k_atoms_eval when one of their atoms lies in a near cell of
 // the solute molecule: (slot, placed sample, sample, 1).  The grid's frames
-// are queried by k_agrid_random, which reads these positions.  Persistent
-// grid over the list.
-__device__ __forceinline__ void k_atoms_place_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B, int sample0) {
+// are queried by k_agrid_random, which reads these positions in the sorted
+// order written here.  Persistent grid over the list.
+__device__ __forceinline__ void k_atoms_place_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B, int sample0,
+                                                   int frame0) {
     const int n = min(B.counters[5], B.aslot_cap);
     for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n; it += gridDim.x * blockDim.x) {
         const int e = B.aslot[it];
@@ -2005,7 +2084,11 @@ __device__ __forceinline__ void k_atoms_place_body(const uint3 blockIdx, const d
             placed_store(S, B, G, F, B.off64 + (int64_t)f * kOffEntries, A, B.u64 + (int64_t)f * B.Nv + (int64_t)P.jmol * S.apv,
                          c0, q0, P.fc, base);
         }
-        if (F.agrid) continue;
+        if (F.agrid) {
+            const int2 kr = B.skey[it];
+            B.sslot[B.scount[(int64_t)(f - frame0) * B.gfs + kr.x] + kr.y] = e;
+            continue;
+        }
         bool near = false;
         for (int b = 0; b < S.apv && !near; ++b) {
             const int pc = B.pcell[base + b];
@@ -2019,8 +2102,8 @@ __device__ __forceinline__ void k_atoms_place_body(const uint3 blockIdx, const d
     }
 }
 
-__global__ void k_atoms_place(DevSys S, Bufs B, int sample0) {
-    k_atoms_place_body(blockIdx, gridDim, S, B, sample0);
+__global__ void k_atoms_place(DevSys S, Bufs B, int sample0, int frame0) {
+    k_atoms_place_body(blockIdx, gridDim, S, B, sample0, frame0);
 }
 
 // DCD decode (src/trajectory_formats/NamdDCD.jl:141-169): a frame of the file

@@ -25,7 +25,8 @@ struct __align__(16) MArgs {
     Bufs B;
     const void *p;   // coordinates (prep), bulk table (k_bulk)
     int64_t i0, i1;  // coordinate stride (prep); item range (k_atoms_filter)
-    int a0, a1;      // iref, centroids (prep solvent); pairs (frame consts); atoms_layout (scan); sample0, ny (random)
+    int a0, a1;      // iref, centroids (prep solvent); pairs (frame consts); atoms_layout (scan); sample0, ny (random);
+                     // sample0, frame0 (slot filter, place); frame0 (slot scan)
 };
 
 struct MTask {
@@ -47,9 +48,12 @@ enum MKid : int {
     MK_AGRID_BUILD,
     MK_AGRID_REAL,
     MK_AGRID_RANDOM,
+    MK_AGRID_REC_REAL,
+    MK_AGRID_REC_RANDOM,
     MK_ATOMS_FILTER,
     MK_ATOMS_PLACE,
     MK_SLOT_FILTER,
+    MK_SLOT_SCAN,
     MK_BULK,
     MK_EVAL_REAL_CELL,
     MK_EVAL_RANDOM_CELL,
@@ -69,9 +73,10 @@ __host__ __device__ constexpr int mk_threads(int kid) {
          : (kid == MK_PREP_SOLVENT_F32 || kid == MK_PREP_SOLVENT_F64) ? 128
          : (kid == MK_PREP_SOLUTE_F32 || kid == MK_PREP_SOLUTE_F64) ? 256
          : kid == MK_FRAME_CONSTS ? 128
-         : kid == MK_SCAN ? 1024
+         : (kid == MK_SCAN || kid == MK_SLOT_SCAN) ? 1024
          : (kid == MK_SCATTER_ATOMS || kid == MK_ATOMS_NEAR) ? 256
          : kid == MK_AGRID_BUILD ? kAgridBuildThreads
+         : (kid == MK_AGRID_REC_REAL || kid == MK_AGRID_REC_RANDOM) ? kAgridRecThreads
          : (kid == MK_AGRID_REAL || kid == MK_AGRID_RANDOM || kid == MK_ATOMS_FILTER) ? 256
          : (kid == MK_ATOMS_PLACE || kid == MK_SLOT_FILTER) ? 128
          : kid == MK_BULK ? 1024
@@ -94,9 +99,12 @@ __device__ __forceinline__ void mk_body(const uint3 vb, const dim3 vg, const MAr
     else if constexpr (KID == MK_AGRID_BUILD) k_agrid_build_body(vb, vg, a.S, a.B);
     else if constexpr (KID == MK_AGRID_REAL) k_agrid_real_body(vb, vg, a.S, a.B);
     else if constexpr (KID == MK_AGRID_RANDOM) k_agrid_random_body(vb, vg, a.S, a.B, a.a0, a.a1);
+    else if constexpr (KID == MK_AGRID_REC_REAL) k_agrid_records_body<false>(vb, vg, a.S, a.B, 0);
+    else if constexpr (KID == MK_AGRID_REC_RANDOM) k_agrid_records_body<true>(vb, vg, a.S, a.B, a.a0);
     else if constexpr (KID == MK_ATOMS_FILTER) k_atoms_filter_body(vb, vg, a.S, a.B, a.i0, a.i1);
-    else if constexpr (KID == MK_ATOMS_PLACE) k_atoms_place_body(vb, vg, a.S, a.B, a.a0);
-    else if constexpr (KID == MK_SLOT_FILTER) k_slot_filter_body(vb, vg, a.S, a.B, a.a0);
+    else if constexpr (KID == MK_ATOMS_PLACE) k_atoms_place_body(vb, vg, a.S, a.B, a.a0, a.a1);
+    else if constexpr (KID == MK_SLOT_FILTER) k_slot_filter_body(vb, vg, a.S, a.B, a.a0, a.a1);
+    else if constexpr (KID == MK_SLOT_SCAN) k_slot_scan_body(vb, vg, a.B, a.a0);
     else if constexpr (KID == MK_BULK) k_bulk_body(vb, vg, a.S, a.B, (const int4 *)a.p);
     else if constexpr (KID == MK_EVAL_REAL_CELL) k_atoms_eval_body<true, false, kSchedCell>(vb, vg, a.S, a.B);
     else if constexpr (KID == MK_EVAL_RANDOM_CELL) k_atoms_eval_body<true, true, kSchedCell>(vb, vg, a.S, a.B);

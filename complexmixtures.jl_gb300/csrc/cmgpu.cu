@@ -165,7 +165,21 @@ BlockCache &blocks() {
     return *c;
 }
 
-constexpr int kChunkSamples = 32;  // random samples placed per launch in the ATOMS regime
+constexpr int kCounters = 12;  // ints of Bufs::counters
+
+// Random samples placed per launch in the ATOMS layout.  FP64, or under an HBM
+// budget: 32 samples' worth of FP64 slots (52 bytes a site and 20 more); FP32
+// slots are smaller (20 a site and 32 more), so 44 to 77 samples fit the same
+// memory.  FP32 without a budget: up to kPieceSlots slots.  A piece's launches
+// end on their slowest warps and on the latency of its few exact records, so
+// fewer and larger pieces are faster.
+constexpr int64_t kPieceSlots = 1 << 22;
+int chunk_samples(const cm_system_desc &d) {
+    if (d.precision != CM_PRECISION_FP32_GUARD) return 32;
+    const int64_t apv = d.solvent_natomspermol;
+    const int64_t fit = 32 * (52 * apv + 20) / (20 * apv + 32);
+    return (int)(d.hbm_budget_bytes > 0 ? fit : std::max(fit, kPieceSlots / d.solvent_nmols));
+}
 
 }  // namespace
 
@@ -208,7 +222,7 @@ struct cm_handle {
     DevBuf g_soff, g_sidx, g_voff, g_vidx;
     // ATOMS
     DevBuf akey, atq32, atq64, asq32, asq64, acount, astart, afill, avcell, avq32, avq64, u64, u32, rc, pcell, pq32, pq64,
-        anear, aq, aslot;
+        anear, aq, aslot, skey, sslot, scount;
     int aq_cap = 0;
     int aslot_cap = 0;     // random-insertion slot list (slots of one placement piece)
     int atoms_ctas = 0;    // resident CTAs per SM of k_atoms_eval
@@ -667,6 +681,10 @@ void kernel_smem_limits(int device) {
     raise((const void *)k_agrid_real);
     raise((const void *)k_agrid_random);
     raise((const void *)k_agrid_build);
+    raise((const void *)k_agrid_records<false>);
+    raise((const void *)k_agrid_records<true>);
+    raise((const void *)k_multi<MK_AGRID_REC_REAL>);
+    raise((const void *)k_multi<MK_AGRID_REC_RANDOM>);
     raise((const void *)k_multi<MK_AGRID_BUILD>);
     raise((const void *)k_multi<MK_AGRID_REAL>);
     raise((const void *)k_multi<MK_AGRID_RANDOM>);
@@ -739,6 +757,7 @@ void ensure_cells(cm_handle *h, int64_t ncell) {
             dev_alloc(h, h->gstart, (size_t)h->fc * ncell * k3 * (kAgridBuckets + 1) * 4);
             dev_alloc(h, h->gedge, (size_t)h->fc * ncell * k3 * sizeof(float2));
             dev_alloc(h, h->gpool, (size_t)h->fc * 4);
+            if (h->mddf) dev_alloc(h, h->scount, (size_t)h->fc * ncell * k3 * 4);
         }
     }
 }
@@ -798,7 +817,7 @@ void plan(cm_handle *h, const cm_frames *f) {
     dev_alloc(h, h->fscratch, sizeof(FrameScratch) * fc);
     dev_alloc(h, h->off64, sizeof(d4) * cmgeom::kOffEntries * fc);
     dev_alloc(h, h->off32, sizeof(float4) * cmgeom::kOffEntries * fc);
-    dev_alloc(h, h->counters, 8 * sizeof(int));
+    dev_alloc(h, h->counters, kCounters * sizeof(int));
     if (h->mddf) {
         const int nd = h->ndist_max;
         dev_alloc(h, h->slot, (size_t)fc * ms * 4);
@@ -851,14 +870,16 @@ void plan(cm_handle *h, const cm_frames *f) {
             dev_alloc(h, h->u32, fc * h->Nv * 16);
             dev_alloc(h, h->rc, fc * mv * 4);
             // the work queue holds every slot of the samples placed in one launch
-            const int64_t want = std::min<int64_t>((int64_t)kChunkSamples * mv, std::max<int64_t>(1 << 22, mv));
-            h->atoms_piece = (int)std::max<int64_t>(1, std::min<int64_t>(kChunkSamples, want / mv));
+            const int64_t cs = chunk_samples(d);
+            const int64_t want = std::min<int64_t>(cs * mv, std::max<int64_t>(1 << 22, mv));
+            h->atoms_piece = (int)std::max<int64_t>(1, std::min<int64_t>(cs, want / mv));
             const int chunk = std::min(h->atoms_piece, std::max(1, fc * d.n_random_samples));
             dev_alloc(h, h->pcell, (size_t)chunk * h->Nv * 4);
             h->aslot_cap = (int)std::min<int64_t>((int64_t)chunk * mv, (int64_t)INT32_MAX);
             dev_alloc(h, h->aslot, (size_t)h->aslot_cap * 4);
             dev_alloc(h, h->pq32, (size_t)chunk * h->Nv * 16);
-            dev_alloc(h, h->pq64, (size_t)chunk * h->Nv * 32);
+            // the FP32 search and its exact scans do not read the FP64 positions
+            if (d.precision != CM_PRECISION_FP32_GUARD) dev_alloc(h, h->pq64, (size_t)chunk * h->Nv * 32);
         }
     }
     if (h->regime == CM_REGIME_ATOMS) {
@@ -905,6 +926,10 @@ void plan(cm_handle *h, const cm_frames *f) {
                 h->agk = K;
                 h->gcap = gcap;
                 dev_alloc(h, h->gent, (size_t)bytes);
+                if (h->mddf) {
+                    dev_alloc(h, h->skey, (size_t)h->aslot_cap * 8);
+                    dev_alloc(h, h->sslot, (size_t)h->aslot_cap * 4);
+                }
             }
         }
         if (h->agk > 0) {
@@ -1076,6 +1101,11 @@ Bufs chunk_bufs(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample 
             B.gpool = P<int>(h->gpool);
             B.gedge = P<float2>(h->gedge);
             B.gent = P<float4>(h->gent);
+            B.skey = P<int2>(h->skey);
+            B.sslot = P<int>(h->sslot);
+            B.adefer = P<int>(h->aslot);
+            B.adefer_cap = h->mddf ? h->aslot_cap : 0;
+            B.scount = P<int>(h->scount);
         }
         if (h->mddf) {
             B.u64 = P<d4>(h->u64);
@@ -1109,9 +1139,12 @@ void launch_one(int kid, dim3 g, size_t smem, cudaStream_t st, const MArgs &a) {
     case MK_AGRID_BUILD: k_agrid_build<<<g, t, smem, st>>>(a.S, a.B); break;
     case MK_AGRID_REAL: k_agrid_real<<<g, t, smem, st>>>(a.S, a.B); break;
     case MK_AGRID_RANDOM: k_agrid_random<<<g, t, smem, st>>>(a.S, a.B, a.a0, a.a1); break;
+    case MK_AGRID_REC_REAL: k_agrid_records<false><<<g, t, smem, st>>>(a.S, a.B, 0); break;
+    case MK_AGRID_REC_RANDOM: k_agrid_records<true><<<g, t, smem, st>>>(a.S, a.B, a.a0); break;
     case MK_ATOMS_FILTER: k_atoms_filter<<<g, t, smem, st>>>(a.S, a.B, a.i0, a.i1); break;
-    case MK_ATOMS_PLACE: k_atoms_place<<<g, t, smem, st>>>(a.S, a.B, a.a0); break;
-    case MK_SLOT_FILTER: k_slot_filter<<<g, t, smem, st>>>(a.S, a.B, a.a0); break;
+    case MK_ATOMS_PLACE: k_atoms_place<<<g, t, smem, st>>>(a.S, a.B, a.a0, a.a1); break;
+    case MK_SLOT_FILTER: k_slot_filter<<<g, t, smem, st>>>(a.S, a.B, a.a0, a.a1); break;
+    case MK_SLOT_SCAN: k_slot_scan<<<g, t, smem, st>>>(a.B, a.a0); break;
     case MK_BULK: k_bulk<<<g, t, smem, st>>>(a.S, a.B, (const int4 *)a.p); break;
     case MK_EVAL_REAL_CELL: k_atoms_eval<true, false, kSchedCell><<<g, t, smem, st>>>(a.S, a.B); break;
     case MK_EVAL_RANDOM_CELL: k_atoms_eval<true, true, kSchedCell><<<g, t, smem, st>>>(a.S, a.B); break;
@@ -1209,7 +1242,7 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
         return a;
     };
     em.zero(B.FS, sizeof(FrameScratch) * nf);
-    em.zero(B.counters, 8 * sizeof(int));
+    em.zero(B.counters, kCounters * sizeof(int));
     em.kernel(MK_OFFTABLE, dim3(grid_for(cmgeom::kOffEntries, 256), nf), 0, CM_K_PREP, base);
     const T *xsolv = self ? xs : xv;
     em.kernel(f32 ? MK_PREP_SOLVENT_F32 : MK_PREP_SOLVENT_F64, dim3(grid_for(mv, 128), nf), 0, CM_K_PREP,
@@ -1231,6 +1264,10 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
     auto agrid_grid = [&](int64_t n, int ctas) {
         return (int)std::min<int64_t>(grid_for(n, 256), (int64_t)sms * ctas);
     };
+    // k_agrid_records: a grid for one query in 64
+    auto rec_grid = [&](int64_t n) {
+        return (int)std::min<int64_t>(grid_for(n, 64 * (kAgridRecThreads / kAgridRecLanes)), (int64_t)sms * 16);
+    };
     if (agrid) {
         // the single solute molecule's candidate lists of every frame
         em.zero(B.gpool, (size_t)nf * sizeof(int));
@@ -1240,6 +1277,7 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
         // counters[6 .. 7]: the queries' next molecule (zeroed with the chunk's counters)
         em.zero(B.counters + 2, sizeof(int));
         em.kernel(MK_AGRID_REAL, dim3(agrid_grid((int64_t)nf * mv, h->agrid_real_ctas)), hsm, CM_K_REAL, base);
+        if (h->mddf) em.kernel(MK_AGRID_REC_REAL, dim3(rec_grid((int64_t)nf * mv)), hsm, CM_K_REAL, base);
         // the queue is empty unless a frame lost its grid: a grid for one
         // entry per 32 molecules
         em.kernel(eval_kid(h, false), dim3(wgrid_for((int64_t)nf * mv / 32)), hsm, CM_K_REAL, base);
@@ -1258,16 +1296,24 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
         em.kernel(MK_BULK, dim3(c.ntab), 0, CM_K_BULK, args(dtab + c.tab0, 0, 0, 0, 0));
         for (int s0 = 0; s0 < c.nsmp; s0 += h->atoms_piece) {
             const int ny = std::min(h->atoms_piece, c.nsmp - s0);
-            // the evaluation queue, the slot list and the queries' next slot (counters 2 .. 6)
-            em.zero(B.counters + 2, 5 * sizeof(int));
-            // slots that can reach the solute, their FP64 placement on full
-            // warps, then (candidate grid) their queries
-            em.kernel(MK_SLOT_FILTER, dim3(grid_for(mv, 128), ny), 0, CM_K_RANDOM, args(nullptr, 0, 0, c.smp0 + s0, 0));
+            // the piece's frames (every frame of a chunk has n_random_samples samples)
+            const int f0 = s0 / d.n_random_samples, f1 = (s0 + ny - 1) / d.n_random_samples;
+            // the evaluation queue, the slot list, the queries' next slot, the sorted list and the deferred queries
+            // (counters 2 .. 9)
+            em.zero(B.counters + 2, 8 * sizeof(int));
+            if (agrid) em.zero(B.scount, (size_t)(f1 - f0 + 1) * B.gfs * sizeof(int));
+            // slots that can reach the solute, their placement on full warps,
+            // then (candidate grid) their queries in fine-cell order
+            em.kernel(MK_SLOT_FILTER, dim3(grid_for(mv, 128), ny), 0, CM_K_RANDOM, args(nullptr, 0, 0, c.smp0 + s0, f0));
+            if (agrid) em.kernel(MK_SLOT_SCAN, dim3(f1 - f0 + 1), 0, CM_K_RANDOM, args(nullptr, 0, 0, f0, 0));
             em.kernel(MK_ATOMS_PLACE, dim3((unsigned)std::min<int64_t>(grid_for((int64_t)ny * mv, 128), (int64_t)sms * 16)),
-                      0, CM_K_RANDOM, args(nullptr, 0, 0, c.smp0 + s0, 0));
-            if (agrid)
+                      0, CM_K_RANDOM, args(nullptr, 0, 0, c.smp0 + s0, f0));
+            if (agrid) {
                 em.kernel(MK_AGRID_RANDOM, dim3(agrid_grid((int64_t)ny * mv, h->agrid_rand_ctas)), hsm, CM_K_RANDOM,
                           args(nullptr, 0, 0, c.smp0 + s0, ny));
+                em.kernel(MK_AGRID_REC_RANDOM, dim3(rec_grid((int64_t)ny * mv)), hsm, CM_K_RANDOM,
+                          args(nullptr, 0, 0, c.smp0 + s0, 0));
+            }
             em.kernel(eval_kid(h, true), dim3(wgrid_for((int64_t)ny * mv / (agrid ? 32 : 1))), hsm, CM_K_RANDOM, base);
         }
     }
@@ -1298,7 +1344,7 @@ void run_chunk(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample *
     int launches = 0;
     if (h->regime == CM_REGIME_PAIRS) {
         CM_CUDA(cudaMemsetAsync(B.FS, 0, sizeof(FrameScratch) * nf, st));
-        CM_CUDA(cudaMemsetAsync(B.counters, 0, 8 * sizeof(int), st));
+        CM_CUDA(cudaMemsetAsync(B.counters, 0, kCounters * sizeof(int), st));
         CM_LAUNCH(CM_K_PREP, k_offtable<<<dim3(grid_for(cmgeom::kOffEntries, 256), nf), 256, 0, st>>>(B));
         if (rnd) CM_CUDA(cudaMemsetAsync(B.flags, 0, (size_t)nf * B.ndist * mv, st));
         CM_CUDA(cudaMemsetAsync(B.ccount, 0, (size_t)nf * B.cs * 4, st));
@@ -1755,7 +1801,7 @@ void free_all(cm_handle *h) {
                      &h->vo32, &h->vo64, &h->u64, &h->u32, &h->rc, &h->ccount, &h->cstart, &h->cfill, &h->cmol, &h->cq32, &h->gq, &h->eq, &h->rq, &h->akey, &h->atq32,
                      &h->atq64, &h->asq32, &h->asq64, &h->acount, &h->astart, &h->afill, &h->avcell, &h->avq32, &h->avq64,
                      &h->pcell, &h->pq32, &h->pq64, &h->anear, &h->aq, &h->g_soff, &h->g_sidx, &h->g_voff, &h->g_vidx,
-                     &h->dcd_sidx, &h->dcd_vidx, &h->dcd_raw[0], &h->dcd_raw[1], &h->final_out, &h->final_job,
+                     &h->aslot, &h->skey, &h->sslot, &h->scount, &h->gstart, &h->gedge, &h->gpool, &h->gent, &h->dcd_sidx, &h->dcd_vidx, &h->dcd_raw[0], &h->dcd_raw[1], &h->final_out, &h->final_job,
                      &h->contrib_q, &h->contrib_g, &h->contrib_out};
     for (DevBuf *b : all) {
         blocks().put(h->device, false, b->p, b->bytes);
@@ -1843,7 +1889,7 @@ void noalloc_fixed(cm_handle *h, Carve &c) {
     c.take(h->fscratch, sizeof(FrameScratch));
     c.take(h->off64, sizeof(d4) * cmgeom::kOffEntries);
     c.take(h->off32, sizeof(float4) * cmgeom::kOffEntries);
-    c.take(h->counters, 8 * sizeof(int));
+    c.take(h->counters, kCounters * sizeof(int));
     c.take(h->stats, ST_N * 8);
     if (d.precision == CM_PRECISION_FP32_GUARD) {
         c.take(h->hist_snap, (size_t)h->hist_n * 8);
@@ -2129,9 +2175,12 @@ void launch_multi(int kid, unsigned grid, size_t smem, cudaStream_t st, const MT
         CM_MK(MK_AGRID_BUILD)
         CM_MK(MK_AGRID_REAL)
         CM_MK(MK_AGRID_RANDOM)
+        CM_MK(MK_AGRID_REC_REAL)
+        CM_MK(MK_AGRID_REC_RANDOM)
         CM_MK(MK_ATOMS_FILTER)
         CM_MK(MK_ATOMS_PLACE)
         CM_MK(MK_SLOT_FILTER)
+        CM_MK(MK_SLOT_SCAN)
         CM_MK(MK_BULK)
         CM_MK(MK_EVAL_REAL_CELL)
         CM_MK(MK_EVAL_RANDOM_CELL)
@@ -2172,7 +2221,7 @@ void record_chunk(cm_handle *h, const Staged &S, const Chunk &c, std::vector<Ste
 // stage differ (the ATOMS evaluation schedule follows each solute's density)
 // the stage takes one launch per kernel.  False (nothing launched) when the
 // systems cannot share the launches: another layout or precision, a weight
-// class change inside the round, or chains of different lengths.
+// class change inside the round, or chains of different stages.
 bool batch_round_fused(cm_batch *bt, std::vector<Staged> &st, const std::vector<char> &active) {
     const size_t n = bt->hs.size();
     size_t nchunks = 0;
@@ -2200,9 +2249,10 @@ bool batch_round_fused(cm_batch *bt, std::vector<Staged> &st, const std::vector<
             const std::vector<Step> &r = rec[j][i];
             if (!shape) shape = &r;
             else {
-                if (r.size() != shape->size()) return false;
-                for (size_t k = 0; k < r.size(); ++k)
+                // a system of fewer random-insertion pieces has the shorter chain; its steps are the first ones
+                for (size_t k = 0; k < std::min(r.size(), shape->size()); ++k)
                     if (r[k].kernel != (*shape)[k].kernel) return false;
+                if (r.size() > shape->size()) shape = &r;
             }
         }
     }
