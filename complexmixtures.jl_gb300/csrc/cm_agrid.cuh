@@ -499,12 +499,6 @@ __device__ __forceinline__ void agrid_query(int gl, const Bufs &B, const FrameGe
     }
 }
 
-// The lanes of the calling lane's group of G.
-template <int G>
-__device__ __forceinline__ unsigned agrid_group_mask() {
-    return G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
-}
-
 // Exact scan of a slot's or molecule's sites over their lists: every list
 // entry whose FP32 squared distance is within thr_arg (or, for the reference
 // site, thr_r1) is evaluated exactly (exact_d2 on the input coordinates) and
@@ -512,7 +506,8 @@ __device__ __forceinline__ unsigned agrid_group_mask() {
 // for the same thresholds.  The thresholds come from the query's minima plus
 // 2 delta, so each such atom lies within (nearest distance + 3 delta) of its
 // site, which the list's margin covers, and the buckets past sqrt(thr) + band
-// hold none of them.
+// hold none of them.  A group of GL lanes (gl the lane in it) splits the lists;
+// every lane of the warp calls it (both thresholds negative: nothing to scan).
 template <int GL>
 __device__ __noinline__ void agrid_exact(int gl, const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F,
                                          int f, ExactMol &X, const int *vc, const float4 *vq, float band, float thr_arg,
@@ -520,8 +515,9 @@ __device__ __noinline__ void agrid_exact(int gl, const DevSys &S, const Bufs &B,
     best_init(Bst);
     rr1 = INFINITY;
     evals = 0;
+    const int apv = fmaxf(thr_arg, thr_r1) >= 0.f ? S.apv : 0;
     const float4 *e = B.gent + (int64_t)f * B.gcap;
-    for (int b = 0; b < S.apv; ++b) {
+    for (int b = 0; b < apv; ++b) {
         const bool isref = b == S.iref;
         const float thr = isref ? fmaxf(thr_arg, thr_r1) : thr_arg;
         if (!(thr >= 0.f)) continue;
@@ -565,19 +561,18 @@ __device__ __noinline__ void agrid_exact(int gl, const DevSys &S, const Bufs &B,
     if (GL > 1) {
         // the group's smallest d = sqrt(d2), among equal d the larger (a, b); every lane ends with it
         double d = Bst.d2 <= S.cut2 ? best_d(Bst) : INFINITY;
-        const unsigned mask = agrid_group_mask<GL>();
 #pragma unroll
         for (int o = GL / 2; o > 0; o >>= 1) {
-            const double od = __shfl_xor_sync(mask, d, o), od2 = __shfl_xor_sync(mask, Bst.d2, o);
-            const int oa = __shfl_xor_sync(mask, Bst.a, o), ob = __shfl_xor_sync(mask, Bst.b, o);
+            const double od = __shfl_xor_sync(0xffffffffu, d, o), od2 = __shfl_xor_sync(0xffffffffu, Bst.d2, o);
+            const int oa = __shfl_xor_sync(0xffffffffu, Bst.a, o), ob = __shfl_xor_sync(0xffffffffu, Bst.b, o);
             if (od < d || (od == d && (oa > Bst.a || (oa == Bst.a && ob > Bst.b)))) {
                 if (od < d) Bst.d2 = od2;
                 d = od;
                 Bst.a = oa;
                 Bst.b = ob;
             }
-            rr1 = fmin(rr1, __shfl_xor_sync(mask, rr1, o));
-            evals += __shfl_xor_sync(mask, evals, o);
+            rr1 = fmin(rr1, __shfl_xor_sync(0xffffffffu, rr1, o));
+            evals += __shfl_xor_sync(0xffffffffu, evals, o);
         }
         Bst.d = d <= 1e300 ? d : -1.0;
     }
@@ -611,140 +606,133 @@ __device__ __forceinline__ int agrid_decide(const DevSys &S, const Guard &g, con
 // The record of a query inside the band (agrid_decide's 2), decided by
 // atoms_decide's rules with the exact scans over the sites' lists (agrid_exact)
 // instead of the stencil walk: v the solvent molecule (sample < 0) or the
-// slot of sample `sample`, whose placement is drawn again in FP64.  The GL
-// lanes of a group share the scans and return the same record; the first one
-// counts the statistics.
+// slot of sample `sample`, whose placement is drawn again in FP64.  Every lane
+// of the warp calls it (active: the lane's group has a record), so that the
+// groups go through the FP64 chain together; the GL lanes of a group share the
+// scan and return the same record, the first one counts the statistics.
 template <int GL>
-__device__ __noinline__ DirRec agrid_record(int gl, const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F,
-                                            int f, int v, int sample, const int *vc, const float4 *vq, const Top2 &T,
-                                            LocalStats &st) {
+__device__ __forceinline__ DirRec agrid_record(int gl, bool active, const DevSys &S, const Bufs &B, const FrameGeom &G,
+                                               const FrameScratch &F, int f, int v, int sample, const int *vc,
+                                               const float4 *vq, const Top2 &T, LocalStats &st) {
     const Guard &g = F.g;
     const float band = g.two_delta + 1e-3f * (1.0f + (float)S.cut);
     const int64_t vb = (int64_t)v * S.apv;
     ExactMol X;
-    if (sample < 0) {
-        X = exact_mol(S, f, 0, v);
-    } else {
-        const Sample sm = B.samples[sample];
-        const Placement P = draw_placement(S, G.frame_id, sm, v, B.bulk + (int64_t)f * B.ndist * B.mv,
-                                           B.nbulk + (int64_t)f * B.ndist);
-        uint64_t rs = P.st;
-        double R[9];
-        draw_rotation(rs, R);
-        X = exact_mol_placed(S, G, f, sm.s, P.jmol, P.fc, R);
+    if (active) {
+        if (sample < 0) {
+            X = exact_mol(S, f, 0, v);
+        } else {
+            const Sample sm = B.samples[sample];
+            const Placement P = draw_placement(S, G.frame_id, sm, v, B.bulk + (int64_t)f * B.ndist * B.mv,
+                                               B.nbulk + (int64_t)f * B.ndist);
+            uint64_t rs = P.st;
+            double R[9];
+            draw_rotation(rs, R);
+            X = exact_mol_placed(S, G, f, sm.s, P.jmol, P.fc, R);
+            exact_mol_ready(B, G, X);
+        }
     }
+    __syncwarp();
     DirRec r = dir_none(S);
-    if (!(T.m1 <= g.cutp2)) return r;
+    active = active && T.m1 <= g.cutp2;
     const float d1 = sqrtf(T.m1);
-    if (T.m1 >= g.cutm2 || (sqrtf(T.m2) - d1) <= g.two_delta) {
-        const float thr1 = T.r1 <= g.cutp2 ? r_sq_ru(sqrtf(T.r1) + g.two_delta) : -1.f;
-        Best64 Bst;
-        double rr1;
-        long long ev;
-        agrid_exact<GL>(gl, S, B, G, F, f, X, vc, vq, band, r_sq_ru(d1 + g.two_delta), thr1, Bst, rr1, ev);
-        if (gl == 0) {
+    // amb: the closest pair or the cutoff decision needs the exact scan; else
+    // the search's minimum pair is the exact minimum pair
+    const bool amb = active && (T.m1 >= g.cutm2 || (sqrtf(T.m2) - d1) <= g.two_delta);
+    int bin = active && !amb ? bin_of(g, d1) : -1;
+    const bool edge = active && !amb && (bin < 0 || (S.usecutoff && d1 >= g.dbulk_lo && d1 <= g.dbulk_hi));
+    const bool ref = active && T.r1 <= g.cutp2;
+    int rb = ref && !amb && T.r1 < g.cutm2 ? bin_of(g, sqrtf(T.r1)) : -1;
+    const bool rscan = ref && rb < 0;
+    Best64 Bst;
+    double rr1;
+    long long ev;
+    agrid_exact<GL>(gl, S, B, G, F, f, X, vc, vq, band, amb ? r_sq_ru(d1 + g.two_delta) : -1.f,
+                    rscan ? r_sq_ru(sqrtf(T.r1) + g.two_delta) : -1.f, Bst, rr1, ev);
+    double d64 = -1.0;
+    if (edge) d64 = sqrt(exact_pair_d2(B, G, X, T.p1, T.b1));
+    if (!active) return r;
+    if (gl == 0) {
+        if (amb || rscan) {
             st.guard++;
             st.guard_pairs += ev;
         }
-        if (Bst.d2 <= S.cut2) {
-            const double d = best_d(Bst);
-            if (gl == 0) st.maxerr = fmax(st.maxerr, fabs((double)d1 - d));
-            r.within = 1;
-            r.i_local = Bst.a;
-            r.j = vb + Bst.b;
-            r.bin = setbin0(d, S.binstep);
-            r.bulk = inbulk64(S, true, d);
-            if (rr1 <= S.cut2) {
-                r.ref = 1;
-                r.rbin = setbin0(sqrt(rr1), S.binstep);
-            }
-        }
-        return r;
-    }
-    // the search's minimum pair is the exact minimum pair
-    int bin = bin_of(g, d1);
-    double d64 = -1.0;
-    if (bin < 0 || (S.usecutoff && d1 >= g.dbulk_lo && d1 <= g.dbulk_hi)) {
-        d64 = sqrt(exact_pair_d2(B, G, X, T.p1, T.b1));
-        bin = setbin0(d64, S.binstep);
-        if (gl == 0) {
+        if (edge) {
             st.guard++;
             st.guard_pairs++;
-            st.maxerr = fmax(st.maxerr, fabs((double)d1 - d64));
         }
     }
     r.within = 1;
-    r.i_local = T.p1;
-    r.j = vb + T.b1;
+    if (amb) {
+        if (!(Bst.d2 <= S.cut2)) {
+            r.within = 0;
+            return r;
+        }
+        d64 = best_d(Bst);
+        r.i_local = Bst.a;
+        r.j = vb + Bst.b;
+    } else {
+        r.i_local = T.p1;
+        r.j = vb + T.b1;
+    }
+    if (amb || edge) {
+        if (gl == 0) st.maxerr = fmax(st.maxerr, fabs((double)d1 - d64));
+        bin = setbin0(d64, S.binstep);
+    }
     r.bin = bin;
     r.bulk = S.usecutoff ? (d64 >= 0.0 ? (d64 > S.dbulk) : (d1 > g.dbulk_hi)) : 0;
-    if (T.r1 <= g.cutp2) {
-        const int rb = T.r1 < g.cutm2 ? bin_of(g, sqrtf(T.r1)) : -1;
-        if (rb >= 0) {
-            r.ref = 1;
-            r.rbin = rb;
-        } else {
-            Best64 Bst;
-            double rr1;
-            long long ev;
-            agrid_exact<GL>(gl, S, B, G, F, f, X, vc, vq, band, -1.f, r_sq_ru(sqrtf(T.r1) + g.two_delta), Bst, rr1, ev);
-            if (gl == 0) {
-                st.guard++;
-                st.guard_pairs += ev;
-            }
-            if (rr1 <= S.cut2) {
-                r.ref = 1;
-                r.rbin = setbin0(sqrt(rr1), S.binstep);
-            }
-        }
+    if (rscan) rb = rr1 <= S.cut2 ? setbin0(sqrt(rr1), S.binstep) : -1;
+    if (rb >= 0) {
+        r.ref = 1;
+        r.rbin = rb;
     }
     return r;
 }
 
 // Top-2 of a molecule's or slot's sites over their lists (vc, vq: its sites'
-// cells and positions); false when no listed atom was met.
+// cells and positions); false when no listed atom was met.  With GL > 1 every
+// lane of the warp calls it (active: the lane's group has a query) and a group
+// ends with the same values.
 template <int GL>
-__device__ __forceinline__ bool agrid_top2(int gl, const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F, int f,
+__device__ __forceinline__ bool agrid_top2(int gl, bool active, const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F, int f,
                                            const int *vc, const float4 *vq, Top2 &T, long long &ev) {
     top2_init(T);
     ev = 0;
     const float band = F.g.two_delta + 1e-3f * (1.0f + (float)S.cut);
-    for (int b = 0; b < S.apv; ++b) agrid_query<GL>(gl, B, G, F, f, vc[b], vq[b], b, b == S.iref, band, T, ev);
+    const int apv = active ? S.apv : 0;
+    for (int b = 0; b < apv; ++b) agrid_query<GL>(gl, B, G, F, f, vc[b], vq[b], b, b == S.iref, band, T, ev);
     if (GL > 1) {
         // the group's top-2; every lane ends with it
-        const unsigned mask = agrid_group_mask<GL>();
 #pragma unroll
         for (int o = GL / 2; o > 0; o >>= 1) {
-            const float m1 = __shfl_xor_sync(mask, T.m1, o), m2 = __shfl_xor_sync(mask, T.m2, o);
-            const int p1 = __shfl_xor_sync(mask, T.p1, o), b1 = __shfl_xor_sync(mask, T.b1, o);
+            const float m1 = __shfl_xor_sync(0xffffffffu, T.m1, o), m2 = __shfl_xor_sync(0xffffffffu, T.m2, o);
+            const int p1 = __shfl_xor_sync(0xffffffffu, T.p1, o), b1 = __shfl_xor_sync(0xffffffffu, T.b1, o);
             T.m2 = fminf(fmaxf(T.m1, m1), fminf(T.m2, m2));
             if (m1 < T.m1 || (m1 == T.m1 && (p1 < T.p1 || (p1 == T.p1 && b1 < T.b1)))) {
                 T.p1 = p1;
                 T.b1 = b1;
             }
             T.m1 = fminf(T.m1, m1);
-            T.r1 = fminf(T.r1, __shfl_xor_sync(mask, T.r1, o));
+            T.r1 = fminf(T.r1, __shfl_xor_sync(0xffffffffu, T.r1, o));
         }
+        return __shfl_sync(0xffffffffu, (int)(ev != 0), 0, GL) != 0;
     }
     return ev != 0;
 }
 
 // A query inside the band: listed for k_agrid_records (counters[9] entries in
-// adefer), false when there is no room for it.  About one query in a hundred
+// adefer, which holds every query of a launch).  About one query in a hundred
 // is inside the band, and decided on the spot it left its warp on one lane of
 // dependent FP64 operations in a third of the warp's rounds.
-__device__ __forceinline__ bool agrid_defer(const Bufs &B, int entry) {
-    if (B.adefer_cap == 0) return false;
-    const int at = atomicAdd(B.counters + 9, 1);
-    if (at >= B.adefer_cap) return false;
-    B.adefer[at] = entry;
-    return true;
+__device__ __forceinline__ void agrid_defer(const Bufs &B, int entry) {
+    B.adefer[atomicAdd(B.counters + 9, 1)] = entry;
 }
 
-// Real pass of a single solute molecule, one thread per (frame, solvent
+// Real pass of a single solute molecule, GL lanes per (frame, solvent
 // molecule), persistent grid; frames without a grid queue their near pairs
 // for k_atoms_eval (k_atoms_filter's rule).
-__device__ __forceinline__ void k_agrid_real_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B) {
+template <int GL>
+__device__ __forceinline__ void agrid_real(const DevSys &S, const Bufs &B) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned int *hbase = (unsigned int *)smem_raw;
     shist_zero(S, hbase);
@@ -764,41 +752,41 @@ __device__ __forceinline__ void k_agrid_real_body(const uint3 blockIdx, const di
             }
         }
     };
-    auto one_molecule = [&](int it) {
+    const int lane = threadIdx.x & 31, gl = lane % GL;
+    auto one_molecule = [&](int it, bool active) {
         const int f = it / S.mv, v = it - f * S.mv;
         const FrameScratch &F = B.FS[f];
         const FrameGeom &G = B.G[f];
         const int *vc = B.avcell + (int64_t)f * B.Nv + (int64_t)v * apv;
-        if (!F.agrid) {
-            if (!F.ok) {
-                raise_err(S, ERR_STENCIL);
-                return;
+        if (!F.agrid && active) {
+            active = false;
+            if (gl == 0) {
+                if (!F.ok) raise_err(S, ERR_STENCIL);
+                else if (atoms_near(B, G, f, 0, vc, apv)) atoms_push(S, B, make_int4(v, 0, f, 0));
             }
-            if (atoms_near(B, G, f, 0, vc, apv)) atoms_push(S, B, make_int4(v, 0, f, 0));
-            return;
         }
         const float4 *vq = B.avq32 + (int64_t)f * B.Nv + (int64_t)v * apv;
         Top2 T;
         long long ev;
-        if (!agrid_top2<1>(0, S, B, G, F, f, vc, vq, T, ev)) return;
+        if (!agrid_top2<GL>(gl, active, S, B, G, F, f, vc, vq, T, ev)) return;
         DirRec r;
+        if (gl != 0) return;
         if (agrid_decide(S, F.g, T, (int64_t)v * apv, r) == 2) {
-            if (agrid_defer(B, it)) return;
-            r = agrid_record<1>(0, S, B, G, F, f, v, -1, vc, vq, T, st);
+            agrid_defer(B, it);
+            return;
         }
         st.atompairs += (unsigned long long)ev;
         put(r, f, v);
     };
-    // warps take 32 molecules at a time from counters[6] (zeroed with the
+    // warps take their molecules from counters[6] (zeroed with the
     // chunk's counters), as k_agrid_random takes its slots; nf mv < 2^31 (the
     // fallback's queue holds every item of the chunk)
-    const int lane = threadIdx.x & 31;
     for (;;) {
         long long at = 0;
-        if (lane == 0) at = (long long)atomicAdd((unsigned long long *)(B.counters + 6), 32ull);
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (at >= n) break;
-        if (at + lane < n) one_molecule((int)at + lane);
+        if (lane == 0) at = (long long)atomicAdd((unsigned long long *)(B.counters + 6), (unsigned long long)(32 / GL));
+        at = __shfl_sync(0xffffffffu, at, 0) + lane / GL;
+        if (at - lane / GL >= n) break;
+        one_molecule((int)(at < n ? at : n - 1), at < n);
         __syncwarp();
     }
     stats_flush(S, st, false);
@@ -806,12 +794,18 @@ __device__ __forceinline__ void k_agrid_real_body(const uint3 blockIdx, const di
     shist_flush(S, h, false);
 }
 
-// four resident CTAs per SM: the queries wait on their list entries (agrid_record is out of line)
+// Lanes per query: one for small solvent molecules, whose slots are many;
+// four for larger ones (more than four sites), whose lists are long and whose
+// slots do not fill the SMs (181 14-site molecules, 20 frames, 10 samples:
+// 235 us with one lane, 96 with four; 2,000 around a 20,000-atom chain, 16
+// frames: 891 and 436).  Four resident CTAs per SM: the queries wait on their
+// list entries.
+template <int GL>
 __global__ void __launch_bounds__(256, 4) k_agrid_real(DevSys S, Bufs B) {
-    k_agrid_real_body(blockIdx, gridDim, S, B);
+    agrid_real<GL>(S, B);
 }
 
-// Random insertion of a single solute molecule, last pass: one thread per
+// Random insertion of a single solute molecule, last pass: GL lanes per
 // slot that k_atoms_place placed, in the order of the slots' fine cells;
 // persistent grid.  The slot's sites are queried and the record is decided
 // (agrid_record inside the band).  k_atoms_place has
@@ -825,7 +819,8 @@ __global__ void __launch_bounds__(256, 4) k_agrid_real(DevSys S, Bufs B) {
 // samples) the queries went from 2,850 to 1,980 us sorted and four wide, to
 // 1,250 us (978 here, 274 in k_agrid_records) with the records inside the
 // band apart and 4 M slots a launch instead of 32 samples.
-__device__ __forceinline__ void k_agrid_random_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B, int sample0, int ny) {
+template <int GL>
+__device__ __forceinline__ void agrid_random(const DevSys &S, const Bufs &B, int sample0) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned int *hbase = (unsigned int *)smem_raw;
     shist_zero(S, hbase);
@@ -833,7 +828,7 @@ __device__ __forceinline__ void k_agrid_random_body(const uint3 blockIdx, const 
     const SHist h = shist_bind(S, hbase);
     LocalStats st;
     const int apv = S.apv;
-    (void)ny;
+    const int lane = threadIdx.x & 31, gl = lane % GL;
     const int n = min(B.counters[8], B.aslot_cap);
     auto put = [&](const DirRec &r) {
         st.molpairs++;
@@ -842,7 +837,7 @@ __device__ __forceinline__ void k_agrid_random_body(const uint3 blockIdx, const 
             st.hits++;
         }
     };
-    auto one_slot = [&](int e) {
+    auto one_slot = [&](int e, bool active) {
         const int y = e / S.mv, k = e - y * S.mv;
         const int f = B.samples[sample0 + y].pad;
         const FrameScratch &F = B.FS[f];
@@ -850,25 +845,25 @@ __device__ __forceinline__ void k_agrid_random_body(const uint3 blockIdx, const 
         const int64_t base = (int64_t)y * B.Nv + (int64_t)k * apv;
         Top2 T;
         long long ev;
-        if (!agrid_top2<1>(0, S, B, G, F, f, B.pcell + base, B.pq32 + base, T, ev)) return;
+        if (!agrid_top2<GL>(gl, active, S, B, G, F, f, B.pcell + base, B.pq32 + base, T, ev)) return;
         DirRec r;
+        if (gl != 0) return;
         if (agrid_decide(S, F.g, T, (int64_t)k * apv, r) == 2) {
-            if (agrid_defer(B, e)) return;
-            r = agrid_record<1>(0, S, B, G, F, f, k, sample0 + y, B.pcell + base, B.pq32 + base, T, st);
+            agrid_defer(B, e);
+            return;
         }
         st.atompairs += (unsigned long long)ev;
         put(r);
     };
-    // warps take 32 slots at a time from counters[6] (zeroed with the slot
-    // list): a fixed share per thread left the CTAs' warps waiting for their
-    // slowest one
-    const int lane = threadIdx.x & 31;
+    // warps take their slots from counters[6] (zeroed with the slot list): a
+    // fixed share per thread left the CTAs' warps waiting for their slowest one
     for (;;) {
         int at = 0;
-        if (lane == 0) at = atomicAdd(B.counters + 6, 32);
+        if (lane == 0) at = atomicAdd(B.counters + 6, 32 / GL);
         at = __shfl_sync(0xffffffffu, at, 0);
         if (at >= n) break;
-        if (at + lane < n) one_slot(B.sslot[at + lane]);
+        at += lane / GL;
+        one_slot(B.sslot[min(at, n - 1)], at < n);
         __syncwarp();
     }
     stats_flush(S, st, true);
@@ -876,18 +871,20 @@ __device__ __forceinline__ void k_agrid_random_body(const uint3 blockIdx, const 
     shist_flush(S, h, true);
 }
 
-__global__ void __launch_bounds__(256, 4) k_agrid_random(DevSys S, Bufs B, int sample0, int ny) {
-    k_agrid_random_body(blockIdx, gridDim, S, B, sample0, ny);
+template <int GL>
+__global__ void __launch_bounds__(256, 4) k_agrid_random(DevSys S, Bufs B, int sample0) {
+    agrid_random<GL>(S, B, sample0);
 }
 
 // The listed queries inside the band, a group of lanes each: queried again and
-// decided by agrid_record.  RANDOM: entries y mv + slot of the piece from
+// decided by agrid_record, the groups of a warp in step (left to run apart
+// they took 176 us instead of 51 on 50,000 slots of 1,200 atoms).  RANDOM: entries y mv + slot of the piece from
 // sample sample0 on; else entries frame mv + molecule.  Its time is the
 // latency of one record's FP64 chain; the list holds a few per SM, so they run
 // side by side.
 template <bool RANDOM>
 __device__ __forceinline__ void k_agrid_records_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B, int sample0) {
-    const int n = min(B.counters[9], B.adefer_cap);
+    const int n = B.counters[9];
     if ((int64_t)blockIdx.x * (blockDim.x / kAgridRecLanes) >= n) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned int *hbase = (unsigned int *)smem_raw;
@@ -897,8 +894,11 @@ __device__ __forceinline__ void k_agrid_records_body(const uint3 blockIdx, const
     LocalStats st;
     const int gl = threadIdx.x % kAgridRecLanes;
     const int per = blockDim.x / kAgridRecLanes;
-    for (int it = blockIdx.x * per + threadIdx.x / kAgridRecLanes; it < n; it += gridDim.x * per) {
-        const int e = B.adefer[it];
+    // every lane takes every round: the groups stay together
+    for (int i0 = blockIdx.x * per; i0 < n; i0 += gridDim.x * per) {
+        const int it = i0 + threadIdx.x / kAgridRecLanes;
+        const bool active = it < n;
+        const int e = B.adefer[min(it, n - 1)];
         const int row = e / S.mv, v = e - row * S.mv;
         const int f = RANDOM ? B.samples[sample0 + row].pad : row;
         const FrameScratch &F = B.FS[f];
@@ -908,9 +908,9 @@ __device__ __forceinline__ void k_agrid_records_body(const uint3 blockIdx, const
         const float4 *vq = (RANDOM ? B.pq32 : B.avq32) + base;
         Top2 T;
         long long ev;
-        agrid_top2<kAgridRecLanes>(gl, S, B, G, F, f, vc, vq, T, ev);
-        const DirRec r = agrid_record<kAgridRecLanes>(gl, S, B, G, F, f, v, RANDOM ? sample0 + row : -1, vc, vq, T, st);
-        if (gl != 0) continue;
+        agrid_top2<kAgridRecLanes>(gl, active, S, B, G, F, f, vc, vq, T, ev);
+        const DirRec r = agrid_record<kAgridRecLanes>(gl, active, S, B, G, F, f, v, RANDOM ? sample0 + row : -1, vc, vq, T, st);
+        if (!active || gl != 0) continue;
         st.molpairs++;
         st.atompairs += (unsigned long long)ev;
         if (r.within) {

@@ -402,7 +402,7 @@ struct Bufs {
     // ATOMS
     int *akey;                      // [nf][Ns]
     float4 *atq32, *asq32;
-    d4 *atq64, *asq64;
+    d4 *atq64, *asq64;              // the FP64 search only (nullptr in FP32, as avq64 and pq64)
     int *acount, *astart, *afill;   // [nf][as]
     int64_t as;
     int *avcell;                    // [nf][Nv]
@@ -423,8 +423,7 @@ struct Bufs {
     // centre (k_slot_filter counts, k_slot_scan, k_atoms_place scatters)
     int2 *skey;                     // [aslot_cap]: fine cell of the slot's frame (-1: no grid), rank among that cell's slots
     int *sslot;                     // [aslot_cap]: slots in fine-cell order; count in counters[8]
-    int *adefer;                    // queries inside the band (the slot list's memory, done with by then); count in counters[9]
-    int adefer_cap;
+    int *adefer;                    // queries inside the band; count in counters[9]
     int *scount;                    // [nf][gfs]: slots of each fine cell, then the first position of each in sslot
     // ATOMS candidate grid (one solute molecule, FP32 search): each search
     // cell split into agk^3 fine cells, each with the list of solute atoms
@@ -1756,7 +1755,7 @@ __device__ __forceinline__ void k_prep_atoms_solvent_body(const uint3 blockIdx, 
         const int64_t i = fo + (int64_t)m * apm + b;
         B.avcell[i] = pack_cell(c);
         B.avq32[i] = make_float4((float)q[0], (float)q[1], (float)q[2], 0.f);
-        B.avq64[i] = make_d4(q[0], q[1], q[2], 0.0);
+        if (B.avq64) B.avq64[i] = make_d4(q[0], q[1], q[2], 0.0);
     }
     warp_max_pos(&B.FS[f].xmax, __double2float_ru(xm));
     if (centroids) {
@@ -1794,7 +1793,7 @@ __device__ __forceinline__ void k_prep_atoms_solute_body(const uint3 blockIdx, c
     const int64_t fi = (int64_t)f * B.Ns + i;
     B.akey[fi] = k;
     B.atq32[fi] = make_float4((float)q[0], (float)q[1], (float)q[2], __int_as_float(a));
-    B.atq64[fi] = make_d4(q[0], q[1], q[2], 0.0);
+    if (B.atq64) B.atq64[fi] = make_d4(q[0], q[1], q[2], 0.0);
     atomicAdd(B.acount + (int64_t)f * B.as + k, 1);
     warp_max_pos(&B.FS[f].xmax, __double2float_ru(fmax(fabs(x[0]), fmax(fabs(x[1]), fabs(x[2])))));
 }
@@ -1811,7 +1810,7 @@ __device__ __forceinline__ void k_scatter_atoms_body(const uint3 blockIdx, const
     const int64_t fi = (int64_t)f * B.Ns + i;
     const int p = atomicAdd(B.afill + (int64_t)f * B.as + B.akey[fi], 1);
     B.asq32[(int64_t)f * B.Ns + p] = B.atq32[fi];
-    B.asq64[(int64_t)f * B.Ns + p] = B.atq64[fi];
+    if (B.asq64) B.asq64[(int64_t)f * B.Ns + p] = B.atq64[fi];
 }
 
 __global__ void k_scatter_atoms(Bufs B) {

@@ -25,7 +25,7 @@ struct __align__(16) MArgs {
     Bufs B;
     const void *p;   // coordinates (prep), bulk table (k_bulk)
     int64_t i0, i1;  // coordinate stride (prep); item range (k_atoms_filter)
-    int a0, a1;      // iref, centroids (prep solvent); pairs (frame consts); atoms_layout (scan); sample0, ny (random);
+    int a0, a1;      // iref, centroids (prep solvent); pairs (frame consts); atoms_layout (scan); sample0 (random);
                      // sample0, frame0 (slot filter, place); frame0 (slot scan)
 };
 
@@ -47,7 +47,9 @@ enum MKid : int {
     MK_ATOMS_NEAR,
     MK_AGRID_BUILD,
     MK_AGRID_REAL,
+    MK_AGRID_REAL4,
     MK_AGRID_RANDOM,
+    MK_AGRID_RANDOM4,
     MK_AGRID_REC_REAL,
     MK_AGRID_REC_RANDOM,
     MK_ATOMS_FILTER,
@@ -67,6 +69,10 @@ enum MKid : int {
     MK_NKIDS
 };
 
+__host__ __device__ constexpr bool mk_query(int kid) {
+    return kid == MK_AGRID_REAL || kid == MK_AGRID_REAL4 || kid == MK_AGRID_RANDOM || kid == MK_AGRID_RANDOM4;
+}
+
 // Threads per CTA of each stage (the stand-alone launch's block size).
 __host__ __device__ constexpr int mk_threads(int kid) {
     return kid == MK_OFFTABLE ? 256
@@ -77,7 +83,7 @@ __host__ __device__ constexpr int mk_threads(int kid) {
          : (kid == MK_SCATTER_ATOMS || kid == MK_ATOMS_NEAR) ? 256
          : kid == MK_AGRID_BUILD ? kAgridBuildThreads
          : (kid == MK_AGRID_REC_REAL || kid == MK_AGRID_REC_RANDOM) ? kAgridRecThreads
-         : (kid == MK_AGRID_REAL || kid == MK_AGRID_RANDOM || kid == MK_ATOMS_FILTER) ? 256
+         : (mk_query(kid) || kid == MK_ATOMS_FILTER) ? 256
          : (kid == MK_ATOMS_PLACE || kid == MK_SLOT_FILTER) ? 128
          : kid == MK_BULK ? 1024
          : kAtomsWarps * 32;
@@ -97,8 +103,10 @@ __device__ __forceinline__ void mk_body(const uint3 vb, const dim3 vg, const MAr
     else if constexpr (KID == MK_SCATTER_ATOMS) k_scatter_atoms_body(vb, vg, a.B);
     else if constexpr (KID == MK_ATOMS_NEAR) k_atoms_near_body(vb, vg, a.B);
     else if constexpr (KID == MK_AGRID_BUILD) k_agrid_build_body(vb, vg, a.S, a.B);
-    else if constexpr (KID == MK_AGRID_REAL) k_agrid_real_body(vb, vg, a.S, a.B);
-    else if constexpr (KID == MK_AGRID_RANDOM) k_agrid_random_body(vb, vg, a.S, a.B, a.a0, a.a1);
+    else if constexpr (KID == MK_AGRID_REAL) agrid_real<1>(a.S, a.B);
+    else if constexpr (KID == MK_AGRID_REAL4) agrid_real<4>(a.S, a.B);
+    else if constexpr (KID == MK_AGRID_RANDOM) agrid_random<1>(a.S, a.B, a.a0);
+    else if constexpr (KID == MK_AGRID_RANDOM4) agrid_random<4>(a.S, a.B, a.a0);
     else if constexpr (KID == MK_AGRID_REC_REAL) k_agrid_records_body<false>(vb, vg, a.S, a.B, 0);
     else if constexpr (KID == MK_AGRID_REC_RANDOM) k_agrid_records_body<true>(vb, vg, a.S, a.B, a.a0);
     else if constexpr (KID == MK_ATOMS_FILTER) k_atoms_filter_body(vb, vg, a.S, a.B, a.i0, a.i1);
@@ -117,7 +125,7 @@ __device__ __forceinline__ void mk_body(const uint3 vb, const dim3 vg, const MAr
 // come from the work table instead of the parameter space, and the register
 // budget of the stand-alone kernels is kept.
 __host__ __device__ constexpr int mk_min_ctas(int kid) {
-    return (kid == MK_AGRID_REAL || kid == MK_AGRID_RANDOM) ? 4 : mk_threads(kid) <= 256 ? 2 : 1;
+    return mk_query(kid) ? 4 : mk_threads(kid) <= 256 ? 2 : 1;
 }
 
 template <int KID>

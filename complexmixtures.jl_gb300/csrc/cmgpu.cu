@@ -169,7 +169,7 @@ constexpr int kCounters = 12;  // ints of Bufs::counters
 
 // Random samples placed per launch in the ATOMS layout.  FP64, or under an HBM
 // budget: 32 samples' worth of FP64 slots (52 bytes a site and 20 more); FP32
-// slots are smaller (20 a site and 32 more), so 44 to 77 samples fit the same
+// slots are smaller (20 a site and 36 more), so 41 to 76 samples fit the same
 // memory.  FP32 without a budget: up to kPieceSlots slots.  A piece's launches
 // end on their slowest warps and on the latency of its few exact records, so
 // fewer and larger pieces are faster.
@@ -177,9 +177,12 @@ constexpr int64_t kPieceSlots = 1 << 22;
 int chunk_samples(const cm_system_desc &d) {
     if (d.precision != CM_PRECISION_FP32_GUARD) return 32;
     const int64_t apv = d.solvent_natomspermol;
-    const int64_t fit = 32 * (52 * apv + 20) / (20 * apv + 32);
+    const int64_t fit = 32 * (52 * apv + 20) / (20 * apv + 36);
     return (int)(d.hbm_budget_bytes > 0 ? fit : std::max(fit, kPieceSlots / d.solvent_nmols));
 }
+
+// Lanes per candidate-grid query (k_agrid_real, k_agrid_random).
+int agrid_lanes(const cm_system_desc &d) { return d.solvent_natomspermol > 4 ? 4 : 1; }
 
 }  // namespace
 
@@ -222,7 +225,7 @@ struct cm_handle {
     DevBuf g_soff, g_sidx, g_voff, g_vidx;
     // ATOMS
     DevBuf akey, atq32, atq64, asq32, asq64, acount, astart, afill, avcell, avq32, avq64, u64, u32, rc, pcell, pq32, pq64,
-        anear, aq, aslot, skey, sslot, scount;
+        anear, aq, aslot, skey, sslot, scount, adefer;
     int aq_cap = 0;
     int aslot_cap = 0;     // random-insertion slot list (slots of one placement piece)
     int atoms_ctas = 0;    // resident CTAs per SM of k_atoms_eval
@@ -678,8 +681,10 @@ void kernel_smem_limits(int device) {
     raise((const void *)k_pairs_guard<false>);
     raise((const void *)k_pairs_edge<true>);
     raise((const void *)k_pairs_edge<false>);
-    raise((const void *)k_agrid_real);
-    raise((const void *)k_agrid_random);
+    raise((const void *)k_agrid_real<1>);
+    raise((const void *)k_agrid_real<4>);
+    raise((const void *)k_agrid_random<1>);
+    raise((const void *)k_agrid_random<4>);
     raise((const void *)k_agrid_build);
     raise((const void *)k_agrid_records<false>);
     raise((const void *)k_agrid_records<true>);
@@ -688,6 +693,8 @@ void kernel_smem_limits(int device) {
     raise((const void *)k_multi<MK_AGRID_BUILD>);
     raise((const void *)k_multi<MK_AGRID_REAL>);
     raise((const void *)k_multi<MK_AGRID_RANDOM>);
+    raise((const void *)k_multi<MK_AGRID_REAL4>);
+    raise((const void *)k_multi<MK_AGRID_RANDOM4>);
     raise((const void *)k_multi<MK_EVAL_REAL_CELL>);
     raise((const void *)k_multi<MK_EVAL_RANDOM_CELL>);
     raise((const void *)k_multi<MK_EVAL_REAL_BALANCED>);
@@ -859,12 +866,15 @@ void plan(cm_handle *h, const cm_frames *f) {
     } else {
         dev_alloc(h, h->akey, fc * h->Ns * 4);
         dev_alloc(h, h->atq32, fc * h->Ns * 16);
-        dev_alloc(h, h->atq64, fc * h->Ns * 32);
         dev_alloc(h, h->asq32, fc * h->Ns * 16);
-        dev_alloc(h, h->asq64, fc * h->Ns * 32);
         dev_alloc(h, h->avcell, fc * h->Nv * 4);
         dev_alloc(h, h->avq32, fc * h->Nv * 16);
-        dev_alloc(h, h->avq64, fc * h->Nv * 32);
+        if (d.precision != CM_PRECISION_FP32_GUARD) {
+            // the FP64 positions (the FP32 search's exact distances come from the input coordinates)
+            dev_alloc(h, h->atq64, fc * h->Ns * 32);
+            dev_alloc(h, h->asq64, fc * h->Ns * 32);
+            dev_alloc(h, h->avq64, fc * h->Nv * 32);
+        }
         if (h->mddf) {
             dev_alloc(h, h->u64, fc * h->Nv * 32);
             dev_alloc(h, h->u32, fc * h->Nv * 16);
@@ -902,17 +912,22 @@ void plan(cm_handle *h, const cm_frames *f) {
         h->atoms_dense = h->d.atoms_schedule == CM_SCHED_AUTO ? dense : h->d.atoms_schedule == CM_SCHED_CELL;
         h->atoms_ctas = atoms_setup(h);
         // candidate grid of a single solute molecule in the FP32 search (the
-        // plain FP64 path keeps the walk): by default for dense solutes, whose
-        // stencils hold many atoms per query, with fine cells of about 2.5 A.
+        // plain FP64 path keeps the walk), by default with fine cells of about
+        // 4.5 A when enough sites are asked for each solute atom.
         // The fallback of a frame whose lists overflow queues its near pairs,
         // so every item of a chunk must fit the queue.
         h->agk = 0;
         const bool fp32 = d.precision == CM_PRECISION_FP32_GUARD;
-        // a query is one thread per solvent molecule over its sites, so the
-        // grid pays off for small solvent molecules queried many times per
-        // frame (each real molecule and every random-insertion slot)
-        const bool pays = d.solvent_natomspermol <= 4 &&
-                          mv * (1 + (h->mddf ? (int64_t)d.n_random_samples : 0)) >= 4 * h->Ns;
+        // the build's cost follows the solute's atoms, the queries' the sites
+        // asked per frame (each real molecule and every random-insertion
+        // slot).  Walk and grid, us for 16 frames: 2,000 14-site molecules
+        // around 20,000 atoms (15 sites asked per atom) 7,300 and 2,800, 500
+        // around 8,000 (10) 1,870 and 1,590, 2,000 around 4,000 without
+        // insertions (7) 750 and 780, 1,000 single sites around 9,000 (0.4)
+        // 510 and 1,230
+        const int64_t asked = mv * (1 + (h->mddf ? (int64_t)d.n_random_samples : 0));
+        const bool pays = (d.solvent_natomspermol <= 4 && asked >= 4 * h->Ns) ||
+                          (d.solvent_natomspermol <= kMaxSmallMol && asked * d.solvent_natomspermol >= 8 * h->Ns);
         (void)dense;
         const bool want = d.atoms_grid > 0 || (d.atoms_grid == 0 && pays);
         if (want && fp32 && ms == 1 && !d.autocorrelation && (int64_t)fc * mv <= h->aq_cap) {
@@ -926,6 +941,7 @@ void plan(cm_handle *h, const cm_frames *f) {
                 h->agk = K;
                 h->gcap = gcap;
                 dev_alloc(h, h->gent, (size_t)bytes);
+                dev_alloc(h, h->adefer, (size_t)std::max<int64_t>(fc * mv, h->aslot_cap) * 4);
                 if (h->mddf) {
                     dev_alloc(h, h->skey, (size_t)h->aslot_cap * 8);
                     dev_alloc(h, h->sslot, (size_t)h->aslot_cap * 4);
@@ -934,8 +950,9 @@ void plan(cm_handle *h, const cm_frames *f) {
         }
         if (h->agk > 0) {
             const size_t hsm = hist_smem_bytes(h, h->smem_groups);
-            h->agrid_real_ctas = resident_ctas((const void *)k_agrid_real, 256, hsm);
-            h->agrid_rand_ctas = resident_ctas((const void *)k_agrid_random, 256, hsm);
+            const bool four = agrid_lanes(d) == 4;
+            h->agrid_real_ctas = resident_ctas(four ? (const void *)k_agrid_real<4> : (const void *)k_agrid_real<1>, 256, hsm);
+            h->agrid_rand_ctas = resident_ctas(four ? (const void *)k_agrid_random<4> : (const void *)k_agrid_random<1>, 256, hsm);
         }
     }
     h->planned = true;
@@ -1103,8 +1120,7 @@ Bufs chunk_bufs(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample 
             B.gent = P<float4>(h->gent);
             B.skey = P<int2>(h->skey);
             B.sslot = P<int>(h->sslot);
-            B.adefer = P<int>(h->aslot);
-            B.adefer_cap = h->mddf ? h->aslot_cap : 0;
+            B.adefer = P<int>(h->adefer);
             B.scount = P<int>(h->scount);
         }
         if (h->mddf) {
@@ -1137,8 +1153,10 @@ void launch_one(int kid, dim3 g, size_t smem, cudaStream_t st, const MArgs &a) {
     case MK_SCATTER_ATOMS: k_scatter_atoms<<<g, t, smem, st>>>(a.B); break;
     case MK_ATOMS_NEAR: k_atoms_near<<<g, t, smem, st>>>(a.B); break;
     case MK_AGRID_BUILD: k_agrid_build<<<g, t, smem, st>>>(a.S, a.B); break;
-    case MK_AGRID_REAL: k_agrid_real<<<g, t, smem, st>>>(a.S, a.B); break;
-    case MK_AGRID_RANDOM: k_agrid_random<<<g, t, smem, st>>>(a.S, a.B, a.a0, a.a1); break;
+    case MK_AGRID_REAL: k_agrid_real<1><<<g, t, smem, st>>>(a.S, a.B); break;
+    case MK_AGRID_RANDOM: k_agrid_random<1><<<g, t, smem, st>>>(a.S, a.B, a.a0); break;
+    case MK_AGRID_REAL4: k_agrid_real<4><<<g, t, smem, st>>>(a.S, a.B); break;
+    case MK_AGRID_RANDOM4: k_agrid_random<4><<<g, t, smem, st>>>(a.S, a.B, a.a0); break;
     case MK_AGRID_REC_REAL: k_agrid_records<false><<<g, t, smem, st>>>(a.S, a.B, 0); break;
     case MK_AGRID_REC_RANDOM: k_agrid_records<true><<<g, t, smem, st>>>(a.S, a.B, a.a0); break;
     case MK_ATOMS_FILTER: k_atoms_filter<<<g, t, smem, st>>>(a.S, a.B, a.i0, a.i1); break;
@@ -1262,7 +1280,7 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
     };
     const bool agrid = h->agk > 0;
     auto agrid_grid = [&](int64_t n, int ctas) {
-        return (int)std::min<int64_t>(grid_for(n, 256), (int64_t)sms * ctas);
+        return (int)std::min<int64_t>(grid_for(n * agrid_lanes(d), 256), (int64_t)sms * ctas);
     };
     // k_agrid_records: a grid for one query in 64
     auto rec_grid = [&](int64_t n) {
@@ -1276,8 +1294,8 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
         // decided in place); frames without a grid go to the evaluation queue.
         // counters[6 .. 7]: the queries' next molecule (zeroed with the chunk's counters)
         em.zero(B.counters + 2, sizeof(int));
-        em.kernel(MK_AGRID_REAL, dim3(agrid_grid((int64_t)nf * mv, h->agrid_real_ctas)), hsm, CM_K_REAL, base);
-        if (h->mddf) em.kernel(MK_AGRID_REC_REAL, dim3(rec_grid((int64_t)nf * mv)), hsm, CM_K_REAL, base);
+        em.kernel(agrid_lanes(d) == 4 ? MK_AGRID_REAL4 : MK_AGRID_REAL, dim3(agrid_grid((int64_t)nf * mv, h->agrid_real_ctas)), hsm, CM_K_REAL, base);
+        em.kernel(MK_AGRID_REC_REAL, dim3(rec_grid((int64_t)nf * mv)), hsm, CM_K_REAL, base);
         // the queue is empty unless a frame lost its grid: a grid for one
         // entry per 32 molecules
         em.kernel(eval_kid(h, false), dim3(wgrid_for((int64_t)nf * mv / 32)), hsm, CM_K_REAL, base);
@@ -1309,7 +1327,7 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
             em.kernel(MK_ATOMS_PLACE, dim3((unsigned)std::min<int64_t>(grid_for((int64_t)ny * mv, 128), (int64_t)sms * 16)),
                       0, CM_K_RANDOM, args(nullptr, 0, 0, c.smp0 + s0, f0));
             if (agrid) {
-                em.kernel(MK_AGRID_RANDOM, dim3(agrid_grid((int64_t)ny * mv, h->agrid_rand_ctas)), hsm, CM_K_RANDOM,
+                em.kernel(agrid_lanes(d) == 4 ? MK_AGRID_RANDOM4 : MK_AGRID_RANDOM, dim3(agrid_grid((int64_t)ny * mv, h->agrid_rand_ctas)), hsm, CM_K_RANDOM,
                           args(nullptr, 0, 0, c.smp0 + s0, ny));
                 em.kernel(MK_AGRID_REC_RANDOM, dim3(rec_grid((int64_t)ny * mv)), hsm, CM_K_RANDOM,
                           args(nullptr, 0, 0, c.smp0 + s0, 0));
@@ -1801,7 +1819,7 @@ void free_all(cm_handle *h) {
                      &h->vo32, &h->vo64, &h->u64, &h->u32, &h->rc, &h->ccount, &h->cstart, &h->cfill, &h->cmol, &h->cq32, &h->gq, &h->eq, &h->rq, &h->akey, &h->atq32,
                      &h->atq64, &h->asq32, &h->asq64, &h->acount, &h->astart, &h->afill, &h->avcell, &h->avq32, &h->avq64,
                      &h->pcell, &h->pq32, &h->pq64, &h->anear, &h->aq, &h->g_soff, &h->g_sidx, &h->g_voff, &h->g_vidx,
-                     &h->aslot, &h->skey, &h->sslot, &h->scount, &h->gstart, &h->gedge, &h->gpool, &h->gent, &h->dcd_sidx, &h->dcd_vidx, &h->dcd_raw[0], &h->dcd_raw[1], &h->final_out, &h->final_job,
+                     &h->aslot, &h->skey, &h->adefer, &h->sslot, &h->scount, &h->gstart, &h->gedge, &h->gpool, &h->gent, &h->dcd_sidx, &h->dcd_vidx, &h->dcd_raw[0], &h->dcd_raw[1], &h->final_out, &h->final_job,
                      &h->contrib_q, &h->contrib_g, &h->contrib_out};
     for (DevBuf *b : all) {
         blocks().put(h->device, false, b->p, b->bytes);
@@ -2175,6 +2193,8 @@ void launch_multi(int kid, unsigned grid, size_t smem, cudaStream_t st, const MT
         CM_MK(MK_AGRID_BUILD)
         CM_MK(MK_AGRID_REAL)
         CM_MK(MK_AGRID_RANDOM)
+        CM_MK(MK_AGRID_REAL4)
+        CM_MK(MK_AGRID_RANDOM4)
         CM_MK(MK_AGRID_REC_REAL)
         CM_MK(MK_AGRID_REC_RANDOM)
         CM_MK(MK_ATOMS_FILTER)

@@ -76,8 +76,9 @@ def system_desc(
     real-pass schedule of the molecule layout (speed only); ``atoms_grid``
     (ATOMS layout, one solute molecule, FP32) sets the fine cells per
     search-cell axis of the per-frame candidate grid (1-6; 0 = fine cells of
-    about 2.5 A for dense solutes, the walk for sparse ones; -1 = no grid,
-    every query walks the stencil; speed only) and
+    about 4.5 A when at least 8 solvent sites are asked per solute atom and
+    frame, the walk otherwise; -1 = no grid, every query walks the stencil;
+    speed only) and
     ``atoms_grid_capacity`` its list entries per frame (0 = sized by the
     engine; a frame whose lists do not fit walks the stencil)."""
     d = N.cm_system_desc()

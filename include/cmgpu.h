@@ -136,9 +136,9 @@ typedef struct cm_system_desc {
                                          not depend on it */
     int32_t atoms_grid;               /* ATOMS layout with one solute molecule, FP32 search: fine cells per
                                          search-cell axis of the per-frame candidate grid (1-6; 0 = a grid of
-                                         fine cells of about 2.5 A for dense solutes, the stencil walk for
-                                         sparse ones; -1 = no grid, every query walks the stencil).  The
-                                         counts do not depend on it */
+                                         fine cells of about 4.5 A when at least 8 solvent sites are asked per
+                                         solute atom and frame, the stencil walk otherwise; -1 = no grid, every
+                                         query walks the stencil).  The counts do not depend on it */
     int32_t atoms_grid_capacity;      /* list entries per frame of that grid; 0 = sized by the engine.  A frame
                                          whose lists do not fit walks the stencil instead, so the counts do
                                          not depend on it (a small value only exercises that path) */

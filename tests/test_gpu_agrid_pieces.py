@@ -12,11 +12,11 @@ from test_gpu_agrid import chain_system
 
 pytestmark = pytest.mark.gpu
 
-# under a budget a piece is 61 samples for three-site molecules and 44 for one-site ones
+# under a budget a piece is 58 samples for three-site molecules and 41 for one-site ones
 BUDGET = 4 << 30
 
 
-@pytest.mark.parametrize("apv,samples", [(3, 30), (3, 31), (3, 61), (3, 62), (1, 44), (1, 50)])
+@pytest.mark.parametrize("apv,samples", [(3, 29), (3, 30), (3, 58), (3, 59), (1, 41), (1, 50)])
 @pytest.mark.parametrize("H", [ORTHO, TRICLINIC], ids=["ortho", "triclinic"])
 def test_pieces_match_oracle(cm, orc, gpu_ready, apv, samples, H):
     rng = np.random.default_rng(31)
@@ -61,3 +61,19 @@ def test_fused_batch_of_different_piece_counts(cm, gpu_ready):
             assert np.array_equal(got[k], ref[k]), k
         assert got["md_random"].sum() > 0
         e.close()
+
+
+@pytest.mark.parametrize("apv,mv,aps", [(4, 120, 200), (5, 120, 200), (14, 60, 300), (32, 20, 150)])
+def test_default_grid_of_larger_solvent_molecules(cm, orc, gpu_ready, apv, mv, aps):
+    """Four lanes a query from five sites on (one below), by the default rule,
+    against the oracle and with far fewer atom pairs than the walk."""
+    rng = np.random.default_rng(34)
+    H = np.diag([40.0, 38.0, 42.0])
+    xs, xv, cells = chain_system(rng, H, n=aps, nframes=3, mv=mv, apv=apv, spread=1.2)
+    opt = dict(irefatom=2, cutoff=6.0, dbulk=6.0, usecutoff=False, n_random_samples=20, binstep=0.01, nbins=600, seed=97)
+    evals = {}
+    for grid in (0, -1):
+        got, ref, st = compare(cm, orc, ms=1, aps=aps, mv=mv, apv=apv, xs=xs, xv=xv, cells=cells, self_mode=False,
+                               precision="fp32", regime="atoms", engine_kw=dict(atoms_grid=grid), **opt)
+        evals[grid] = st["atom_pairs_evaluated"]
+    assert ref["md_random"].sum() > 0 and evals[0] < evals[-1]
