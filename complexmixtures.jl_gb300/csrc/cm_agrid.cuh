@@ -615,7 +615,7 @@ __device__ __forceinline__ DirRec agrid_record(int gl, bool active, const DevSys
                                                const FrameScratch &F, int f, int v, int sample, const int *vc,
                                                const float4 *vq, const Top2 &T, LocalStats &st) {
     const Guard &g = F.g;
-    const float band = g.two_delta + 1e-3f * (1.0f + (float)S.cut);
+    const float band = g.list_band;
     const int64_t vb = (int64_t)v * S.apv;
     ExactMol X;
     if (active) {
@@ -698,7 +698,7 @@ __device__ __forceinline__ bool agrid_top2(int gl, bool active, const DevSys &S,
                                            const int *vc, const float4 *vq, Top2 &T, long long &ev) {
     top2_init(T);
     ev = 0;
-    const float band = F.g.two_delta + 1e-3f * (1.0f + (float)S.cut);
+    const float band = F.g.list_band;
     const int apv = active ? S.apv : 0;
     for (int b = 0; b < apv; ++b) agrid_query<GL>(gl, B, G, F, f, vc[b], vq[b], b, b == S.iref, band, T, ev);
     if (GL > 1) {

@@ -13,31 +13,39 @@
 // Each batch of up to 32 candidates is expanded into its atoms; an atom
 // farther than cutoff + solute radius from the solute centroid cannot hold a
 // pair within the cutoff and is dropped.  The remaining atoms are evaluated 32
-// at a time, one per lane, against the solute atoms in shared memory, and the
-// lanes fold their results into per-candidate slots with shared-memory atomics:
-//   k1  (d^2 bits << 32 | a << 8 | b): the closest pair and its atoms,
-//   m2  the second-smallest d^2 over all pairs (top-2 by displacement:
-//       old = atomicMin(k1, key); atomicMin(m2, max(old, d^2)), together with
-//       each lane's own second-smallest),
+// at a time, one per lane, against the solute atoms in shared memory (two
+// solute atoms per instruction), and the lanes fold their rows into
+// per-candidate slots with shared-memory atomics:
+//   k1  the smallest row (d^2 bits, the solvent atom in the lowest five),
+//   m2  the second-smallest row (by displacement: old = atomicMin(k1, key);
+//       atomicMin(m2, max(old, key))),
 //   r1  d^2 of the solvent molecule's reference atom to the closest solute atom,
 //   r2  (self) d^2 of the solute molecule's reference atom to the closest atom
 //       of the solvent molecule.
-// Lane c then decides candidate c: records inside the guard band of the
-// cutoff, of a bin edge or of dbulk, or with a second-closest pair within
-// 2 delta of the closest, go to the guard queue for the exact FP64 rules.
+// Lane c then goes through candidate c's winning row again for the solute
+// atom and the second-smallest distance, and decides: records inside the
+// guard band of the cutoff, of a bin edge or of dbulk, or with a
+// second-closest pair within 2 delta of the closest, go to the guard queue
+// for the exact FP64 rules.
+//
+// On 10,000 14-atom molecules (cutoff 10 A, 64 frames) the tiled real pass
+// took 10,220 us with 64-bit keys that carried the solute atom through every
+// row (eleven operations a pair), 8,000 us so; its counters: 61 % issue, 74 %
+// of the L1 port (gathers of the candidates' atoms and the shared-memory
+// traffic of the queues).
 #pragma once
 #include "cm_kernels.cuh"
 
 namespace cmk {
 
-// One CTA of 32 warps per SM at 64 registers: the SM's 32 warps share one
-// privatised histogram (measured 3.8% faster on config 3 than 2 CTAs of 16
-// warps, each zeroing and flushing its own histogram).
+// Two CTAs of 12 warps per SM at 80 registers.  At 64 registers (one CTA of 32
+// warps) the batch spills 170 bytes: 174 us instead of 130 on 181 14-atom
+// molecules in 19,338 waters, 20 frames; three CTAs of 8 warps 132.
 #ifndef CM_FLAT_WARPS
-#define CM_FLAT_WARPS 32
+#define CM_FLAT_WARPS 12
 #endif
 #ifndef CM_FLAT_MIN_CTAS
-#define CM_FLAT_MIN_CTAS 1
+#define CM_FLAT_MIN_CTAS 2
 #endif
 constexpr int kFlatWarps = CM_FLAT_WARPS;  // warps per CTA
 constexpr int kAtomQueue = 64;   // per-warp atom queue (float4: t, tag)
@@ -45,155 +53,143 @@ constexpr int kAtomQueue = 64;   // per-warp atom queue (float4: t, tag)
 // The 32 candidates' fold slots, one array per field: the lanes of a flush
 // hold different candidates, and their atomics then fall on distinct banks.
 struct CandSlots {
-    unsigned long long k1[32];
-    unsigned int m2[32], r1[32], r2[32];
+    unsigned int k1[32], m2[32], r1[32], r2[32];
 };
 
-constexpr unsigned long long kNoPair = (0x7f800000ull << 32) | 0xffffffffull;  // +inf, largest index
+constexpr unsigned kNoRow = 0xffffffffu;
+constexpr unsigned kRowBits = 31u;  // the low bits of a row's key hold the solvent atom (kMaxSmallMol = 32)
 
 // Shared memory of one warp after the histograms.
 struct FlatWarpSmem {
-    float4 os[kMaxSmallMol];      // solute atom offsets (x, y, z)
-    float4 aq[kAtomQueue];        // atom queue: t = position relative to the solute centroid, w = tag c << 8 | b
-    float4 cq[kQueue];            // candidate queue: D = centroid displacement, w = molecule index
-    int cc[kQueue];               // candidate queue: packed cell offset
+    float4 oxy[kMaxSmallMol / 2];  // solute atom offsets, negated, two atoms (a, a + 1): -x, -x', -y, -y'
+    float2 oz[kMaxSmallMol / 2];   // -z, -z'
+    float4 oref;                   // the reference atom's offset, negated
+    float4 aq[kAtomQueue];         // atom queue (circular): t = position relative to the solute centroid, w = tag c << 8 | b
+    float4 cq[kQueue];             // candidate queue: D = centroid displacement, w = molecule index
+    int cc[kQueue];                // candidate queue: packed cell offset | 1 << 31: may be sampled
     CandSlots cand;
 };
 
 __host__ __device__ constexpr size_t flat_warp_smem() { return sizeof(FlatWarpSmem); }
 
-// Top-2 of the squared distances of one solvent atom t to solute atoms
-// [a0, a1) with step 2 (two independent chains per lane).
-__device__ __forceinline__ void top2_step(const float4 &e, const float4 &oa, int a, float &m1, float &m2, int &k1) {
-    const float dx = e.x - oa.x, dy = e.y - oa.y, dz = e.z - oa.z;
-    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-    m2 = fminf(m2, fmaxf(m1, d2));
-    k1 = d2 < m1 ? a : k1;
-    m1 = fminf(m1, d2);
+// Two FP32 operations per instruction (each IEEE round to nearest, as the
+// scalar ones).
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
-// Evaluate the first n queued atoms (one per lane) and fold them into the
-// candidate slots.  APS > 0 is the compile-time solute molecule size.
-template <bool SELF, int APS>
-__device__ __forceinline__ void flat_flush(const DevSys &S, FlatWarpSmem &W, int n, int lane, LocalStats &st) {
+// The solute molecule's offsets into the warp's shared memory (negated pairs;
+// the odd atom's partner lies beyond every cutoff).
+__device__ __forceinline__ void load_solute(FlatWarpSmem &W, const float4 *so, int aps, int iref, int lane) {
+    for (int i = lane; 2 * i < aps; i += 32) {
+        const float4 u = so[2 * i];
+        const float4 v = 2 * i + 1 < aps ? so[2 * i + 1] : make_float4(-1e18f, -1e18f, -1e18f, 0.f);
+        W.oxy[i] = make_float4(-u.x, -v.x, -u.y, -v.y);
+        W.oz[i] = make_float2(-u.z, -v.z);
+        if (iref >> 1 == i) W.oref = iref & 1 ? make_float4(-v.x, -v.y, -v.z, 0.f) : make_float4(-u.x, -u.y, -u.z, 0.f);
+    }
+}
+
+// Squared distances of t to the two solute atoms of pair i.
+struct T2 {
+    unsigned long long x, y, z;
+};
+__device__ __forceinline__ unsigned long long d2_pair(const FlatWarpSmem &W, const T2 &t, int i) {
+    const float4 xy = W.oxy[i];
+    const float2 z = W.oz[i];
+    const unsigned long long ex = add2(t.x, pack2(xy.x, xy.y)), ey = add2(t.y, pack2(xy.z, xy.w)),
+                             ez = add2(t.z, pack2(z.x, z.y));
+    return fma2(ez, ez, fma2(ey, ey, mul2(ex, ex)));
+}
+
+// Evaluate n queued atoms from `head` on (one per lane): each lane's smallest
+// squared distance to the solute atoms, its row, is folded into its
+// candidate's slots.  k1 keeps the smallest row and m2 the second-smallest, as
+// the row's bits with the solvent atom in the five lowest: a lower bound of
+// the row, 2^-18 below it at most.  Which solute atom it was, and the
+// second-smallest distance inside the row, is left to the candidate's winning
+// row (flat_decide), so the loop is three packed operations and a minimum per
+// atom pair.  APS > 0 is the compile-time solute molecule size.
+template <bool SELF, int APS, bool IMAGES>
+__device__ __forceinline__ void flat_flush(const DevSys &S, FlatWarpSmem &W, int head, int n, int lane, LocalStats &st) {
     if (lane < n) {
-        const float4 e = W.aq[lane];
+        const float4 e = W.aq[(head + lane) & (kAtomQueue - 1)];
         const int tag = __float_as_int(e.w);
         const int c = tag >> 8, b = tag & 0xff;
-        float m1a = INFINITY, m2a = INFINITY, m1b = INFINITY, m2b = INFINITY;
-        int k1a = 0, k1b = 0;
+        const T2 t{pack2(e.x, e.x), pack2(e.y, e.y), pack2(e.z, e.z)};
+        float ma = INFINITY, mb = INFINITY;
         const int aps = APS > 0 ? APS : S.aps;
         if (APS > 0) {
-            // fully unrolled for small molecules; two pairs of steps per
-            // iteration otherwise, so the solute atoms are not all held live
-#pragma unroll(APS <= 6 ? 3 : 2)
-            for (int a = 0; a + 1 < APS; a += 2) {
-                top2_step(e, W.os[a], a, m1a, m2a, k1a);
-                top2_step(e, W.os[a + 1], a + 1, m1b, m2b, k1b);
+#pragma unroll
+            for (int i = 0; i < (APS + 1) / 2; ++i) {
+                float lo, hi;
+                unpack2(d2_pair(W, t, i), lo, hi);
+                ma = fminf(ma, lo);
+                mb = fminf(mb, hi);
             }
-            if (APS & 1) top2_step(e, W.os[APS - 1], APS - 1, m1a, m2a, k1a);
         } else {
-            int a = 0;
-#pragma unroll 1
-            for (; a + 1 < aps; a += 2) {
-                top2_step(e, W.os[a], a, m1a, m2a, k1a);
-                top2_step(e, W.os[a + 1], a + 1, m1b, m2b, k1b);
+#pragma unroll 2
+            for (int i = 0; 2 * i < aps; ++i) {
+                float lo, hi;
+                unpack2(d2_pair(W, t, i), lo, hi);
+                ma = fminf(ma, lo);
+                mb = fminf(mb, hi);
             }
-            if (a < aps) top2_step(e, W.os[a], a, m1a, m2a, k1a);
         }
-        // merge the two chains (equal minima leave m2 == m1, which the guard catches)
-        const float m1 = fminf(m1a, m1b);
-        const float m2 = fminf(fmaxf(m1a, m1b), fminf(m2a, m2b));
-        const int k1 = m1b < m1a ? k1b : k1a;
+        const unsigned row = __float_as_uint(fminf(ma, mb));
         st.atompairs += (unsigned long long)aps;
         CandSlots &C = W.cand;
-        const unsigned long long key = ((unsigned long long)__float_as_uint(m1) << 32) | (unsigned)(k1 << 8 | b);
-        const unsigned long long old = atomicMin(&C.k1[c], key);
-        const float displaced = fmaxf(m1, __uint_as_float((unsigned)(old >> 32)));
-        atomicMin(&C.m2[c], __float_as_uint(fminf(displaced, m2)));
-        if (b == S.iref) C.r1[c] = __float_as_uint(m1);
+        const unsigned key = (row & ~kRowBits) | (unsigned)b;
+        const unsigned old = atomicMin(&C.k1[c], key);
+        atomicMin(&C.m2[c], max(old, key));
+        if (b == S.iref) {
+            if (IMAGES) atomicMin(&C.r1[c], row);  // a row per image
+            else C.r1[c] = row;
+        }
         if (SELF) {
-            const float4 oi = W.os[S.iref];
-            const float dx = e.x - oi.x, dy = e.y - oi.y, dz = e.z - oi.z;
+            const float4 o = W.oref;
+            const float dx = e.x + o.x, dy = e.y + o.y, dz = e.z + o.z;
             atomicMin(&C.r2[c], __float_as_uint(fmaf(dz, dz, fmaf(dy, dy, dx * dx))));
         }
     }
     __syncwarp();
 }
 
-// One batch: the first nc (<= 32) entries of the warp's candidate queue.
-// Expansion runs one lane per (candidate, atom) in atom-major order, so the
-// lanes of one flush hold atoms of different candidates and their
-// shared-memory atomics rarely meet on one slot; then lane c decides
-// candidate c.
-template <bool SELF, int APS>
-__device__ __forceinline__ void flat_batch(const DevSys &S, const Bufs &B, const SHist &h, FlatWarpSmem &W,
-                                           const PairsFrame &Pf, const Guard &g, int f, int s, int sslot, float rs2,
-                                           int lane, int nc, LocalStats &st) {
-    if (lane < nc) {
-        CandSlots &C = W.cand;
-        C.k1[lane] = kNoPair;
-        C.m2[lane] = 0x7f800000u;
-        C.r1[lane] = 0x7f800000u;
-        C.r2[lane] = 0x7f800000u;
-    }
-    __syncwarp();
-    const int apv = S.apv;
-    const float inv_nc = 1.0f / (float)nc;
-    const int total = nc * apv;
-    int nq = 0;
-    for (int base = 0; base < total; base += 64) {
-        // two rounds of 32 (candidate, atom) entries; their loads are independent
-        bool keep[2];
-        float4 t[2];
-        int tag[2];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int i = base + 32 * r + lane;
-            const bool in = i < total;
-            // b = i / nc, exact for i < 2^16: (i + 0.5) / nc stays within half of 1/nc of the quotient
-            const int b = in ? (int)((float(i) + 0.5f) * inv_nc) : 0;
-            const int c = in ? i - b * nc : 0;
-            const float4 D = W.cq[c];
-            float4 ob = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (in) ob = Pf.vo32[(int64_t)__float_as_int(D.w) * apv + b];
-            t[r] = make_float4(D.x + ob.x, D.y + ob.y, D.z + ob.z, 0.f);
-            keep[r] = in && fmaf(t[r].z, t[r].z, fmaf(t[r].y, t[r].y, t[r].x * t[r].x)) <= rs2;
-            tag[r] = c << 8 | b;
-        }
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const unsigned mask = __ballot_sync(0xffffffffu, keep[r]);
-            if (keep[r]) W.aq[nq + __popc(mask & ((1u << lane) - 1u))] = make_float4(t[r].x, t[r].y, t[r].z, __int_as_float(tag[r]));
-            nq += __popc(mask);
-            if (nq >= 32) {
-                __syncwarp();
-                flat_flush<SELF, APS>(S, W, 32, lane, st);
-                float4 rest = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (lane < nq - 32) rest = W.aq[32 + lane];
-                __syncwarp();
-                if (lane < nq - 32) W.aq[lane] = rest;
-                nq -= 32;
-                __syncwarp();
-            }
-        }
-    }
-    __syncwarp();
-    if (nq > 0) flat_flush<SELF, APS>(S, W, nq, lane, st);
-    if (lane >= nc) return;
-    st.molpairs++;
-    const CandSlots &C = W.cand;
-    const unsigned long long k1 = C.k1[lane];
-    if (k1 == kNoPair) return;
-    const float m1 = __uint_as_float((unsigned)(k1 >> 32));
+// The record of a molecule pair from its FP32 pass: the smallest squared
+// distance m1 and its atoms (a1, b1), the second-smallest m2, the solvent
+// reference atom's row r1 and (self) the solute reference atom's column r2.
+// sslot: the solute molecule's row of the bulk flags, -1 if it is not sampled;
+// vsampled: (self) the solvent molecule may be sampled.
+template <bool SELF>
+__device__ __forceinline__ void decide_pair(const DevSys &S, const Bufs &B, const SHist &h, const PairsFrame &Pf,
+                                            const Guard &g, int f, int s, int sslot, bool vsampled, int v, int code, float m1, float m2,
+                                            int a1, int b1, float r1, float r2, LocalStats &st) {
     if (m1 > g.cutp2) return;  // no atom pair within the cutoff
-    const int v = __float_as_int(W.cq[lane].w), code = W.cc[lane];
-    const int a1 = (int)((unsigned)k1 >> 8) & 0xff, b1 = (int)(k1 & 0xff);
-    const float m2 = __uint_as_float(C.m2[lane]), r1 = __uint_as_float(C.r1[lane]), r2 = __uint_as_float(C.r2[lane]);
     const float dmin = sqrtf(m1);
     // hard: the closest pair, or the cutoff or dbulk decision, needs the full
     // FP64 rules (guard queue)
-    bool hard = m1 >= g.cutm2 || (sqrtf(m2) - dmin) <= g.two_delta;
+    const float d2nd = __fadd_ru(dmin, g.two_delta);
+    bool hard = m1 >= g.cutm2 || m2 <= __fmul_ru(d2nd, d2nd);
     if (S.usecutoff) hard = hard || (dmin >= g.dbulk_lo && dmin <= g.dbulk_hi);
     if (hard) {
         // past the capacity the record is dropped and k_queue_check has the
@@ -228,18 +224,243 @@ __device__ __forceinline__ void flat_batch(const DevSys &S, const Bufs &B, const
     }
     const int bulk = S.usecutoff ? (dmin > g.dbulk_hi) : 0;
     if (SELF) {
-        apply_pair_self(S, h, bin, a1, (int64_t)s * S.aps + a1, b1, (int64_t)v * apv + b1, rb1 >= 0, rb1, rb2 >= 0, rb2);
+        apply_pair_self(S, h, bin, a1, (int64_t)s * S.aps + a1, b1, (int64_t)v * S.apv + b1, rb1 >= 0, rb1, rb2 >= 0, rb2);
         st.hits += 2;
     } else {
-        apply_hit_local(S, h, false, bin, a1, (int64_t)v * apv + b1, b1, rb1 >= 0, rb1);
+        apply_hit_local(S, h, false, bin, a1, (int64_t)v * S.apv + b1, b1, rb1 >= 0, rb1);
         st.hits++;
     }
     if (Pf.slot) {
         const unsigned char code1 = (unsigned char)(1 + bulk);
         if (sslot >= 0) Pf.flags[(int64_t)sslot * S.mv + v] = code1;
-        if (SELF) {
+        if (SELF && vsampled) {
             const int vs = Pf.slot[v];
             if (vs >= 0) Pf.flags[(int64_t)vs * S.mv + s] = code1;
+        }
+    }
+}
+
+__device__ __forceinline__ void cand_slots_clear(CandSlots &C, int lane) {
+    C.k1[lane] = kNoRow;
+    C.m2[lane] = kNoRow;
+    C.r1[lane] = 0x7f800000u;
+    C.r2[lane] = 0x7f800000u;
+}
+
+// The atoms of the first nc (<= 32) entries of the warp's candidate queue
+// against the solute.  An entry folds into the slot of its place in the queue
+// or (IMAGES) into the slot W.cc names.  The expansion takes two adjacent
+// atoms of every entry at a time: one 32-byte sector per load and entry (the
+// gathers through the SM's L1 port weigh most), and the lanes of one flush
+// hold at most two atoms of an entry, so their shared-memory atomics rarely
+// meet on one slot.
+template <bool SELF, int APS, bool IMAGES>
+__device__ __forceinline__ void flat_expand(const DevSys &S, FlatWarpSmem &W, const PairsFrame &Pf, float rs2, int lane, int nc,
+                                            LocalStats &st) {
+    const int apv = S.apv;
+    // 2^sh lanes per entry: two in a full batch, whose entries go in two halves
+    // (the lanes of entry i, then of 16 + i), more in a short one
+    const bool two = nc > 16;
+    const int sh = two ? 1 : max(1, min(5, __clz(nc - 1) - 27));
+    const int ci = lane >> sh, sub = lane & ((1 << sh) - 1);
+    const int i0 = ci < nc ? ci : 0, i1 = two && 16 + ci < nc ? 16 + ci : 0;
+    const float4 D0 = W.cq[i0], D1 = W.cq[i1];
+    const int s0 = IMAGES ? W.cc[i0] : ci, s1 = IMAGES ? W.cc[i1] : 16 + ci;
+    const float4 *o0 = Pf.vo32 + (int64_t)__float_as_int(D0.w) * apv, *o1 = Pf.vo32 + (int64_t)__float_as_int(D1.w) * apv;
+    int head = 0, nq = 0;
+    auto queue = [&](const float4 &t, bool keep) {
+        const unsigned mask = __ballot_sync(0xffffffffu, keep);
+        if (keep) W.aq[(head + nq + __popc(mask & ((1u << lane) - 1u))) & (kAtomQueue - 1)] = t;
+        nq += __popc(mask);
+        if (nq >= 32) {
+            __syncwarp();
+            flat_flush<SELF, APS, IMAGES>(S, W, head, 32, lane, st);
+            head += 32;
+            nq -= 32;
+        }
+    };
+    for (int b0 = 0; b0 < apv; b0 += 1 << sh) {
+        const int b = b0 + sub;
+        const int bl = b < apv ? b : b0;
+        const float4 oa = o0[bl];
+        float4 ob = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (two) ob = o1[bl];
+        const float4 t0 = make_float4(D0.x + oa.x, D0.y + oa.y, D0.z + oa.z, __int_as_float(s0 << 8 | b));
+        queue(t0, ci < nc && b < apv && fmaf(t0.z, t0.z, fmaf(t0.y, t0.y, t0.x * t0.x)) <= rs2);
+        if (two) {
+            const float4 t1 = make_float4(D1.x + ob.x, D1.y + ob.y, D1.z + ob.z, __int_as_float(s1 << 8 | b));
+            queue(t1, 16 + ci < nc && b < apv && fmaf(t1.z, t1.z, fmaf(t1.y, t1.y, t1.x * t1.x)) <= rs2);
+        }
+    }
+    __syncwarp();
+    if (nq > 0) flat_flush<SELF, APS, IMAGES>(S, W, head, nq, lane, st);
+}
+
+// The winning row of a slot again, against every solute atom: the smallest
+// distance of t with its atom, and the second-smallest.
+template <int APS>
+__device__ __forceinline__ void winning_row(const DevSys &S, const FlatWarpSmem &W, float tx, float ty, float tz, float &m1,
+                                            float &m2, int &a1) {
+    const T2 t{pack2(tx, tx), pack2(ty, ty), pack2(tz, tz)};
+    const int aps = APS > 0 ? APS : S.aps;
+#pragma unroll 2
+    for (int i = 0; 2 * i < aps; ++i) {
+        float lo, hi;
+        unpack2(d2_pair(W, t, i), lo, hi);
+        m2 = fminf(m2, fmaxf(m1, lo));
+        a1 = lo < m1 ? 2 * i : a1;
+        m1 = fminf(m1, lo);
+        m2 = fminf(m2, fmaxf(m1, hi));
+        a1 = hi < m1 ? 2 * i + 1 : a1;
+        m1 = fminf(m1, hi);
+    }
+}
+
+// One batch: the first nc (<= 32) entries of the warp's candidate queue, lane
+// c candidate c.  After the expansion lane c goes through its candidate's
+// winning row again, for the solute atom and the second-smallest distance in
+// it, and decides.  A row whose key is not the smallest although its distance
+// is (keys are truncated) leaves m2 at most its distance, which makes the
+// record hard, so the winning row is the right one wherever it is used.
+template <bool SELF, int APS>
+__device__ __forceinline__ void flat_batch(const DevSys &S, const Bufs &B, const SHist &h, FlatWarpSmem &W,
+                                           const PairsFrame &Pf, const Guard &g, int f, int s, int sslot, float rs2,
+                                           int lane, int nc, LocalStats &st) {
+    CandSlots &C = W.cand;
+    cand_slots_clear(C, lane);
+    __syncwarp();
+    flat_expand<SELF, APS, false>(S, W, Pf, rs2, lane, nc, st);
+    if (lane >= nc) return;
+    st.molpairs++;
+    const unsigned k1 = C.k1[lane];
+    // no row, or (the key is a lower bound) no atom pair within the cutoff
+    if (k1 == kNoRow || __uint_as_float(k1 & ~kRowBits) > g.cutp2) return;
+    const int b1 = (int)(k1 & kRowBits);
+    const float4 D = W.cq[lane];
+    const int v = __float_as_int(D.w);
+    const float4 ob = Pf.vo32[(int64_t)v * S.apv + b1];
+    float m1 = INFINITY, m2 = C.m2[lane] == kNoRow ? INFINITY : __uint_as_float(C.m2[lane] & ~kRowBits);
+    int a1 = 0;
+    winning_row<APS>(S, W, D.x + ob.x, D.y + ob.y, D.z + ob.z, m1, m2, a1);
+    const int cc = W.cc[lane];
+    decide_pair<SELF>(S, B, h, Pf, g, f, s, sslot, cc < 0, v, cc & 0x7fffffff, m1, m2, a1, b1, __uint_as_float(C.r1[lane]),
+                      __uint_as_float(C.r2[lane]), st);
+}
+
+__device__ __forceinline__ void image_at(const Images &im, int img, int &dx, int &dy, int &dz) {
+    const int ix = img % im.cnt[0], iy = (img / im.cnt[0]) % im.cnt[1], iz = img / (im.cnt[0] * im.cnt[1]);
+    dx = im.base[0] + ix * im.step[0];
+    dy = im.base[1] + iy * im.step[1];
+    dz = im.base[2] + iz * im.step[2];
+}
+
+// One solute molecule of a frame that needs several images per molecule pair
+// (a box of less than three search cells along an axis): 32 molecules of a
+// cell at a time, lane c molecule c.  An image whose molecule's bounding sphere
+// reaches the solute's is an entry of the queue and folds into its molecule's
+// slot, so the slots end with the values over all images.  (The generic
+// kernel evaluates every atom pair of every image, one lane per molecule: 300
+// 9-atom molecules in a 30 A box, cutoff 9 A, 16 frames: 5,473 us a pass with the
+// generic kernel, 1,048 with this one.)
+template <bool SELF, int APS>
+__device__ __forceinline__ void flat_images(const DevSys &S, const Bufs &B, const SHist &h, FlatWarpSmem &W,
+                                            const PairsFrame &Pf, const Guard &g, int f, int s, int sslot, const float4 qs,
+                                            int sc, float rsc, int part, int parts, int lane, LocalStats &st) {
+    const FrameGeom &G = *Pf.G;
+    const FrameScratch &F = *Pf.F;
+    CandSlots &C = W.cand;
+    const unsigned below = (1u << lane) - 1u;
+    const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
+    const bool m0 = F.multi & 1, m1 = F.multi & 2, m2 = F.multi & 4;
+    const int e0 = m0 ? n0 : 2 * F.L[0] + 1, e1 = m1 ? n1 : 2 * F.L[1] + 1, e2 = m2 ? n2 : 2 * F.L[2] + 1;
+    const int cx = sc % n0, cy = (sc / n0) % n1, cz = sc / (n0 * n1);
+    const float rs2 = rsc * rsc;
+    const float4 *cq32 = B.cq32 + (int64_t)f * B.mv;
+    for (int ic = part; ic < e0 * e1 * e2; ic += parts) {
+        const int ix = ic % e0, iy = (ic / e0) % e1, iz = ic / (e0 * e1);
+        const int dx = m0 ? ix - cx : ix - F.L[0], dy = m1 ? iy - cy : iy - F.L[1], dz = m2 ? iz - cz : iz - F.L[2];
+        const int xc = m0 ? ix : wrap_cell(cx + dx, n0), yc = m1 ? iy : wrap_cell(cy + dy, n1),
+                  zc = m2 ? iz : wrap_cell(cz + dz, n2);
+        const int cell = (zc * n1 + yc) * n0 + xc;
+        const int beg = Pf.cstart[cell], end = Pf.cstart[cell + 1];
+        const int code = pack_delta(dx, dy, dz);
+        const Images im = images_of(G, F, code);
+        const int ni = image_count(im);
+        for (int p0 = beg; p0 < end; p0 += 32) {
+            const int p = min(p0 + lane, end - 1);
+            const float4 q = cq32[p];
+            const int v = Pf.cmol[p];
+            const bool valid = p0 + lane < end && (!SELF || v > s);
+            const float R = rsc + q.w;
+            const float bx = q.x - qs.x, by = q.y - qs.y, bz = q.z - qs.z;
+            cand_slots_clear(C, lane);
+            __syncwarp();
+            int cnt = 0;
+            unsigned mine = 0;  // the lane's images in reach, of the first 32
+            for (int i = 0; i < ni; ++i) {
+                int jx, jy, jz;
+                image_at(im, i, jx, jy, jz);
+                const float4 o = Pf.off32[off_index(jx, jy, jz)];
+                const float Dx = bx + o.x, Dy = by + o.y, Dz = bz + o.z;
+                const bool in = valid && fmaf(Dz, Dz, fmaf(Dy, Dy, Dx * Dx)) <= R * R;
+                const unsigned mask = __ballot_sync(0xffffffffu, in);
+                if (in) {
+                    const int pos = cnt + __popc(mask & below);
+                    W.cq[pos] = make_float4(Dx, Dy, Dz, __int_as_float(v));
+                    W.cc[pos] = lane;
+                    if (i < 32) mine |= 1u << i;
+                }
+                cnt += __popc(mask);
+                if (cnt >= 32) {
+                    __syncwarp();
+                    flat_expand<SELF, APS, true>(S, W, Pf, rs2, lane, 32, st);
+                    __syncwarp();
+                    cnt -= 32;
+                    float4 rq = make_float4(0.f, 0.f, 0.f, 0.f);
+                    int rc = 0;
+                    if (lane < cnt) {
+                        rq = W.cq[32 + lane];
+                        rc = W.cc[32 + lane];
+                    }
+                    __syncwarp();
+                    if (lane < cnt) {
+                        W.cq[lane] = rq;
+                        W.cc[lane] = rc;
+                    }
+                    __syncwarp();
+                }
+            }
+            __syncwarp();
+            if (cnt > 0) flat_expand<SELF, APS, true>(S, W, Pf, rs2, lane, cnt, st);
+            __syncwarp();
+            if (valid) st.molpairs++;
+            const unsigned k1 = C.k1[lane];
+            if (valid && k1 != kNoRow && !(__uint_as_float(k1 & ~kRowBits) > g.cutp2)) {
+                const int b1 = (int)(k1 & kRowBits);
+                const float4 ob = Pf.vo32[(int64_t)v * S.apv + b1];
+                float d1 = INFINITY, d2 = C.m2[lane] == kNoRow ? INFINITY : __uint_as_float(C.m2[lane] & ~kRowBits);
+                int a1 = 0;
+                // the winning atom's row in every image it was evaluated in: m2 already holds all but the smallest,
+                // truncated, and those found here again only confirm it
+                float e1 = INFINITY, e2 = INFINITY;
+                unsigned left = ni > 32 ? 1u : mine;
+                for (int i = 0; left; i += ni > 32) {
+                    const int j = ni > 32 ? i : __ffs(left) - 1;
+                    if (ni > 32) left = i + 1 < ni;
+                    else left &= left - 1;
+                    int jx, jy, jz;
+                    image_at(im, j, jx, jy, jz);
+                    const float4 o = Pf.off32[off_index(jx, jy, jz)];
+                    const float tx = (bx + o.x) + ob.x, ty = (by + o.y) + ob.y, tz = (bz + o.z) + ob.z;
+                    if (!(fmaf(tz, tz, fmaf(ty, ty, tx * tx)) <= rs2)) continue;
+                    winning_row<APS>(S, W, tx, ty, tz, e1, e2, a1);
+                }
+                d1 = e1;
+                d2 = fminf(d2, e2);
+                decide_pair<SELF>(S, B, h, Pf, g, f, s, sslot, true, v, code, d1, d2, a1, b1, __uint_as_float(C.r1[lane]),
+                                  __uint_as_float(C.r2[lane]), st);
+            }
+            __syncwarp();
         }
     }
 }
@@ -273,7 +494,7 @@ __global__ void __launch_bounds__(kFlatWarps * 32, CM_FLAT_MIN_CTAS) k_pairs_fla
             if (lane == 0) raise_err(S, ERR_STENCIL);
             continue;
         }
-        if (F.multi) continue;  // several images per pair: the generic kernel takes the frame
+        if (F.multi) continue;  // several images per pair: k_pairs_images32 takes the frame
         if (skip_tile && F.tile) continue;
         const FrameGeom &G = *Pf.G;
         const Guard g = F.g;
@@ -281,7 +502,7 @@ __global__ void __launch_bounds__(kFlatWarps * 32, CM_FLAT_MIN_CTAS) k_pairs_fla
         const int sc = Pf.scell[s];
         const int sslot = Pf.slot ? Pf.slot[s] : -1;
         __syncwarp();
-        for (int a = lane; a < aps; a += 32) W.os[a] = Pf.so32[(int64_t)s * aps + a];
+        load_solute(W, Pf.so32 + (int64_t)s * aps, aps, S.iref, lane);
         __syncwarp();
         const float rsc = g.cut_pre + qs.w;     // candidate molecules: centroid within rsc + r_v
         const float rs2 = rsc * rsc;            // candidate atoms: within rsc of the solute centroid
@@ -342,7 +563,7 @@ __global__ void __launch_bounds__(kFlatWarps * 32, CM_FLAT_MIN_CTAS) k_pairs_fla
                         const int pos = cnt + __popc(mask & ((1u << lane) - 1u));
                         if (cand) {
                             W.cq[pos] = Dv;
-                            W.cc[pos] = pack_delta(dx, dy, dz);
+                            W.cc[pos] = pack_delta(dx, dy, dz) | 0x80000000;
                         }
                         cnt += __popc(mask);
                         if (cnt >= 32) {
@@ -376,6 +597,43 @@ __global__ void __launch_bounds__(kFlatWarps * 32, CM_FLAT_MIN_CTAS) k_pairs_fla
     shist_flush(S, h, false);
 }
 
+// The frames that need several images per molecule pair, `parts` warps per
+// (frame, solute molecule), each on every parts-th cell; returns at once when
+// the chunk has none.
+template <bool SELF, int APS>
+__global__ void __launch_bounds__(kFlatWarps * 32, CM_FLAT_MIN_CTAS) k_pairs_images32(DevSys S, Bufs B, int parts) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned int *hbase = (unsigned int *)smem_raw;
+    FlatWarpSmem *wsm = (FlatWarpSmem *)(smem_raw + (((size_t)hist_words(S) * 4 + 15) & ~(size_t)15));
+    int any = 0;
+    for (int f = threadIdx.x; f < B.nf; f += blockDim.x) any |= B.FS[f].multi;
+    if (!__syncthreads_or(any)) return;
+    shist_zero(S, hbase);
+    __syncthreads();
+    const SHist h = shist_bind(S, hbase);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    FlatWarpSmem &W = wsm[warp];
+    LocalStats st;
+    const int64_t items = (int64_t)B.nf * B.ms * parts;
+    for (int64_t t = (int64_t)blockIdx.x * kFlatWarps + warp; t < items; t += (int64_t)gridDim.x * kFlatWarps) {
+        const int part = (int)(t % parts);
+        const int f = (int)(t / parts / B.ms), s = (int)(t / parts - (int64_t)f * B.ms);
+        const PairsFrame Pf = pairs_frame(B, f, SELF);
+        const FrameScratch &F = *Pf.F;
+        if (!F.ok || !F.multi) continue;
+        const Guard g = F.g;
+        const float4 qs = Pf.sq32[s];
+        __syncwarp();
+        load_solute(W, Pf.so32 + (int64_t)s * S.aps, S.aps, S.iref, lane);
+        __syncwarp();
+        flat_images<SELF, APS>(S, B, h, W, Pf, g, f, s, Pf.slot ? Pf.slot[s] : -1, qs, Pf.scell[s], g.cut_pre + qs.w, part,
+                               parts, lane, st);
+    }
+    stats_flush(S, st, false);
+    __syncthreads();
+    shist_flush(S, h, false);
+}
+
 // ------------------------------------------------------------ tiled real pass
 // Self mode.  The stencil walk of k_pairs_flat32 gathers each neighbour
 // cell's molecule table from L2 once per solute molecule, one warp per
@@ -398,12 +656,17 @@ __global__ void __launch_bounds__(kFlatWarps * 32, CM_FLAT_MIN_CTAS) k_pairs_fla
 constexpr int kTileWarps = CM_TILE_WARPS;
 constexpr int kTileStage = 1024;  // staged neighbour molecules per pass
 
-struct TileSmem {
-    float4 w[kTileStage];       // staged molecule: centroid + stencil offset (x, y, z), radius
-    int v[kTileStage];          // molecule index | staged cell << 24
+// The half-stencil cells of a home cell.
+struct TileCellTab {
     int nbeg[kTileCells + 1];   // first staged position of each cell (prefix of the cells' molecule counts)
     int cbeg[kTileCells];       // the cell's first position in the cell-sorted molecule table
     int code[kTileCells];       // the cell's packed stencil offset
+};
+
+struct TileSmem {
+    float4 w[kTileStage];       // staged molecule: centroid + stencil offset (x, y, z), half its square
+    int v[kTileStage];          // molecule index | staged cell << 24 | sampled << 31
+    TileCellTab c;
     int next;                   // next home molecule to claim
     int item;                   // the CTA's current (frame, home cell) item
 };
@@ -431,6 +694,61 @@ __device__ __forceinline__ void half_stencil_cell(int k, const int *L, int &dx, 
     dx = r % wx - L[0];
 }
 
+// Fill the cell table of home cell (cx, cy, cz), K <= kTileCells cells; every
+// thread of the CTA calls it (two barriers).
+__device__ __forceinline__ void tile_cells(const FrameGeom &G, const FrameScratch &F, const int *cstart, int cx, int cy,
+                                           int cz, int K, TileCellTab &T) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
+    if (tid < K) {
+        int dx, dy, dz;
+        half_stencil_cell(tid, F.L, dx, dy, dz);
+        const int c = (wrap_cell(cz + dz, n2) * n1 + wrap_cell(cy + dy, n1)) * n0 + wrap_cell(cx + dx, n0);
+        T.cbeg[tid] = cstart[c];
+        T.nbeg[tid + 1] = cstart[c + 1] - cstart[c];
+        T.code[tid] = pack_delta(dx, dy, dz);
+    }
+    if (tid == 0) T.nbeg[0] = 0;
+    __syncthreads();
+    if (tid < 32) {
+        // inclusive prefix of the K <= kTileCells counts, four per lane
+        int c[4], sum = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = 4 * lane + j;
+            c[j] = k < K ? T.nbeg[k + 1] : 0;
+            sum += c[j];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        int run = incl - sum;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = 4 * lane + j;
+            run += c[j];
+            if (k < K) T.nbeg[k + 1] = run;
+        }
+    }
+    __syncthreads();
+}
+
+// Staged molecule m of the table: its cell k and its position in the
+// cell-sorted molecule table.
+__device__ __forceinline__ int tile_molecule(const TileCellTab &T, int K, int m, int &k) {
+    int lo = 0, hi = K;  // the cell with nbeg[k] <= m < nbeg[k + 1]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (T.nbeg[mid] <= m) lo = mid;
+        else hi = mid;
+    }
+    k = lo;
+    return T.cbeg[lo] + (m - T.nbeg[lo]);
+}
+
 template <int APS>
 __global__ void __launch_bounds__(kTileWarps * 32, CM_TILE_MIN_CTAS) k_pairs_tile32(DevSys S, Bufs B) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -442,6 +760,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, CM_TILE_MIN_CTAS) k_pairs_til
     __syncthreads();
     SHist h = shist_bind(S, hbase);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const unsigned below = (1u << lane) - 1u;
     FlatWarpSmem &W = wsm[warp];
     LocalStats st;
     const int aps = S.aps;
@@ -463,69 +782,34 @@ __global__ void __launch_bounds__(kTileWarps * 32, CM_TILE_MIN_CTAS) k_pairs_til
         if (!F.ok || !F.tile || H >= G.ncell) continue;
         const int hbeg = Pf.cstart[H], nH = Pf.cstart[H + 1] - hbeg;
         if (nH == 0) continue;
-        const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
+        const int n0 = G.n[0], n1 = G.n[1];
         const int cx = H % n0, cy = (H / n0) % n1, cz = H / (n0 * n1);
         const int K = (F.L[0] + 1) + (2 * F.L[0] + 1) * F.L[1] + (2 * F.L[0] + 1) * (2 * F.L[1] + 1) * F.L[2];
         const Guard g = F.g;
         const float4 *cq32 = B.cq32 + (int64_t)f * B.mv;
-        if (tid < K) {
-            int dx, dy, dz;
-            half_stencil_cell(tid, F.L, dx, dy, dz);
-            const int c = (wrap_cell(cz + dz, n2) * n1 + wrap_cell(cy + dy, n1)) * n0 + wrap_cell(cx + dx, n0);
-            T.cbeg[tid] = Pf.cstart[c];
-            T.nbeg[tid + 1] = Pf.cstart[c + 1] - Pf.cstart[c];
-            T.code[tid] = pack_delta(dx, dy, dz);
-        }
-        if (tid == 0) T.nbeg[0] = 0;
-        __syncthreads();
-        if (warp == 0) {
-            // inclusive prefix of the K <= kTileCells counts, four per lane
-            int c[4], sum = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int k = 4 * lane + j;
-                c[j] = k < K ? T.nbeg[k + 1] : 0;
-                sum += c[j];
-            }
-            int incl = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += u;
-            }
-            int run = incl - sum;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int k = 4 * lane + j;
-                run += c[j];
-                if (k < K) T.nbeg[k + 1] = run;
-            }
-        }
-        __syncthreads();
-        const int M = T.nbeg[K];
+        tile_cells(G, F, Pf.cstart, cx, cy, cz, K, T.c);
+        const int M = T.c.nbeg[K];
         for (int m0 = 0; m0 < M; m0 += kTileStage) {
-            const int n = min(kTileStage, M - m0);
+            const int n = min(kTileStage, M - m0), nr = (n + 31) & ~31;
             if (m0 > 0) __syncthreads();  // the previous pass's table is no longer read
-            for (int i = tid; i < n; i += blockDim.x) {
-                const int m = m0 + i;
-                int lo = 0, hi = K;  // the cell k with nbeg[k] <= m < nbeg[k + 1]
-                while (hi - lo > 1) {
-                    const int mid = (lo + hi) >> 1;
-                    if (T.nbeg[mid] <= m) lo = mid;
-                    else hi = mid;
+            for (int i = tid; i < nr; i += blockDim.x) {
+                if (i >= n) {
+                    T.w[i] = make_float4(0.f, 0.f, 0.f, INFINITY);  // never a candidate
+                    continue;
                 }
-                int dx, dy, dz;
-                half_stencil_cell(lo, F.L, dx, dy, dz);
+                int k, dx, dy, dz;
+                const int p = tile_molecule(T.c, K, m0 + i, k);
+                half_stencil_cell(k, F.L, dx, dy, dz);
                 const float4 of = Pf.off32[off_index(dx, dy, dz)];
-                const int p = T.cbeg[lo] + (m - T.nbeg[lo]);
                 const float4 q = cq32[p];
-                T.w[i] = make_float4(q.x + of.x, q.y + of.y, q.z + of.z, q.w);
-                T.v[i] = Pf.cmol[p] | (lo << 24);
+                const float x = q.x + of.x, y = q.y + of.y, z = q.z + of.z;
+                T.w[i] = make_float4(x, y, z, 0.5f * fmaf(z, z, fmaf(y, y, x * x)));
+                const int v = Pf.cmol[p];
+                T.v[i] = v | (k << 24) | (Pf.slot && Pf.slot[v] >= 0 ? 0x80000000 : 0);
             }
             if (tid == 0) T.next = 0;
             __syncthreads();
             // the home molecules, claimed one at a time
-            const int own_end = T.nbeg[1] - m0;  // staged positions below this are the home cell (pass 0)
             for (;;) {
                 int sl = 0;
                 if (lane == 0) sl = atomicAdd(&T.next, 1);
@@ -535,50 +819,55 @@ __global__ void __launch_bounds__(kTileWarps * 32, CM_TILE_MIN_CTAS) k_pairs_til
                 const float4 qs = Pf.sq32[s];
                 const int sslot = Pf.slot ? Pf.slot[s] : -1;
                 __syncwarp();
-                for (int a = lane; a < aps; a += 32) W.os[a] = Pf.so32[(int64_t)s * aps + a];
+                load_solute(W, Pf.so32 + (int64_t)s * aps, aps, S.iref, lane);
                 __syncwarp();
                 const float rsc = g.cut_pre + qs.w;
                 const float rs2 = rsc * rsc;
+                const float R = rsc + F.rmax_s;
+                const float thr = 0.5f * (R * R - fmaf(qs.z, qs.z, fmaf(qs.y, qs.y, qs.x * qs.x)));
+                // within the home cell (the first staged positions) only the molecules after this one
+                const int lo = max(0, sl + 1 - m0);
                 int cnt = 0;
-                for (int p0 = 0; p0 < n; p0 += 32) {
-                    const int p = p0 + lane;
-                    const bool in = p < n;
-                    const int pc = in ? p : n - 1;
-                    const float4 w = T.w[pc];
-                    const int vk = T.v[pc];
-                    const int v = vk & 0xffffff;
-                    float4 Dv;
-                    Dv.x = w.x - qs.x;
-                    Dv.y = w.y - qs.y;
-                    Dv.z = w.z - qs.z;
-                    Dv.w = __int_as_float(v);
-                    const float rr = rsc + w.w;
-                    const bool cand = in && fmaf(Dv.z, Dv.z, fmaf(Dv.y, Dv.y, Dv.x * Dv.x)) <= rr * rr &&
-                                      !(p < own_end && v <= s);
-                    const unsigned mask = __ballot_sync(0xffffffffu, cand);
-                    const int pos = cnt + __popc(mask & ((1u << lane) - 1u));
-                    if (cand) {
-                        W.cq[pos] = Dv;
-                        W.cc[pos] = T.code[vk >> 24];
+                for (int base = lo & ~31; base < nr; base += 1024) {
+                    const int nj = min(32, (nr - base) >> 5);
+                    unsigned bits = 0;
+#pragma unroll 4
+                    for (int j = 0; j < nj; ++j) {
+                        const float4 w = T.w[base + 32 * j + lane];
+                        if (fmaf(-w.x, qs.x, fmaf(-w.y, qs.y, fmaf(-w.z, qs.z, w.w))) <= thr) bits |= 1u << j;
                     }
-                    cnt += __popc(mask);
-                    if (cnt >= 32) {
-                        __syncwarp();
-                        flat_batch<true, APS>(S, B, h, W, Pf, g, f, s, sslot, rs2, lane, 32, st);
-                        __syncwarp();
-                        float4 rq = make_float4(0.f, 0.f, 0.f, 0.f);
-                        int rc = 0;
-                        if (lane < cnt - 32) {
-                            rq = W.cq[32 + lane];
-                            rc = W.cc[32 + lane];
+                    if (base + lane < lo) bits &= ~1u;
+                    for (;;) {
+                        const unsigned mask = __ballot_sync(0xffffffffu, bits != 0);
+                        if (mask == 0) break;
+                        if (bits) {
+                            const int p = base + 32 * (__ffs(bits) - 1) + lane;
+                            const int pos = cnt + __popc(mask & below);
+                            const float4 w = T.w[p];
+                            const int vk = T.v[p];
+                            W.cq[pos] = make_float4(w.x - qs.x, w.y - qs.y, w.z - qs.z, __int_as_float(vk & 0xffffff));
+                            W.cc[pos] = T.c.code[(vk >> 24) & 127] | (vk & 0x80000000);
+                            bits &= bits - 1;
                         }
-                        __syncwarp();
-                        if (lane < cnt - 32) {
-                            W.cq[lane] = rq;
-                            W.cc[lane] = rc;
+                        cnt += __popc(mask);
+                        if (cnt >= 32) {
+                            __syncwarp();
+                            flat_batch<true, APS>(S, B, h, W, Pf, g, f, s, sslot, rs2, lane, 32, st);
+                            __syncwarp();
+                            cnt -= 32;
+                            float4 rq = make_float4(0.f, 0.f, 0.f, 0.f);
+                            int rc = 0;
+                            if (lane < cnt) {
+                                rq = W.cq[32 + lane];
+                                rc = W.cc[32 + lane];
+                            }
+                            __syncwarp();
+                            if (lane < cnt) {
+                                W.cq[lane] = rq;
+                                W.cc[lane] = rc;
+                            }
+                            __syncwarp();
                         }
-                        cnt -= 32;
-                        __syncwarp();
                     }
                 }
                 __syncwarp();
@@ -586,6 +875,207 @@ __global__ void __launch_bounds__(kTileWarps * 32, CM_TILE_MIN_CTAS) k_pairs_til
                 __syncwarp();
             }
         }
+    }
+    stats_flush(S, st, false);
+    __syncthreads();
+    shist_flush(S, h, false);
+}
+
+// ----------------------------------------------- tiled real pass, small molecules
+// Self mode, molecules of up to kDirectMax atoms (water).  k_pairs_tile32
+// spends most of its instructions per candidate on expanding it into atoms,
+// on the shared-memory folds and on batches that end with every home molecule
+// (53 candidates of a water at cutoff 10: batches of 32 and 21).  A small
+// molecule's few atom pairs fit one lane's registers, so here a lane takes a
+// whole candidate pair, and the warp's queue holds (home molecule, staged
+// molecule) pairs of any home molecules, so that its batches are full until the
+// staged table changes.  The test of a home molecule against the staged
+// table is |w - q|^2 <= R^2 as |w|^2 / 2 - w q <= (R^2 - |q|^2) / 2, three
+// multiply-adds on a staged (w, |w|^2 / 2), R the reach of the largest
+// molecule of the frame; its rounding (4 u (|w|^2 / 2 + |w| |q|), under 2e-3
+// A^2 for cells of 25 A) is far inside the margin of cut_pre (R times 1e-3 (1 +
+// range), 0.15 A^2 for water).  A lane keeps its hits of up to 32 rounds in a
+// bit mask; the masks are compacted into the queue afterwards.  The distances
+// are formed as in flat_flush, so the records and the queues are the same.
+// 19,338 waters, cutoff 10 A, 16 frames: 1,979 us in k_pairs_tile32, 746 here
+// (12 or 20 warps per CTA: 801, 825); the candidates' decisions and the gathers
+// of their atoms bound it (73 % issue, 69 % of the L1 port).
+#ifndef CM_DIRECT_WARPS
+#define CM_DIRECT_WARPS 16
+#endif
+constexpr int kDirectWarps = CM_DIRECT_WARPS;
+constexpr int kDirectMax = 5;       // atoms per molecule
+constexpr int kDirectStage = 1536;  // staged molecules per pass (a multiple of 32; positions take 11 bits of a queue entry)
+constexpr int kDirectHome = 256;    // home molecules per pass
+
+struct DirectSmem {
+    float4 w[kDirectStage];   // staged molecule: centroid + stencil offset, half its square
+    int v[kDirectStage];      // molecule index | staged cell << 24 | sampled << 31
+    float4 hq[kDirectHome];   // home molecule: centroid, test threshold
+    int hs[kDirectHome];      // its index | sampled << 31
+    int q[kDirectWarps][64];  // the warps' pair queues: staged position | home molecule << 11
+    TileCellTab c;
+    int next;
+    int item;
+};
+
+__host__ __device__ constexpr size_t direct_smem_extra() { return sizeof(DirectSmem) + 16; }
+
+template <int APM>
+__global__ void __launch_bounds__(kDirectWarps * 32, 2) k_pairs_direct32(DevSys S, Bufs B) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned int *hbase = (unsigned int *)smem_raw;
+    DirectSmem &T = *(DirectSmem *)(smem_raw + (((size_t)hist_words(S) * 4 + 15) & ~(size_t)15));
+    shist_zero(S, hbase);
+    __syncthreads();
+    const SHist h = shist_bind(S, hbase);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const unsigned below = (1u << lane) - 1u;
+    int *Q = T.q[warp];
+    LocalStats st;
+    const int64_t ncap = B.cs - 1;
+    const int64_t items = (int64_t)B.nf * ncap;
+    // CTAs claim (frame, home cell) items from counters[6], as k_pairs_tile32
+    for (;;) {
+        __syncthreads();  // the previous item's table and claim are no longer read
+        if (tid == 0) T.item = atomicAdd(B.counters + 6, 1);
+        __syncthreads();
+        const int64_t t = T.item;
+        if (t >= items) break;
+        const int f = (int)(t / ncap), H = (int)(t - (int64_t)f * ncap);
+        const PairsFrame Pf = pairs_frame(B, f, true);
+        const FrameScratch &F = *Pf.F;
+        const FrameGeom &G = *Pf.G;
+        if (!F.ok || !F.tile || H >= G.ncell) continue;
+        const int hbeg = Pf.cstart[H], nH = Pf.cstart[H + 1] - hbeg;
+        if (nH == 0) continue;
+        const int n0 = G.n[0], n1 = G.n[1];
+        const int cx = H % n0, cy = (H / n0) % n1, cz = H / (n0 * n1);
+        const int K = (F.L[0] + 1) + (2 * F.L[0] + 1) * F.L[1] + (2 * F.L[0] + 1) * (2 * F.L[1] + 1) * F.L[2];
+        const Guard g = F.g;
+        const float rmax = F.rmax_s;
+        const float4 *cq32 = B.cq32 + (int64_t)f * B.mv;
+        tile_cells(G, F, Pf.cstart, cx, cy, cz, K, T.c);
+        const int M = T.c.nbeg[K];
+        // one pair per lane: the first n entries of the warp's queue
+        auto evaluate = [&](int n) {
+            __syncwarp();
+            if (lane < n) {
+                const int e = Q[lane];
+                const int p = e & 2047, sl = e >> 11;
+                const float4 w = T.w[p], q = T.hq[sl];
+                const int vk = T.v[p], hs = T.hs[sl];
+                const int v = vk & 0xffffff, s = hs & 0x7fffffff;
+                const float Dx = w.x - q.x, Dy = w.y - q.y, Dz = w.z - q.z;
+                float4 oa[APM];
+#pragma unroll
+                for (int a = 0; a < APM; ++a) oa[a] = Pf.so32[(int64_t)s * APM + a];
+                float m1 = INFINITY, m2 = INFINITY, r1 = INFINITY, r2 = INFINITY;
+                int k1 = 0;
+#pragma unroll
+                for (int b = 0; b < APM; ++b) {
+                    const float4 ob = Pf.so32[(int64_t)v * APM + b];
+                    const float tx = Dx + ob.x, ty = Dy + ob.y, tz = Dz + ob.z;
+                    float row = INFINITY;
+#pragma unroll
+                    for (int a = 0; a < APM; ++a) {
+                        const float ex = tx - oa[a].x, ey = ty - oa[a].y, ez = tz - oa[a].z;
+                        const float d2 = fmaf(ez, ez, fmaf(ey, ey, ex * ex));
+                        m2 = fminf(m2, fmaxf(m1, d2));
+                        k1 = d2 < m1 ? (a << 8 | b) : k1;
+                        m1 = fminf(m1, d2);
+                        row = fminf(row, d2);
+                        if (a == S.iref) r2 = fminf(r2, d2);
+                    }
+                    if (b == S.iref) r1 = row;
+                }
+                st.molpairs++;
+                st.atompairs += (unsigned long long)(APM * APM);
+                decide_pair<true>(S, B, h, Pf, g, f, s, hs < 0 ? Pf.slot[s] : -1, vk < 0, v, T.c.code[(vk >> 24) & 127], m1,
+                                  m2, k1 >> 8, k1 & 0xff, r1, r2, st);
+            }
+            __syncwarp();
+        };
+        for (int h0 = 0; h0 < nH; h0 += kDirectHome)
+            for (int m0 = 0; m0 < M; m0 += kDirectStage) {
+                const int nh = min(kDirectHome, nH - h0), n = min(kDirectStage, M - m0);
+                const int nr = (n + 31) & ~31;
+                __syncthreads();  // the previous pass's tables are no longer read
+                for (int i = tid; i < nr; i += blockDim.x) {
+                    if (i >= n) {
+                        T.w[i] = make_float4(0.f, 0.f, 0.f, INFINITY);  // never a candidate
+                        continue;
+                    }
+                    int k, dx, dy, dz;
+                    const int p = tile_molecule(T.c, K, m0 + i, k);
+                    half_stencil_cell(k, F.L, dx, dy, dz);
+                    const float4 of = Pf.off32[off_index(dx, dy, dz)];
+                    const float4 q = cq32[p];
+                    const float x = q.x + of.x, y = q.y + of.y, z = q.z + of.z;
+                    T.w[i] = make_float4(x, y, z, 0.5f * fmaf(z, z, fmaf(y, y, x * x)));
+                    const int v = Pf.cmol[p];
+                    T.v[i] = v | (k << 24) | (Pf.slot && Pf.slot[v] >= 0 ? 0x80000000 : 0);
+                }
+                for (int i = tid; i < nh; i += blockDim.x) {
+                    const float4 q = cq32[hbeg + h0 + i];
+                    const float R = (g.cut_pre + q.w) + rmax;
+                    T.hq[i] = make_float4(q.x, q.y, q.z, 0.5f * (R * R - fmaf(q.z, q.z, fmaf(q.y, q.y, q.x * q.x))));
+                    const int s = Pf.cmol[hbeg + h0 + i];
+                    T.hs[i] = s | (Pf.slot && Pf.slot[s] >= 0 ? 0x80000000 : 0);
+                }
+                if (tid == 0) T.next = 0;
+                __syncthreads();
+                int cnt = 0;
+                // the lanes' hits (bit j: staged position base + 32 j + lane) with home molecule sl into the queue
+                auto push = [&](unsigned bits, int base, int sl) {
+                    for (;;) {
+                        const unsigned mask = __ballot_sync(0xffffffffu, bits != 0);
+                        if (mask == 0) break;
+                        if (bits) {
+                            Q[cnt + __popc(mask & below)] = (base + 32 * (__ffs(bits) - 1) + lane) | sl << 11;
+                            bits &= bits - 1;
+                        }
+                        cnt += __popc(mask);
+                        if (cnt >= 32) {
+                            evaluate(32);
+                            cnt -= 32;
+                            const int rest = lane < cnt ? Q[32 + lane] : 0;
+                            __syncwarp();
+                            if (lane < cnt) Q[lane] = rest;
+                            __syncwarp();
+                        }
+                    }
+                };
+                // two home molecules at a time share the loads of the staged table
+                for (;;) {
+                    int sl = 0;
+                    if (lane == 0) sl = atomicAdd(&T.next, 2);
+                    sl = __shfl_sync(0xffffffffu, sl, 0);
+                    if (sl >= nh) break;
+                    const float4 q = T.hq[sl], r = T.hq[min(sl + 1, nh - 1)];
+                    const float rthr = sl + 1 < nh ? r.w : -INFINITY;
+                    // within the home cell (the first staged positions) only the molecules after this one
+                    const int lo = max(0, h0 + sl + 1 - m0), lo2 = max(0, h0 + sl + 2 - m0);
+                    for (int base = lo & ~31; base < nr; base += 1024) {
+                        const int nj = min(32, (nr - base) >> 5);
+                        unsigned bits = 0, bits2 = 0;
+#pragma unroll 4
+                        for (int j = 0; j < nj; ++j) {
+                            const float4 w = T.w[base + 32 * j + lane];
+                            const float u = fmaf(-w.x, q.x, fmaf(-w.y, q.y, fmaf(-w.z, q.z, w.w)));
+                            const float u2 = fmaf(-w.x, r.x, fmaf(-w.y, r.y, fmaf(-w.z, r.z, w.w)));
+                            if (u <= q.w) bits |= 1u << j;
+                            if (u2 <= rthr) bits2 |= 1u << j;
+                        }
+                        if (base + lane < lo) bits &= ~1u;
+                        if (base + lane < lo2) bits2 &= ~1u;
+                        if (base + 32 + lane < lo2) bits2 &= ~2u;
+                        push(bits, base, sl);
+                        push(bits2, base, sl + 1);
+                    }
+                }
+                if (cnt > 0) evaluate(cnt);
+            }
     }
     stats_flush(S, st, false);
     __syncthreads();
@@ -614,13 +1104,6 @@ struct PairIndex {
         a = r - b * aps;
     }
 };
-
-__device__ __forceinline__ void image_at(const Images &im, int img, int &dx, int &dy, int &dz) {
-    const int ix = img % im.cnt[0], iy = (img / im.cnt[0]) % im.cnt[1], iz = img / (im.cnt[0] * im.cnt[1]);
-    dx = im.base[0] + ix * im.step[0];
-    dy = im.base[1] + iy * im.step[1];
-    dz = im.base[2] + iz * im.step[2];
-}
 
 // FP32 pass of pairs_pass32 with the pairs split over the lanes; every lane
 // ends with the merged result (second-smallest over the union: the smaller of

@@ -101,6 +101,8 @@ struct GuardT {
     R bin_band;       // half-width of the bin-edge band in units of bins
     R dbulk_lo, dbulk_hi;
     float cut_pre;    // cutoff + margin of the bounding-sphere tests
+    float list_band;  // candidate grid: 2 delta + the margin of the lists (from here, not from S.cut: a conversion
+                      // from FP64 costs 64 cycles of an SM quarter, and was repeated in the query loops)
 };
 using Guard = GuardT<float>;
 using Guard64 = GuardT<double>;
@@ -1196,24 +1198,16 @@ __device__ __forceinline__ void emit(const DevSys &S, const SHist &h, const DirR
 
 // PAIRS real pass, generic (any molecule size, FP32 or FP64): one warp per
 // (frame, solute molecule) work item, every record decided where it is found
-// (no queues).  only_multi 0: every frame; 1: only the frames that need
-// several images per molecule pair (the rest were done by the specialised
-// FP32 kernel); 2: every frame, if k_queue_check raised the chunk's redo flag.
+// (no queues).  redo: only if k_queue_check raised the chunk's redo flag (the
+// FP32 search's kernels are those of cm_flat32.cuh).
 template <bool FP32, bool SELF>
-__global__ void __launch_bounds__(kWarps * 32) k_pairs_real(DevSys S, Bufs B, int only_multi) {
+__global__ void __launch_bounds__(kWarps * 32) k_pairs_real(DevSys S, Bufs B, int redo) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned int *hbase = (unsigned int *)smem_raw;
     const int hw = hist_words(S);
     float4 *os_all = (float4 *)(smem_raw + (((size_t)hw * 4 + 15) & ~(size_t)15));
     int *q_all = (int *)(os_all + kWarps * kMaxSmallMol);
-    if (only_multi == 2) {
-        if (B.counters[4] == 0) return;
-    } else if (only_multi) {
-        // nothing to do unless a frame of the chunk needs several images
-        int any = 0;
-        for (int f = threadIdx.x; f < B.nf; f += blockDim.x) any |= B.FS[f].multi;
-        if (!__syncthreads_or(any)) return;
-    }
+    if (redo && B.counters[4] == 0) return;
     shist_zero(S, hbase);
     __syncthreads();
     SHist h = shist_bind(S, hbase);
@@ -1228,7 +1222,6 @@ __global__ void __launch_bounds__(kWarps * 32) k_pairs_real(DevSys S, Bufs B, in
         const PairsFrame Pf = pairs_frame(B, f, SELF);
         const FrameGeom &G = *Pf.G;
         const FrameScratch &F = *Pf.F;
-        if (only_multi == 1 && !F.multi) continue;
         if (!F.ok) {
             if (lane == 0) raise_err(S, ERR_STENCIL);
             continue;
@@ -1270,7 +1263,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_pairs_real(DevSys S, Bufs B, in
 // After the FP32 real pass, its guard and edge kernels: if a queue
 // overflowed (records past the capacity were dropped), the accumulators and
 // statistics go back to their values before the real pass and the chunk's
-// redo flag is raised, so k_pairs_real (mode 2) decides every record of the
+// redo flag is raised, so k_pairs_real (redo) decides every record of the
 // chunk again without queues.  Any grid; returns at once without an overflow.
 __global__ void k_queue_check(Bufs B, unsigned long long *__restrict__ hist, const unsigned long long *__restrict__ snap,
                               int64_t n, unsigned long long *__restrict__ stats,
@@ -1675,6 +1668,7 @@ __device__ __forceinline__ void k_frame_consts_body(const uint3 blockIdx, const 
     g.dbulk_lo = __double2float_rd(S.dbulk - delta);
     g.dbulk_hi = __double2float_ru(S.dbulk + delta);
     g.cut_pre = __double2float_ru(S.cut + 1e-3 * (1.0 + range));
+    g.list_band = g.two_delta + 1e-3f * (1.0f + (float)S.cut);
     F.g = g;
     // the FP64 search: the same rules with band eps
     Guard64 g64;
@@ -1688,6 +1682,7 @@ __device__ __forceinline__ void k_frame_consts_body(const uint3 blockIdx, const 
     g64.dbulk_lo = __dsub_rd(S.dbulk, eps);
     g64.dbulk_hi = __dadd_ru(S.dbulk, eps);
     g64.cut_pre = g.cut_pre;
+    g64.list_band = g.list_band;
     F.g64 = g64;
 }
 

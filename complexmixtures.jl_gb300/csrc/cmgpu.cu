@@ -219,7 +219,8 @@ struct cm_handle {
     DevBuf scell, sq32, sq64, so32, so64, vcell, vq32, vq64, vo32, vo64, ccount, cstart, cfill, cmol, cq32, gq, rq, eq;
     int gq_cap = 0, rq_cap = 0;
     int flat_ctas = 0;  // resident CTAs per SM of k_pairs_flat32
-    int tile_ctas = 0;  // resident CTAs per SM of k_pairs_tile32 (self mode)
+    int tile_ctas = 0;  // resident CTAs per SM of k_pairs_tile32 / k_pairs_direct32 (self mode)
+    int images_ctas = 1;  // ... of k_pairs_images32
     int guard_ctas = 1, edge_ctas = 1, rand_ctas = 1, real_ctas = 1;  // ... of the guard, edge, random and generic kernels
     // group tables
     DevBuf g_soff, g_sidx, g_voff, g_vidx;
@@ -527,13 +528,23 @@ double target_cell(const cm_handle *h) {
     return h->pair_cell * scale;
 }
 
-// Per-CTA shared memory of the PAIRS real-pass kernels beyond the histograms.
-size_t pairs_extra_smem() {
-    const size_t real = (size_t)kWarps * kMaxSmallMol * 16 + (size_t)kWarps * kQueue * 8;
-    const size_t flat = (size_t)kFlatWarps * flat_warp_smem();
-    const size_t tile = (size_t)kTileWarps * flat_warp_smem() + tile_smem_extra();
-    return std::max(real, std::max(flat, tile));
+// Warps per CTA of a system's tiled real pass, and its shared memory beyond the histograms.
+int tile_warps(int aps) { return aps <= kDirectMax ? kDirectWarps : kTileWarps; }
+size_t tile_smem(int aps) {
+    return aps <= kDirectMax ? direct_smem_extra() : (size_t)kTileWarps * flat_warp_smem() + tile_smem_extra();
 }
+
+// Per-CTA shared memory that the PAIRS plan sets aside beyond the histograms:
+// what decides whether the group histograms go to shared memory (up to 50 KB
+// of histograms, so that two CTAs of a real-pass kernel fit an SM) and how many
+// bins are accepted.
+constexpr size_t kPairsExtraSmem = 110592;
+static_assert((size_t)kWarps * kMaxSmallMol * 16 + (size_t)kWarps * kQueue * 8 <= kPairsExtraSmem &&
+                  (size_t)kFlatWarps * flat_warp_smem() <= kPairsExtraSmem &&
+                  (size_t)kTileWarps * flat_warp_smem() + tile_smem_extra() <= kPairsExtraSmem &&
+                  direct_smem_extra() <= kPairsExtraSmem,
+              "a real-pass kernel needs more shared memory than the plan sets aside");
+size_t pairs_extra_smem() { return kPairsExtraSmem; }
 
 // The FP32 real-pass kernel for a system: specialised on the solute molecule
 // size for the common sizes, generic otherwise.
@@ -544,6 +555,8 @@ using TileLaunch = void (*)(int, size_t, cudaStream_t, const DevSys &, const Buf
 struct FlatKernel {
     const void *fn;
     FlatLaunch launch;
+    const void *images_fn;
+    FlatLaunch images_launch;
     const void *tile_fn;  // nullptr in cross mode
     TileLaunch tile_launch;
 };
@@ -553,23 +566,40 @@ void launch_flat(int grid, size_t smem, cudaStream_t st, const DevSys &S, const 
     k_pairs_flat32<SELF, APS><<<grid, kFlatWarps * 32, smem, st>>>(S, B, skip_tile);
 }
 
+template <bool SELF, int APS>
+void launch_images(int grid, size_t smem, cudaStream_t st, const DevSys &S, const Bufs &B, int parts) {
+    k_pairs_images32<SELF, APS><<<grid, kFlatWarps * 32, smem, st>>>(S, B, parts);
+}
+
 template <int APS>
 void launch_tile(int grid, size_t smem, cudaStream_t st, const DevSys &S, const Bufs &B) {
-    k_pairs_tile32<APS><<<grid, kTileWarps * 32, smem, st>>>(S, B);
+    if constexpr (APS > 0 && APS <= kDirectMax) k_pairs_direct32<APS><<<grid, kDirectWarps * 32, smem, st>>>(S, B);
+    else k_pairs_tile32<APS><<<grid, kTileWarps * 32, smem, st>>>(S, B);
+}
+
+// The tiled real pass: a lane per molecule pair for molecules of up to
+// kDirectMax atoms, a lane per solvent atom above.
+template <int APS>
+const void *tile_kernel() {
+    if constexpr (APS > 0 && APS <= kDirectMax) return (const void *)k_pairs_direct32<APS>;
+    else return (const void *)k_pairs_tile32<APS>;
 }
 
 template <bool SELF, int APS>
 FlatKernel flat_kernel_for() {
-    if (SELF)
-        return {(const void *)k_pairs_flat32<SELF, APS>, launch_flat<SELF, APS>, (const void *)k_pairs_tile32<APS>,
-                launch_tile<APS>};
-    return {(const void *)k_pairs_flat32<SELF, APS>, launch_flat<SELF, APS>, nullptr, nullptr};
+    if constexpr (SELF)
+        return {(const void *)k_pairs_flat32<SELF, APS>,   launch_flat<SELF, APS>, (const void *)k_pairs_images32<SELF, APS>,
+                launch_images<SELF, APS>, tile_kernel<APS>(), launch_tile<APS>};
+    else
+        return {(const void *)k_pairs_flat32<SELF, APS>,   launch_flat<SELF, APS>, (const void *)k_pairs_images32<SELF, APS>,
+                launch_images<SELF, APS>, nullptr, nullptr};
 }
 
 template <bool SELF>
 FlatKernel flat_kernel_of(int aps) {
     switch (aps) {
         case 1: return flat_kernel_for<SELF, 1>();
+        case 2: return flat_kernel_for<SELF, 2>();
         case 3: return flat_kernel_for<SELF, 3>();
         case 4: return flat_kernel_for<SELF, 4>();
         case 5: return flat_kernel_for<SELF, 5>();
@@ -615,9 +645,9 @@ int flat_setup(cm_handle *h) {
                             : (self ? (const void *)k_pairs_real<false, true> : (const void *)k_pairs_real<false, false>);
     h->real_ctas = resident_ctas(real, kWarps * 32, hsm + (size_t)kWarps * kMaxSmallMol * 16 + (size_t)kWarps * kQueue * 8);
     const FlatKernel fk = flat_kernel(h);
-    h->tile_ctas = fk.tile_fn ? resident_ctas(fk.tile_fn, kTileWarps * 32,
-                                              hsm + (size_t)kTileWarps * flat_warp_smem() + tile_smem_extra())
-                              : 0;
+    const int aps = h->d.solute_natomspermol;
+    h->tile_ctas = fk.tile_fn ? resident_ctas(fk.tile_fn, tile_warps(aps) * 32, hsm + tile_smem(aps)) : 0;
+    h->images_ctas = resident_ctas(fk.images_fn, kFlatWarps * 32, hsm + (size_t)kFlatWarps * flat_warp_smem());
     return resident_ctas(fk.fn, kFlatWarps * 32, hsm + (size_t)kFlatWarps * flat_warp_smem());
 }
 
@@ -699,9 +729,11 @@ void kernel_smem_limits(int device) {
     raise((const void *)k_multi<MK_EVAL_RANDOM_CELL>);
     raise((const void *)k_multi<MK_EVAL_REAL_BALANCED>);
     raise((const void *)k_multi<MK_EVAL_RANDOM_BALANCED>);
-    for (int aps : {0, 1, 3, 4, 5, 14}) {
+    for (int aps : {0, 1, 2, 3, 4, 5, 14}) {
         raise(flat_kernel_of<true>(aps).fn);
         raise(flat_kernel_of<true>(aps).tile_fn);
+        raise(flat_kernel_of<true>(aps).images_fn);
+        raise(flat_kernel_of<false>(aps).images_fn);
         raise(flat_kernel_of<false>(aps).fn);
     }
     g_smem_done[device] = true;
@@ -1375,9 +1407,7 @@ void run_chunk(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample *
         CM_LAUNCH(CM_K_CELLS, k_scatter_mols<<<dim3(grid_for(mv, 256), nf), 256, 0, st>>>(B, self ? 1 : 0));
         const size_t smem = hsm + (size_t)kWarps * kMaxSmallMol * 16 + (size_t)kWarps * kQueue * 8;
         const int grid = (int)std::min<int64_t>(((int64_t)nf * ms + kWarps - 1) / kWarps, (int64_t)sms * h->real_ctas);
-        // FP32: one lane per solvent atom; the frames that need several images
-        // per molecule pair are left to the generic kernel below
-        const bool special = fp32;
+        // FP32: one lane per solvent atom (or molecule pair); FP64: the generic kernel
         if (fp32) {
             // the accumulators before the real pass, for a redo after a queue overflow
             CM_CUDA(cudaMemcpyAsync(h->hist_snap.p, h->hist.p, (size_t)h->hist_n * 8, cudaMemcpyDeviceToDevice, st));
@@ -1390,19 +1420,20 @@ void run_chunk(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample *
             if (tile) {
                 // one CTA per home cell; the per-molecule kernel returns at once
                 // unless a frame's stencil is beyond the tiled kernel's table
-                const size_t tsm = hsm + (size_t)kTileWarps * flat_warp_smem() + tile_smem_extra();
+                const size_t tsm = hsm + tile_smem(d.solute_natomspermol);
                 CM_LAUNCH(CM_K_REAL, fk.tile_launch(sms * h->tile_ctas, tsm, st, S, B));
             }
             CM_LAUNCH(CM_K_REAL, fk.launch(fgrid, fsm, st, S, B, tile ? 1 : 0));
-        }
-        // the generic kernel takes every frame, or after the specialised one
-        // only the frames that need several images per molecule pair
-        const int only_multi = special ? 1 : 0;
-        if (fp32 && self) CM_LAUNCH(CM_K_REAL, k_pairs_real<true, true><<<grid, kWarps * 32, smem, st>>>(S, B, only_multi));
-        else if (fp32) CM_LAUNCH(CM_K_REAL, k_pairs_real<true, false><<<grid, kWarps * 32, smem, st>>>(S, B, only_multi));
-        else if (self) CM_LAUNCH(CM_K_REAL, k_pairs_real<false, true><<<grid, kWarps * 32, smem, st>>>(S, B, only_multi));
-        else CM_LAUNCH(CM_K_REAL, k_pairs_real<false, false><<<grid, kWarps * 32, smem, st>>>(S, B, only_multi));
-        if (special) {
+            // the frames of small boxes: up to 8 warps per solute molecule when
+            // there are too few molecules to fill the SMs
+            const int64_t warps = (int64_t)sms * h->images_ctas * kFlatWarps;
+            const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(8, warps / ((int64_t)nf * ms)));
+            const int igrid = (int)std::min<int64_t>(grid_for((int64_t)nf * ms * parts, kFlatWarps),
+                                                     (int64_t)sms * h->images_ctas);
+            CM_LAUNCH(CM_K_REAL, fk.images_launch(igrid, fsm, st, S, B, parts));
+        } else if (self) CM_LAUNCH(CM_K_REAL, k_pairs_real<false, true><<<grid, kWarps * 32, smem, st>>>(S, B, 0));
+        else CM_LAUNCH(CM_K_REAL, k_pairs_real<false, false><<<grid, kWarps * 32, smem, st>>>(S, B, 0));
+        if (fp32) {
             const int ggrid = sms * h->guard_ctas, egrid = sms * h->edge_ctas;
             if (self) CM_LAUNCH(CM_K_GUARD, k_pairs_guard<true><<<ggrid, kGuardWarps * 32, hsm, st>>>(S, B));
             else CM_LAUNCH(CM_K_GUARD, k_pairs_guard<false><<<ggrid, kGuardWarps * 32, hsm, st>>>(S, B));
@@ -1416,8 +1447,8 @@ void run_chunk(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample *
             CM_LAUNCH(CM_K_GUARD, k_queue_check<<<(int)std::min<int64_t>(grid_for(nrest, 256), (int64_t)sms * 4), 256, 0, st>>>(
                                       B, P<unsigned long long>(h->hist), P<unsigned long long>(h->hist_snap), h->hist_n,
                                       P<unsigned long long>(h->stats), P<unsigned long long>(h->stats_snap)));
-            if (self) CM_LAUNCH(CM_K_REAL, k_pairs_real<true, true><<<grid, kWarps * 32, smem, st>>>(S, B, 2));
-            else CM_LAUNCH(CM_K_REAL, k_pairs_real<true, false><<<grid, kWarps * 32, smem, st>>>(S, B, 2));
+            if (self) CM_LAUNCH(CM_K_REAL, k_pairs_real<true, true><<<grid, kWarps * 32, smem, st>>>(S, B, 1));
+            else CM_LAUNCH(CM_K_REAL, k_pairs_real<true, false><<<grid, kWarps * 32, smem, st>>>(S, B, 1));
         }
         if (rnd) {
             CM_LAUNCH(CM_K_BULK, k_bulk<<<c.ntab, 1024, 0, st>>>(S, B, dtab + c.tab0));
