@@ -421,7 +421,7 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
     sweep(true);
 }
 
-__global__ void __launch_bounds__(kAgridBuildThreads) k_agrid_build(DevSys S, Bufs B) {
+__global__ void __launch_bounds__(kAgridBuildThreads, 3) k_agrid_build(DevSys S, Bufs B) {
     k_agrid_build_body(blockIdx, gridDim, S, B);
 }
 

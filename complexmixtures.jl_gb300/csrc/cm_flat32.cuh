@@ -1355,19 +1355,91 @@ __global__ void __launch_bounds__(kGuardWarps * 32) k_pairs_guard(DevSys S, Bufs
     shist_flush(S, h, false);
 }
 
-// FP32 squared distance of one atom pair, the smallest over the images,
-// formed as in the FP32 passes ((q_v - q_s) + off + offset of b - offset of a).
-__device__ __forceinline__ float edge_d2(const PairsFrame &Pf, const Images &im, int s, int v, float4 oa, float4 ob) {
-    const float4 qs = Pf.sq32[s], qv = Pf.vq32[v];
-    float best = INFINITY;
-    CM_FOR_IMAGES(im, dx, dy, dz) {
-        const float4 o = Pf.off32[off_index(dx, dy, dz)];
-        const float ex = (((qv.x - qs.x) + o.x) + ob.x) - oa.x;
-        const float ey = (((qv.y - qs.y) + o.y) + ob.y) - oa.y;
-        const float ez = (((qv.z - qs.z) + o.z) + ob.z) - oa.z;
-        best = fminf(best, fmaf(ez, ez, fmaf(ey, ey, ex * ex)));
+// The random-insertion slots inside k_random_fast's band (rq2), one warp per
+// slot: placed in FP64 (the narrow band: k_random_eval's argument for the FP32
+// offsets), the pairs and the molecule's atoms split over the lanes, and
+// decided by decide_warp.  One thread per slot waited 360 us for its chain of
+// FP64 operations (14-atom molecules), whatever the number of slots.
+__global__ void __launch_bounds__(kGuardWarps * 32) k_random_records(DevSys S, Bufs B) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ float4 s_os[kGuardWarps][kMaxSmallMol], s_ov[kGuardWarps][kMaxSmallMol];
+    __shared__ double s_u[kGuardWarps][3][kMaxSmallMol];
+    unsigned int *hbase = (unsigned int *)smem_raw;
+    const int n = B.counters[10];
+    if ((int64_t)blockIdx.x * kGuardWarps >= n) return;
+    shist_zero(S, hbase);
+    __syncthreads();
+    const SHist h = shist_bind(S, hbase);
+    LocalStats st;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int aps = S.aps, apv = S.apv;
+    PairIndex pi;
+    pi.per_img = aps * apv;
+    pi.aps = aps;
+    pi.inv_pi = 1.0f / (float)pi.per_img;
+    pi.inv_aps = 1.0f / (float)aps;
+    for (int i = blockIdx.x * kGuardWarps + warp; i < n; i += gridDim.x * kGuardWarps) {
+        const int2 e = B.rq2[i];
+        const Sample sm = B.samples[e.x];
+        const int s = sm.s, k = e.y, f = sm.pad;
+        const PairsFrame Pf = pairs_frame(B, f, S.self);
+        const FrameGeom &G = *Pf.G;
+        const FrameScratch &F = *Pf.F;
+        int jmol, c0[3];
+        uint64_t fk[3];
+        float q0[3];
+        uint64_t rs = draw_slot_bits(S, G.frame_id, sm, k, Pf.bulk, Pf.nbulk, jmol, fk);
+        centre32(G, F.fx, fk, c0, q0);
+        const Images im = centre_images(G, F, Pf.scell[s], c0);
+        double A[9], fc[3];
+        for (int q = 0; q < 3; ++q) fc[q] = (double)fk[q] * 0x1.0p-53;
+        draw_rotation(rs, A);
+        ExactMol X = exact_mol_placed(S, G, f, s, jmol, fc, A);
+        raw_atom(B, true, f, X.vbase + S.iref, X.xr);
+        __syncwarp();
+        if (lane < aps) s_os[warp][lane] = Pf.so32[(int64_t)s * aps + lane];
+        if (lane < apv) {
+            const float4 w = Pf.vo32[(int64_t)jmol * apv + lane];
+            double r[3], x[3], u[3];
+            matvec_rm(A, w.x, w.y, w.z, r);
+            s_ov[warp][lane] = make_float4((float)r[0], (float)r[1], (float)r[2], 0.f);
+            raw_atom(B, true, f, X.vbase + lane, x);
+            exact_unwrapped(G, x, X.xr, u);
+            for (int q = 0; q < 3; ++q) s_u[warp][q][lane] = u[q];
+        }
+        __syncwarp();
+        // the mean in the order of exact_mol_ready
+        double cm = 0.0;
+        if (lane < 3) {
+            for (int b = 0; b < apv; ++b) cm = add(cm, s_u[warp][lane][b]);
+            cm = div(cm, (double)apv);
+        }
+        for (int q = 0; q < 3; ++q) X.cm[q] = __shfl_sync(0xffffffffu, cm, q);
+        X.ready = 1;
+        const float4 qs32 = Pf.sq32[s], qv32 = make_float4(q0[0], q0[1], q0[2], 0.f);
+        const int total = pi.per_img * image_count(im);
+        Pass32 P;
+        pass32_warp<false>(S, Pf.off32, im, qs32, qv32, s_os[warp], s_ov[warp], pi, total, lane, P);
+        DirRec r1, r2;
+        decide_warp<false>(S, G, B, X, F.g, P, Pf.off32, im, qs32, qv32, s_os[warp], s_ov[warp], s, k, pi, total, lane, r1, r2,
+                           st);
+        if (lane == 0 && r1.within) {
+            apply_hit_local(S, h, true, r1.bin, r1.i_local, r1.j, (int)(r1.j - (int64_t)k * apv), r1.ref, r1.rbin);
+            st.hits++;
+        }
     }
-    return best;
+    stats_flush(S, st, true);
+    __syncthreads();
+    shist_flush(S, h, true);
+}
+
+// setbin0 without its FP64 division where the quotient is not near an integer
+// (the product is within 4 u64 of it).
+__device__ __forceinline__ int setbin0_fast(double d, double step, double inv) {
+    const double k = d * inv, r = rint(k);
+    if (fabs(k - r) <= 1e-9 * (k + 1.0)) return setbin0(d, step);
+    const int b = (int)ceil(k);
+    return (b < 1 ? 1 : b) - 1;
 }
 
 // Edge kernel: records whose closest atom pair is known from the FP32 pass
@@ -1375,17 +1447,27 @@ __device__ __forceinline__ float edge_d2(const PairsFrame &Pf, const Images &im,
 // bin, solvent reference-atom row or solute reference-atom column (marked -2)
 // lies within the guard band of a bin edge or of the cutoff.  Each marked
 // value comes from exact pair distances (exact_d2): the closest pair for the
-// md bin, the aps pairs of the solvent molecule's reference atom for the row,
-// the apv pairs of the solute molecule's reference atom for the column.
+// md bin; for the row the pairs of the solvent molecule's reference atom whose
+// FP32 distance is within 2 delta of their smallest (nearly always one), for
+// the column those of the solute molecule's.
+//
+// One thread per record, one marked value per lane and round: a record has
+// nearly always one, and a round takes the warp's lanes through the same FP64
+// chain whichever value theirs is.  FP64 instructions hold a quarter of an SM
+// for 64 cycles each and bound the kernel; with the three kinds of value in
+// separate branches and a division per bin it ran 7.5 lanes wide, 927 us on 64
+// frames of 10,000 14-atom molecules, 300 so.
 template <bool SELF>
 __global__ void __launch_bounds__(128) k_pairs_edge(DevSys S, Bufs B) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned int *hbase = (unsigned int *)smem_raw;
+    const int n = min(B.counters[3], B.eq_cap);
+    if ((int64_t)blockIdx.x * blockDim.x >= n) return;
     shist_zero(S, hbase);
     __syncthreads();
     SHist h = shist_bind(S, hbase);
     LocalStats st;
-    const int n = min(B.counters[3], B.eq_cap);
+    const double inv = 1.0 / S.binstep;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int4 e = B.eq[3 * i], x = B.eq[3 * i + 1], y = B.eq[3 * i + 2];
         const int s = e.x, v = e.y, f = e.w;
@@ -1395,47 +1477,65 @@ __global__ void __launch_bounds__(128) k_pairs_edge(DevSys S, Bufs B) {
         const PairsFrame Pf = pairs_frame(B, f, SELF);
         const Images im = images_of(*Pf.G, *Pf.F, e.z);
         const FrameGeom &G = *Pf.G;
+        const Guard &g = Pf.F->g;
+        const float4 qs = Pf.sq32[s], qv = Pf.vq32[v];
+        const float4 *os32 = Pf.so32 + (int64_t)s * S.aps, *ov32 = Pf.vo32 + (int64_t)v * S.apv;
         ExactMol X = exact_mol(S, f, s, v);
         st.guard++;
-        int bulk = S.usecutoff ? (d32 > Pf.F->g.dbulk_hi) : 0;
-        if (bin == -2) {
-            const double d64 = sqrt(exact_pair_d2(B, G, X, a1, b1));
-            bin = setbin0(d64, S.binstep);
-            bulk = S.usecutoff ? (d64 > S.dbulk) : 0;
+        int bulk = S.usecutoff ? (d32 > g.dbulk_hi) : 0;
+        // FP32 squared distance of atoms a and b, the smallest over the images, formed as in the FP32 passes
+        auto d2_of = [&](int a, int b) {
+            const float4 oa = os32[a], ob = ov32[b];
+            float best = INFINITY;
+            CM_FOR_IMAGES(im, dx, dy, dz) {
+                const float4 o = Pf.off32[off_index(dx, dy, dz)];
+                const float ex = (((qv.x - qs.x) + o.x) + ob.x) - oa.x;
+                const float ey = (((qv.y - qs.y) + o.y) + ob.y) - oa.y;
+                const float ez = (((qv.z - qs.z) + o.z) + ob.z) - oa.z;
+                best = fminf(best, fmaf(ez, ez, fmaf(ey, ey, ex * ex)));
+            }
+            return best;
+        };
+        unsigned need = (bin == -2 ? 1u : 0u) | (rb1 == -2 ? 2u : 0u) | (SELF && rb2 == -2 ? 4u : 0u);
+        while (need) {
+            const int which = __ffs(need) - 1;
+            need &= need - 1;
+            const bool row = which == 1;
+            int a = a1, b = b1, at = 0, cnt = 0;
+            float thr = 0.f, m2 = INFINITY;
+            if (which != 0) {
+                cnt = row ? S.aps : S.apv;
+                float m = INFINITY;
+                for (int j = 0; j < cnt; ++j) {
+                    const float d2 = d2_of(row ? j : S.iref, row ? S.iref : j);
+                    m2 = fminf(m2, fmaxf(m, d2));
+                    at = d2 < m ? j : at;
+                    m = fminf(m, d2);
+                }
+                const float t = sqrtf(m) + g.two_delta;
+                thr = __fmul_ru(t, t);
+                a = row ? at : S.iref;
+                b = row ? S.iref : at;
+            }
+            double rr = exact_pair_d2(B, G, X, a, b);
             st.guard_pairs += 1;
-            st.maxerr = fmax(st.maxerr, fabs((double)d32 - d64));
-        }
-        // a row or column minimum in the band: its FP32 pass picks the pairs
-        // within 2 delta of the FP32 minimum (the exact minimum is among them),
-        // which are then evaluated exactly
-        const Guard &g = Pf.F->g;
-        if (rb1 == -2) {
-            const float4 ob = Pf.vo32[(int64_t)v * S.apv + S.iref];
-            const float4 *os32 = Pf.so32 + (int64_t)s * S.aps;
-            float m = INFINITY;
-            for (int a = 0; a < S.aps; ++a) m = fminf(m, edge_d2(Pf, im, s, v, os32[a], ob));
-            const float t = sqrtf(m) + g.two_delta, thr = __fmul_ru(t, t);
-            double rr = INFINITY;
-            for (int a = 0; a < S.aps; ++a) {
-                if (!(edge_d2(Pf, im, s, v, os32[a], ob) <= thr)) continue;
-                rr = fmin(rr, exact_pair_d2(B, G, X, a, S.iref));
-                st.guard_pairs += 1;
+            if (which != 0 && m2 <= thr)
+                for (int j = 0; j < cnt; ++j) {
+                    if (j == at || !(d2_of(row ? j : S.iref, row ? S.iref : j) <= thr)) continue;
+                    rr = fmin(rr, exact_pair_d2(B, G, X, row ? j : S.iref, row ? S.iref : j));
+                    st.guard_pairs += 1;
+                }
+            const double d64 = sqrt(rr);
+            const int k = setbin0_fast(d64, S.binstep, inv);
+            if (which == 0) {
+                bin = k;
+                bulk = S.usecutoff ? (d64 > S.dbulk) : 0;
+                st.maxerr = fmax(st.maxerr, fabs((double)d32 - d64));
+            } else {
+                const int r = rr <= S.cut2 ? k : -1;
+                if (row) rb1 = r;
+                else rb2 = r;
             }
-            rb1 = rr <= S.cut2 ? setbin0(sqrt(rr), S.binstep) : -1;
-        }
-        if (SELF && rb2 == -2) {
-            const float4 oa = Pf.so32[(int64_t)s * S.aps + S.iref];
-            const float4 *ov32 = Pf.vo32 + (int64_t)v * S.apv;
-            float m = INFINITY;
-            for (int b = 0; b < S.apv; ++b) m = fminf(m, edge_d2(Pf, im, s, v, oa, ov32[b]));
-            const float t = sqrtf(m) + g.two_delta, thr = __fmul_ru(t, t);
-            double rr = INFINITY;
-            for (int b = 0; b < S.apv; ++b) {
-                if (!(edge_d2(Pf, im, s, v, oa, ov32[b]) <= thr)) continue;
-                rr = fmin(rr, exact_pair_d2(B, G, X, S.iref, b));
-                st.guard_pairs += 1;
-            }
-            rb2 = rr <= S.cut2 ? setbin0(sqrt(rr), S.binstep) : -1;
         }
         apply_hit_local(S, h, false, bin, a1, (int64_t)v * S.apv + b1, b1, rb1 >= 0, rb1);
         st.hits++;

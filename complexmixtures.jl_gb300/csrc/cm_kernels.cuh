@@ -33,6 +33,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "cm_fixed.h"
 #include "cm_geom.h"
 
 namespace cmk {
@@ -134,7 +135,9 @@ struct FrameScratch {
     int agrid;      // ATOMS, one solute molecule: the frame's candidate grid is complete (k_agrid_scan clears it on overflow)
     FineCells fcells;  // the candidate grid's fine cells (when agrid)
     int place32;    // ATOMS, FP32 search: random-insertion slots placed in FP32 (placed_store32), the band widened to match
+    FixedGeom fx;   // integer positions of the FP32 search's prep (k_offtable)
     Guard g;        // FP32 search
+    Guard gr;       // FP32 random insertion of the PAIRS layout: slots placed in FP32 (k_random_fast)
     Guard64 g64;    // FP64 search
 };
 
@@ -396,11 +399,13 @@ struct Bufs {
     int gq_cap;
     int2 *rq;                       // (sample, slot)
     int rq_cap;
+    int2 *rq2;                      // slots inside k_random_fast's band (rq_cap entries; nullptr: k_random_eval takes
+                                    // every slot instead); count in counters[10]
     int4 *eq;                       // edge queue: 3 int4 per entry (s, v, code, frame), (a | b << 8, rb1, rb2, bin), (d32 bits)
     int eq_cap;
     int *counters;                  // [0] guard queue, [1] random queue, [2] ATOMS queue, [3] edge queue,
                                     // [4] the chunk's real pass is redone without queues (k_queue_check),
-                                    // [5] slot list, [6..7] work claims, [8] sorted slots, [9] deferred queries
+                                    // [5] slot list, [6..7] work claims, [8] sorted slots, [9] deferred queries, [10] rq2
     // ATOMS
     int *akey;                      // [nf][Ns]
     float4 *atq32, *asq32;
@@ -892,10 +897,20 @@ __device__ bool stencil(const FrameGeom &G, double range, int *L) {
 }
 
 // ------------------------------------------------------------------- kernels
-// Per-frame offset tables: off(Delta) = Hn Delta for Delta in [-kLT, kLT]^3.
+// Per-frame offset tables: off(Delta) = Hn Delta for Delta in [-kLT, kLT]^3;
+// and the integer geometry of the prep kernels (FrameScratch::fx).
 __device__ __forceinline__ void k_offtable_body(const uint3 blockIdx, const dim3 gridDim, const Bufs &B) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y;
     if (i >= kOffEntries) return;
+    if (i < 9) {
+        FixedGeom &X = B.FS[f].fx;
+        if (!fixed_geometry_entry(B.G[f], X, i)) atomicOr(&X.bad, 1);
+        if (i < 3) X.n[i] = B.G[f].n[i];
+        if (i == 0) {
+            X.ortho = B.G[f].hortho;
+            X.set = 1;
+        }
+    }
     const int dx = i % kLTW - kLT, dy = (i / kLTW) % kLTW - kLT, dz = i / (kLTW * kLTW) - kLT;
     double v[3];
     matvec_cm(B.G[f].Hn, (double)dx, (double)dy, (double)dz, v);
@@ -986,6 +1001,93 @@ __global__ void k_prep_pairs(Bufs B, const T *__restrict__ xyz, int64_t xyz_stri
     if (count_cells) atomicAdd(B.ccount + (int64_t)f * B.cs + cell, 1);
     warp_max_pos(solvent_side ? &F.rmax_v : &F.rmax_s, rf);
     warp_max_pos(&F.xmax, __double2float_ru(xm));
+}
+
+// k_prep_pairs of the FP32 search: the same molecule-centred data in integer
+// positions (cm_fixed.h), FP32 results only.  A molecule whose coordinates or
+// images the integers do not decide takes the FP64 chain.  140,000 atoms x 64
+// frames: 547 us with the FP64 chain, 198 here.
+template <typename T>
+__global__ void __launch_bounds__(128) k_prep_pairs32(Bufs B, const T *__restrict__ xyz, int64_t xyz_stride, int solvent_side,
+                                                      int count_cells) {
+    const int f = blockIdx.y;
+    const int nmol = (int)(solvent_side ? B.mv : B.ms);
+    const int64_t Nmol_atoms = solvent_side ? B.Nv : B.Ns;
+    const int apm = (int)(Nmol_atoms / nmol);
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= nmol) return;
+    const FrameGeom &G = B.G[f];
+    FrameScratch &F = B.FS[f];
+    const FixedGeom &X = F.fx;
+    float4 *mo32 = (solvent_side ? B.vo32 : B.so32) + (int64_t)f * Nmol_atoms + (int64_t)m * apm;
+    const T *x = xyz + (int64_t)f * xyz_stride + (int64_t)m * apm * 3;
+    int c[3];
+    float q[3], r = 0.f, xm = 0.f;
+    bool ok = X.set && !X.bad;
+    int64_t x0[3] = {0, 0, 0}, sum[3] = {0, 0, 0};
+    if (ok)
+        for (int k = 0; k < 3; ++k) ok = fixed_of(x[k], x0[k]) && ok;
+    // displacement of atom a from the first one, made its minimum image
+    auto displacement = [&](int a, int64_t *d) {
+        bool good = true;
+        for (int k = 0; k < 3; ++k) {
+            int64_t xa;
+            good = fixed_of(x[3 * a + k], xa) && good;
+            xm = fmaxf(xm, fixed_abs(xa));
+            d[k] = xa - x0[k];
+        }
+        return good && fixed_unwrap(X, d);
+    };
+    for (int a = 0; a < apm && ok; ++a) {
+        int64_t d[3];
+        ok = displacement(a, d);
+        for (int k = 0; k < 3; ++k) sum[k] += d[k];
+    }
+    if (ok) {
+        int64_t mean[3];
+        for (int k = 0; k < 3; ++k) mean[k] = fixed_mean(sum[k], apm);
+        bin_fixed(X, x0[0] + mean[0], x0[1] + mean[1], x0[2] + mean[2], c, q);
+        for (int a = 0; a < apm; ++a) {
+            int64_t d[3];
+            displacement(a, d);
+            const float ox = fixed_f32(d[0] - mean[0]), oy = fixed_f32(d[1] - mean[1]), oz = fixed_f32(d[2] - mean[2]);
+            mo32[a] = make_float4(ox, oy, oz, 0.f);
+            r = fmaxf(r, norm3f(ox, oy, oz));
+        }
+    } else {
+        double xd0[3], s[3] = {0.0, 0.0, 0.0}, qd[3];
+        load_xyz(x, xd0);
+        auto disp = [&](int a, double *d) {
+            double xa[3];
+            load_xyz(x + 3 * a, xa);
+            xm = fmaxf(xm, __double2float_ru(fmax(fabs(xa[0]), fmax(fabs(xa[1]), fabs(xa[2])))));
+            for (int k = 0; k < 3; ++k) d[k] = sub(xa[k], xd0[k]);
+            unwrap(G, d);
+        };
+        for (int a = 0; a < apm; ++a) {
+            double d[3];
+            disp(a, d);
+            for (int k = 0; k < 3; ++k) s[k] = add(s[k], d[k]);
+        }
+        for (int k = 0; k < 3; ++k) s[k] = div(s[k], (double)apm);
+        bin_position(G, add(xd0[0], s[0]), add(xd0[1], s[1]), add(xd0[2], s[2]), c, qd);
+        for (int k = 0; k < 3; ++k) q[k] = (float)qd[k];
+        for (int a = 0; a < apm; ++a) {
+            double d[3];
+            disp(a, d);
+            const float ox = (float)sub(d[0], s[0]), oy = (float)sub(d[1], s[1]), oz = (float)sub(d[2], s[2]);
+            mo32[a] = make_float4(ox, oy, oz, 0.f);
+            r = fmaxf(r, norm3f(ox, oy, oz));
+        }
+    }
+    const int cell = cell_linear(G, c[0], c[1], c[2]);
+    // radius bound: FP32 norm of the rounded offsets, enlarged to cover rounding
+    const float rf = r * (1.0f + 0x1.0p-18f) + 1e-5f;
+    (solvent_side ? B.vcell : B.scell)[(int64_t)f * nmol + m] = cell;
+    (solvent_side ? B.vq32 : B.sq32)[(int64_t)f * nmol + m] = make_float4(q[0], q[1], q[2], rf);
+    if (count_cells) atomicAdd(B.ccount + (int64_t)f * B.cs + cell, 1);
+    warp_max_pos(solvent_side ? &F.rmax_v : &F.rmax_s, rf);
+    warp_max_pos(&F.xmax, xm);
 }
 
 // Exclusive scans of the chunk's per-frame count arrays (one CTA of 1024
@@ -1388,20 +1490,39 @@ __device__ __forceinline__ uint64_t draw_slot_bits(const DevSys &S, int64_t fram
 
 // The centre's cell and its FP32 position from that cell's origin, from the
 // 53-bit uniforms: c = floor(U n) and g = U n - c exactly (integer product
-// fk n < 2^63), q0 = Hn g in FP64, rounded to FP32.
-__device__ __forceinline__ void centre32(const FrameGeom &G, const uint64_t *fk, int *c0, float *q0) {
-    double g[3];
+// fk n < 2^63), q0 = Hn g rounded to FP32 (fixed_lat, from the frame's
+// integer geometry; FP64 where there is none).
+__device__ __forceinline__ void centre32(const FrameGeom &G, const FixedGeom &X, const uint64_t *fk, int *c0, float *q0) {
+    uint64_t r[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         const uint64_t kn = fk[q] * (uint64_t)G.n[q];
         c0[q] = (int)(kn >> 53);
-        g[q] = (double)(kn & ((1ull << 53) - 1)) * 0x1.0p-53;
+        r[q] = kn & ((1ull << 53) - 1);
+    }
+    if (X.set) {
+        float gh[3], gl[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) fixed_split(r[q] << 11, gh[q], gl[q]);
+        fixed_lat(X, gh, gl, q0);
+        return;
     }
     double v[3];
-    matvec_cm(G.Hn, g[0], g[1], g[2], v);
+    matvec_cm(G.Hn, (double)r[0] * 0x1.0p-53, (double)r[1] * 0x1.0p-53, (double)r[2] * 0x1.0p-53, v);
     q0[0] = (float)v[0];
     q0[1] = (float)v[1];
     q0[2] = (float)v[2];
+}
+
+// Images of a slot's centre (cell c0) relative to solute molecule s.
+__device__ __forceinline__ Images centre_images(const FrameGeom &G, const FrameScratch &F, int sc, const int *c0) {
+    const int cs[3] = {sc % G.n[0], (sc / G.n[0]) % G.n[1], sc / (G.n[0] * G.n[1])};
+    Images im;
+    for (int q = 0; q < 3; ++q) {
+        axis_images(c0[q] - cs[q], G.n[q], F.L[q], im.base[q], im.cnt[q]);
+        im.step[q] = G.n[q];
+    }
+    return im;
 }
 
 // Images of a placed molecule (centre in fractional coordinates fc) relative
@@ -1435,12 +1556,15 @@ __global__ void __launch_bounds__(128) k_random_filter(DevSys S, Bufs B, int sam
     const FrameGeom &G = *Pf.G;
     const FrameScratch &F = *Pf.F;
     if (!F.ok) return;
-    const Placement P = draw_placement(S, G.frame_id, sm, k, Pf.bulk, Pf.nbulk);
-    double qp[3];
-    const Images im = placed_images(G, F, Pf.scell[s], P.fc, qp);
+    int jmol, c0[3];
+    uint64_t fk[3];
+    float q0[3];
+    draw_slot_bits(S, G.frame_id, sm, k, Pf.bulk, Pf.nbulk, jmol, fk);
+    centre32(G, F.fx, fk, c0, q0);
+    const Images im = centre_images(G, F, Pf.scell[s], c0);
     const float4 qs = Pf.sq32[s];
-    const float rr = F.g.cut_pre + qs.w + Pf.vq32[P.jmol].w;
-    const float px = (float)qp[0] - qs.x, py = (float)qp[1] - qs.y, pz = (float)qp[2] - qs.z;
+    const float rr = F.g.cut_pre + qs.w + Pf.vq32[jmol].w;
+    const float px = q0[0] - qs.x, py = q0[1] - qs.y, pz = q0[2] - qs.z;
     bool any = false;
     CM_FOR_IMAGES(im, ix, iy, iz) {
         const float4 o = Pf.off32[off_index(ix, iy, iz)];
@@ -1453,18 +1577,94 @@ __global__ void __launch_bounds__(128) k_random_filter(DevSys S, Bufs B, int sam
     else raise_err(S, ERR_QUEUE);
 }
 
-// PAIRS random pass, stage 2: one thread per kept slot.  Rotates the bulk
+// PAIRS random pass, stage 2 of the FP32 search: one thread per kept slot, the
+// slot placed in FP32 (centre32, draw_rotation32, the molecule's FP32
+// offsets) and evaluated against the sampled solute molecule with the band
+// widened by the placement's error (FrameScratch::gr).  A record inside that
+// band goes to the list rq2 (counters[10]) for k_random_records; the others are
+// counted here.  FP64 instructions
+// hold a quarter of an SM for 64 cycles each, and the placement in FP64 took
+// about 100 and 15 per atom of every slot.
+__global__ void __launch_bounds__(128, 5) k_random_fast(DevSys S, Bufs B) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned int *hbase = (unsigned int *)smem_raw;
+    const int n = min(B.counters[1], B.rq_cap);
+    if ((int64_t)blockIdx.x * blockDim.x >= n) return;
+    shist_zero(S, hbase);
+    __syncthreads();
+    const SHist h = shist_bind(S, hbase);
+    LocalStats st;
+    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n; it += gridDim.x * blockDim.x) {
+        const int2 e = B.rq[it];
+        const Sample sm = B.samples[e.x];
+        const int s = sm.s, k = e.y, f = sm.pad;
+        const PairsFrame Pf = pairs_frame(B, f, S.self);
+        const FrameGeom &G = *Pf.G;
+        const FrameScratch &F = *Pf.F;
+        const Guard &g = F.gr;
+        int jmol, c0[3];
+        uint64_t fk[3];
+        float q0[3], A[9];
+        uint64_t rs = draw_slot_bits(S, G.frame_id, sm, k, Pf.bulk, Pf.nbulk, jmol, fk);
+        centre32(G, F.fx, fk, c0, q0);
+        draw_rotation32(rs, A);
+        const Images im = centre_images(G, F, Pf.scell[s], c0);
+        const float4 qs = Pf.sq32[s];
+        const float4 *os = Pf.so32 + (int64_t)s * S.aps, *ov = Pf.vo32 + (int64_t)jmol * S.apv;
+        const float rr = F.g.cut_pre + qs.w + Pf.vq32[jmol].w;
+        PassT<float> P;
+        P.m1 = P.m2 = P.r1 = P.r2 = INFINITY;
+        P.k1 = 0;
+        st.molpairs++;
+        CM_FOR_IMAGES(im, dx, dy, dz) {
+            const float4 o = Pf.off32[off_index(dx, dy, dz)];
+            const float Dx = (q0[0] - qs.x) + o.x, Dy = (q0[1] - qs.y) + o.y, Dz = (q0[2] - qs.z) + o.z;
+            if (sq3(Dx, Dy, Dz) > rr * rr) continue;  // the image is out of reach
+            st.atompairs += (unsigned long long)S.aps * S.apv;
+            for (int b = 0; b < S.apv; ++b) {
+                const float4 w = ov[b];
+                const float tx = Dx + fmaf(A[2], w.z, fmaf(A[1], w.y, A[0] * w.x));
+                const float ty = Dy + fmaf(A[5], w.z, fmaf(A[4], w.y, A[3] * w.x));
+                const float tz = Dz + fmaf(A[8], w.z, fmaf(A[7], w.y, A[6] * w.x));
+                if (b == S.iref) inner_pass<true>(os, S.aps, S.apv, b, tx, ty, tz, P);
+                else inner_pass<false>(os, S.aps, S.apv, b, tx, ty, tz, P);
+            }
+        }
+        if (P.m1 > g.cutp2) continue;
+        const float d1 = sqrtf(P.m1);
+        const int bin = bin32(g, d1);
+        bool band = P.m1 >= g.cutm2 || (sqrtf(P.m2) - d1) <= g.two_delta || bin < 0;
+        int rb = -1;
+        if (P.r1 <= g.cutp2) {
+            rb = P.r1 < g.cutm2 ? bin32(g, sqrtf(P.r1)) : -1;
+            band = band || rb < 0;
+        }
+        if (band) {
+            B.rq2[atomicAdd(B.counters + 10, 1)] = e;
+            continue;
+        }
+        const int a = P.k1 / S.apv, b = P.k1 - a * S.apv;
+        apply_hit_local(S, h, true, bin, a, (int64_t)k * S.apv + b, b, rb >= 0, rb);
+        st.hits++;
+    }
+    stats_flush(S, st, true);
+    __syncthreads();
+    shist_flush(S, h, true);
+}
+
+// PAIRS random pass, stage 2 of the FP64 search and of the allocation-free
+// entry point (no room for rq2): one thread per kept slot.  Rotates the bulk
 // molecule about its centroid (src/rigid_body.jl:73-80, 122-134) and evaluates
 // it against the sampled solute molecule (one direction).
 template <bool FP32>
 __global__ void __launch_bounds__(128) k_random_eval(DevSys S, Bufs B) {
+    const int n = min(B.counters[1], B.rq_cap);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned int *hbase = (unsigned int *)smem_raw;
     shist_zero(S, hbase);
     __syncthreads();
     SHist h = shist_bind(S, hbase);
     LocalStats st;
-    const int n = min(B.counters[1], B.rq_cap);
     for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n; it += gridDim.x * blockDim.x) {
         const int2 e = B.rq[it];
         const Sample sm = B.samples[e.x];
@@ -1480,14 +1680,16 @@ __global__ void __launch_bounds__(128) k_random_eval(DevSys S, Bufs B) {
         // the search places the molecule's centroid-relative atom offsets;
         // the exact distances use the placement of the input coordinates
         const ExactRef X{f, s, P.jmol, A, P.fc};
-        const d4 *o = Pf.vo64 + (int64_t)P.jmol * S.apv;
         DirRec r1, r2;
         st.molpairs++;
         st.atompairs += (unsigned long long)S.aps * S.apv * image_count(im);
         if (FP32) {
+            // the FP32 offsets, rotated in FP64: each coordinate within 2 u r_v of the rotated FP64 offset,
+            // u r_v more than the band's bound counts and well inside its 25 % (E is at least 6 u r_v)
             float4 ov32[kMaxSmallMol];
+            const float4 *o = Pf.vo32 + (int64_t)P.jmol * S.apv;
             for (int b = 0; b < S.apv; ++b) {
-                const d4 w = o[b];
+                const float4 w = o[b];
                 double r[3];
                 matvec_rm(A, w.x, w.y, w.z, r);
                 ov32[b] = make_float4((float)r[0], (float)r[1], (float)r[2], 0.f);
@@ -1500,6 +1702,7 @@ __global__ void __launch_bounds__(128) k_random_eval(DevSys S, Bufs B) {
             pairs_decide<false>(S, G, B, X, F.g, Q, Pf.off32, im, qs32, qp32, os32, (const float4 *)ov32, s, k, r1, r2, st);
         } else {
             d4 ov64[kMaxSmallMol];
+            const d4 *o = Pf.vo64 + (int64_t)P.jmol * S.apv;
             for (int b = 0; b < S.apv; ++b) {
                 const d4 w = o[b];
                 double r[3];
@@ -1628,7 +1831,7 @@ __device__ __forceinline__ void k_frame_consts_body(const uint3 blockIdx, const 
         cn[lane] = norm3d(v[0], v[1], v[2]);
     }
     __syncthreads();
-    if (lane != 0) return;
+    if (lane > 1) return;  // lane 0: the search's constants; lane 1: the band of k_random_fast, beside it
     double Q = 0.0, OFF = 0.0;
     for (int k = 0; k < 8; ++k) {
         Q = fmax(Q, cn[k]);
@@ -1653,22 +1856,31 @@ __device__ __forceinline__ void k_frame_consts_body(const uint3 blockIdx, const 
     // slots per atom and more records per slot in a wider band, and keep the FP64 placement
     const double P = u * (5.0 * Q + 44.0 * (double)F.rcmax);
     const bool place32 = !pairs && S.fp32 && P <= 0.6 * E0;
-    F.place32 = place32 ? 1 : 0;
-    const double E = E0 + (place32 ? P : 0.0);
-    const double delta = 1.25 * (1.7320508075688772 * E + 2.5 * u * (S.cut + 1.0)) + 1e-9 + eps;
-    Guard g;
-    g.delta = delta;
-    const double cp = S.cut + delta, cm = S.cut - delta;
-    g.cutp2 = __double2float_ru(cp * cp);
-    g.cutm2 = cm > 0.0 ? __double2float_rd(cm * cm) : 0.0f;
-    g.two_delta = __double2float_ru(2.0 * delta);
-    g.inv_bs = (float)(1.0 / S.binstep);
-    // |k - d/binstep| <= delta/binstep + (rounding of d * inv_bs and of inv_bs)
-    g.bin_band = __double2float_ru(delta / S.binstep + (double)(S.nbins + 1) * 4.0 * u + 1e-6);
-    g.dbulk_lo = __double2float_rd(S.dbulk - delta);
-    g.dbulk_hi = __double2float_ru(S.dbulk + delta);
-    g.cut_pre = __double2float_ru(S.cut + 1e-3 * (1.0 + range));
-    g.list_band = g.two_delta + 1e-3f * (1.0f + (float)S.cut);
+    if (lane == 0) F.place32 = place32 ? 1 : 0;
+    // the band of displacements within E of the exact ones
+    auto band = [&](double E) {
+        const double delta = 1.25 * (1.7320508075688772 * E + 2.5 * u * (S.cut + 1.0)) + 1e-9 + eps;
+        Guard g;
+        g.delta = delta;
+        const double cp = S.cut + delta, cm = S.cut - delta;
+        g.cutp2 = __double2float_ru(cp * cp);
+        g.cutm2 = cm > 0.0 ? __double2float_rd(cm * cm) : 0.0f;
+        g.two_delta = __double2float_ru(2.0 * delta);
+        g.inv_bs = (float)(1.0 / S.binstep);
+        // |k - d/binstep| <= delta/binstep + (rounding of d * inv_bs and of inv_bs)
+        g.bin_band = __double2float_ru(delta / S.binstep + (double)(S.nbins + 1) * 4.0 * u + 1e-6);
+        g.dbulk_lo = __double2float_rd(S.dbulk - delta);
+        g.dbulk_hi = __double2float_ru(S.dbulk + delta);
+        g.cut_pre = __double2float_ru(S.cut + 1e-3 * (1.0 + range));
+        g.list_band = g.two_delta + 1e-3f * (1.0f + (float)S.cut);
+        return g;
+    };
+    // lane 1: the slots that k_random_fast places in FP32 (r_c: the solvent molecules' radius)
+    const Guard g = band(E0 + (lane == 1 ? u * (5.0 * Q + 44.0 * rv) : place32 ? P : 0.0));
+    if (lane == 1) {
+        F.gr = g;
+        return;
+    }
     F.g = g;
     // the FP64 search: the same rules with band eps
     Guard64 g64;
@@ -1729,7 +1941,10 @@ __device__ void centroid_data(const FrameGeom &G, const T *x, int apm, int iref,
 __device__ __forceinline__ int pack_cell(const int *c) { return c[0] | (c[1] << 10) | (c[2] << 20); }
 
 // Solvent atoms binned individually (grid y = frame); molecule-centred data
-// for random insertion.
+// for random insertion.  The FP32 search (no avq64) takes integer positions
+// (cm_fixed.h): cells, FP32 positions and FP32 molecule-centred offsets; a
+// molecule whose coordinates or images the integers do not decide takes the
+// FP64 chain.  150,000 atoms x 8 frames: 292 us with the FP64 chain, 35 so.
 template <typename T>
 __device__ __forceinline__ void k_prep_atoms_solvent_body(const uint3 blockIdx, const dim3 gridDim, const Bufs &B, const T *__restrict__ xyz, int64_t xyz_stride, int iref, int centroids) {
     const int f = blockIdx.y;
@@ -1737,32 +1952,96 @@ __device__ __forceinline__ void k_prep_atoms_solvent_body(const uint3 blockIdx, 
     if (m >= B.mv) return;
     const int apm = (int)(B.Nv / B.mv);
     const FrameGeom &G = B.G[f];
+    FrameScratch &F = B.FS[f];
     const T *x = xyz + (int64_t)f * xyz_stride + (int64_t)m * apm * 3;
-    const int64_t fo = (int64_t)f * B.Nv;
-    double xm = 0.0;
-    for (int b = 0; b < apm; ++b) {
-        double xb[3];
-        load_xyz(x + 3 * b, xb);
-        xm = fmax(xm, fmax(fabs(xb[0]), fmax(fabs(xb[1]), fabs(xb[2]))));
-        int c[3];
-        double q[3];
-        bin_position(G, xb[0], xb[1], xb[2], c, q);
-        const int64_t i = fo + (int64_t)m * apm + b;
-        B.avcell[i] = pack_cell(c);
-        B.avq32[i] = make_float4((float)q[0], (float)q[1], (float)q[2], 0.f);
-        if (B.avq64) B.avq64[i] = make_d4(q[0], q[1], q[2], 0.0);
-    }
-    warp_max_pos(&B.FS[f].xmax, __double2float_ru(xm));
-    if (centroids) {
-        float r;
-        centroid_data(G, x, apm, iref, B.u64 + fo + (int64_t)m * apm, r);
+    const int64_t at = (int64_t)f * B.Nv + (int64_t)m * apm;
+    float xm = 0.f, r = 0.f;
+    bool done = false;
+    if (!B.avq64 && F.fx.set && !F.fx.bad) {
+        const FixedGeom &X = F.fx;
+        bool ok = true;
+        int64_t xr[3] = {0, 0, 0}, sum[3] = {0, 0, 0};
+        for (int k = 0; k < 3; ++k) ok = fixed_of(x[3 * iref + k], xr[k]) && ok;
         for (int b = 0; b < apm; ++b) {
-            const d4 w = B.u64[fo + (int64_t)m * apm + b];
-            B.u32[fo + (int64_t)m * apm + b] = make_float4((float)w.x, (float)w.y, (float)w.z, 0.f);
+            int64_t p[3];
+            for (int k = 0; k < 3; ++k) {
+                ok = fixed_of(x[3 * b + k], p[k]) && ok;
+                xm = fmaxf(xm, fixed_abs(p[k]));
+            }
+            int c[3];
+            float q[3];
+            bin_fixed(X, p[0], p[1], p[2], c, q);
+            B.avcell[at + b] = pack_cell(c);
+            B.avq32[at + b] = make_float4(q[0], q[1], q[2], 0.f);
+            if (centroids) {
+                int64_t d[3] = {p[0] - xr[0], p[1] - xr[1], p[2] - xr[2]};
+                ok = fixed_unwrap(X, d) && ok;
+                for (int k = 0; k < 3; ++k) sum[k] += d[k];
+            }
         }
-        B.rc[(int64_t)f * B.mv + m] = r;
-        warp_max_pos(&B.FS[f].rcmax, r);
+        if (ok && centroids) {
+            int64_t mean[3];
+            for (int k = 0; k < 3; ++k) mean[k] = fixed_mean(sum[k], apm);
+            for (int b = 0; b < apm; ++b) {
+                int64_t d[3];
+                for (int k = 0; k < 3; ++k) {
+                    fixed_of(x[3 * b + k], d[k]);
+                    d[k] -= xr[k];
+                }
+                fixed_unwrap(X, d);
+                const float wx = fixed_f32(d[0] - mean[0]), wy = fixed_f32(d[1] - mean[1]), wz = fixed_f32(d[2] - mean[2]);
+                B.u32[at + b] = make_float4(wx, wy, wz, 0.f);
+                r = fmaxf(r, norm3f(wx, wy, wz));
+            }
+            // enlarged to cover the rounding of the offsets and of the norm
+            r = r * (1.0f + 0x1.0p-18f) + 1e-5f;
+        }
+        done = ok;
     }
+    if (!done) {
+        xm = 0.f;
+        for (int b = 0; b < apm; ++b) {
+            double xb[3];
+            load_xyz(x + 3 * b, xb);
+            xm = fmaxf(xm, __double2float_ru(fmax(fabs(xb[0]), fmax(fabs(xb[1]), fabs(xb[2])))));
+            int c[3];
+            double q[3];
+            bin_position(G, xb[0], xb[1], xb[2], c, q);
+            B.avcell[at + b] = pack_cell(c);
+            B.avq32[at + b] = make_float4((float)q[0], (float)q[1], (float)q[2], 0.f);
+            if (B.avq64) B.avq64[at + b] = make_d4(q[0], q[1], q[2], 0.0);
+        }
+        if (centroids) {
+            centroid_data(G, x, apm, iref, B.u64 + at, r);
+            for (int b = 0; b < apm; ++b) {
+                const d4 w = B.u64[at + b];
+                B.u32[at + b] = make_float4((float)w.x, (float)w.y, (float)w.z, 0.f);
+            }
+        }
+    }
+    warp_max_pos(&F.xmax, xm);
+    if (centroids) {
+        B.rc[(int64_t)f * B.mv + m] = r;
+        warp_max_pos(&F.rcmax, r);
+    }
+}
+
+// FP64 molecule-centred offsets of the FP32 search's frames that place in FP64
+// (not F.place32: larger molecules), after k_frame_consts has decided that.
+template <typename T>
+__device__ __forceinline__ void k_atoms_u64_body(const uint3 blockIdx, const dim3 gridDim, const Bufs &B, const T *__restrict__ xyz, int64_t xyz_stride, int iref) {
+    const int f = blockIdx.y;
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= B.mv || B.FS[f].place32) return;
+    const int apm = (int)(B.Nv / B.mv);
+    float r;
+    centroid_data(B.G[f], xyz + (int64_t)f * xyz_stride + (int64_t)m * apm * 3, apm, iref,
+                  B.u64 + (int64_t)f * B.Nv + (int64_t)m * apm, r);
+}
+
+template <typename T>
+__global__ void k_atoms_u64(Bufs B, const T *__restrict__ xyz, int64_t xyz_stride, int iref) {
+    k_atoms_u64_body<T>(blockIdx, gridDim, B, xyz, xyz_stride, iref);
 }
 
 template <typename T>
@@ -1778,19 +2057,31 @@ __device__ __forceinline__ void k_prep_atoms_solute_body(const uint3 blockIdx, c
     if (i >= B.Ns) return;
     const int aps = (int)(B.Ns / B.ms);
     const FrameGeom &G = B.G[f];
-    double x[3];
-    load_xyz(xyz + (int64_t)f * xyz_stride + 3 * (int64_t)i, x);
+    FrameScratch &F = B.FS[f];
+    const T *p = xyz + (int64_t)f * xyz_stride + 3 * (int64_t)i;
+    const int64_t fi = (int64_t)f * B.Ns + i;
     int c[3];
-    double q[3];
-    bin_position(G, x[0], x[1], x[2], c, q);
+    float q[3], xm;
+    int64_t X[3];
+    bool ok = !B.atq64 && F.fx.set && !F.fx.bad;
+    for (int k = 0; k < 3; ++k) ok = fixed_of(p[k], X[k]) && ok;
+    if (ok) {
+        bin_fixed(F.fx, X[0], X[1], X[2], c, q);
+        xm = fmaxf(fixed_abs(X[0]), fmaxf(fixed_abs(X[1]), fixed_abs(X[2])));
+    } else {
+        double x[3], qd[3];
+        load_xyz(p, x);
+        bin_position(G, x[0], x[1], x[2], c, qd);
+        for (int k = 0; k < 3; ++k) q[k] = (float)qd[k];
+        if (B.atq64) B.atq64[fi] = make_d4(qd[0], qd[1], qd[2], 0.0);
+        xm = __double2float_ru(fmax(fabs(x[0]), fmax(fabs(x[1]), fabs(x[2]))));
+    }
     const int s = i / aps, a = i - s * aps;
     const int k = s * G.ncell + cell_linear(G, c[0], c[1], c[2]);
-    const int64_t fi = (int64_t)f * B.Ns + i;
     B.akey[fi] = k;
-    B.atq32[fi] = make_float4((float)q[0], (float)q[1], (float)q[2], __int_as_float(a));
-    if (B.atq64) B.atq64[fi] = make_d4(q[0], q[1], q[2], 0.0);
+    B.atq32[fi] = make_float4(q[0], q[1], q[2], __int_as_float(a));
     atomicAdd(B.acount + (int64_t)f * B.as + k, 1);
-    warp_max_pos(&B.FS[f].xmax, __double2float_ru(fmax(fabs(x[0]), fmax(fabs(x[1]), fabs(x[2])))));
+    warp_max_pos(&F.xmax, xm);
 }
 
 template <typename T>
@@ -1873,8 +2164,9 @@ __device__ __forceinline__ void placed_atom(const FrameGeom &G, const FrameScrat
 // positions only for the FP64 search: the FP32 search and its exact scans
 // read the FP32 ones and draw the exact placement again).
 __device__ __forceinline__ void placed_store(const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F,
-                                             const d4 *off64, const double *A, const d4 *u, const int *c0,
+                                             const d4 *off64, const double *A, int f, int jmol, const int *c0,
                                              const double *q0, const double *fc, int64_t base) {
+    const d4 *u = B.u64 + (int64_t)f * B.Nv + (int64_t)jmol * S.apv;
     for (int b = 0; b < S.apv; ++b) {
         int c[3];
         double q[3];
@@ -1882,6 +2174,26 @@ __device__ __forceinline__ void placed_store(const DevSys &S, const Bufs &B, con
         B.pcell[base + b] = pack_cell(c);
         B.pq32[base + b] = make_float4((float)q[0], (float)q[1], (float)q[2], 0.f);
         if (!S.fp32) B.pq64[base + b] = make_d4(q[0], q[1], q[2], 0.0);
+    }
+}
+
+// placed_store for a slot of a frame that places in FP32 (an atom beyond the
+// offset table): there are no FP64 offsets (k_atoms_u64), so they are formed
+// again from the input coordinates.
+__device__ __noinline__ void placed_store_lost(const DevSys &S, const Bufs &B, const FrameGeom &G, const FrameScratch &F,
+                                               const d4 *off64, const double *A, int f, int jmol, const int *c0,
+                                               const double *q0, const double *fc, int64_t base) {
+    ExactMol X = exact_mol(S, f, 0, jmol);
+    exact_mol_ready(B, G, X);
+    for (int b = 0; b < S.apv; ++b) {
+        double x[3], y[3], q[3];
+        int c[3];
+        raw_atom(B, true, f, X.vbase + b, x);
+        exact_unwrapped(G, x, X.xr, y);
+        const d4 w = make_d4(sub(y[0], X.cm[0]), sub(y[1], X.cm[1]), sub(y[2], X.cm[2]), 0.0);
+        placed_atom(G, F, off64, A, w, c0, q0, fc, c, q);
+        B.pcell[base + b] = pack_cell(c);
+        B.pq32[base + b] = make_float4((float)q[0], (float)q[1], (float)q[2], 0.f);
     }
 }
 
@@ -2060,7 +2372,7 @@ __device__ __forceinline__ void k_atoms_place_body(const uint3 blockIdx, const d
             uint64_t rs = draw_slot_bits(S, G.frame_id, sm, k, bulk, nbulk, jmol, fk);
             int c0[3];
             float q0[3];
-            centre32(G, fk, c0, q0);
+            centre32(G, F.fx, fk, c0, q0);
             float A32[9];
             draw_rotation32(rs, A32);
             placed = placed_store32(B, F, G, B.off32 + (int64_t)f * kOffEntries, A32,
@@ -2075,8 +2387,9 @@ __device__ __forceinline__ void k_atoms_place_body(const uint3 blockIdx, const d
             uint64_t rs = P.st;
             double A[9];
             draw_rotation(rs, A);
-            placed_store(S, B, G, F, B.off64 + (int64_t)f * kOffEntries, A, B.u64 + (int64_t)f * B.Nv + (int64_t)P.jmol * S.apv,
-                         c0, q0, P.fc, base);
+            const d4 *off64 = B.off64 + (int64_t)f * kOffEntries;
+            if (F.place32) placed_store_lost(S, B, G, F, off64, A, f, P.jmol, c0, q0, P.fc, base);
+            else placed_store(S, B, G, F, off64, A, f, P.jmol, c0, q0, P.fc, base);
         }
         if (F.agrid) {
             const int2 kr = B.skey[it];

@@ -42,6 +42,8 @@ enum MKid : int {
     MK_PREP_SOLUTE_F32,
     MK_PREP_SOLUTE_F64,
     MK_FRAME_CONSTS,
+    MK_ATOMS_U64_F32,
+    MK_ATOMS_U64_F64,
     MK_SCAN,
     MK_SCATTER_ATOMS,
     MK_ATOMS_NEAR,
@@ -76,7 +78,7 @@ __host__ __device__ constexpr bool mk_query(int kid) {
 // Threads per CTA of each stage (the stand-alone launch's block size).
 __host__ __device__ constexpr int mk_threads(int kid) {
     return kid == MK_OFFTABLE ? 256
-         : (kid == MK_PREP_SOLVENT_F32 || kid == MK_PREP_SOLVENT_F64) ? 128
+         : (kid == MK_PREP_SOLVENT_F32 || kid == MK_PREP_SOLVENT_F64 || kid == MK_ATOMS_U64_F32 || kid == MK_ATOMS_U64_F64) ? 128
          : (kid == MK_PREP_SOLUTE_F32 || kid == MK_PREP_SOLUTE_F64) ? 256
          : kid == MK_FRAME_CONSTS ? 128
          : (kid == MK_SCAN || kid == MK_SLOT_SCAN) ? 1024
@@ -99,6 +101,8 @@ __device__ __forceinline__ void mk_body(const uint3 vb, const dim3 vg, const MAr
     else if constexpr (KID == MK_PREP_SOLUTE_F32) k_prep_atoms_solute_body<float>(vb, vg, a.B, (const float *)a.p, a.i0);
     else if constexpr (KID == MK_PREP_SOLUTE_F64) k_prep_atoms_solute_body<double>(vb, vg, a.B, (const double *)a.p, a.i0);
     else if constexpr (KID == MK_FRAME_CONSTS) k_frame_consts_body(vb, vg, a.S, a.B, a.a0);
+    else if constexpr (KID == MK_ATOMS_U64_F32) k_atoms_u64_body<float>(vb, vg, a.B, (const float *)a.p, a.i0, a.a0);
+    else if constexpr (KID == MK_ATOMS_U64_F64) k_atoms_u64_body<double>(vb, vg, a.B, (const double *)a.p, a.i0, a.a0);
     else if constexpr (KID == MK_SCAN) k_scan_body(vb, vg, a.B, a.a0);
     else if constexpr (KID == MK_SCATTER_ATOMS) k_scatter_atoms_body(vb, vg, a.B);
     else if constexpr (KID == MK_ATOMS_NEAR) k_atoms_near_body(vb, vg, a.B);

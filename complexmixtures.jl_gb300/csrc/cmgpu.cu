@@ -216,12 +216,13 @@ struct cm_handle {
     DevBuf hist_snap, stats_snap;  // accumulators before a chunk's real pass (restored if its queues overflow)
     DevBuf stage_s[2], stage_v[2];
     // PAIRS
-    DevBuf scell, sq32, sq64, so32, so64, vcell, vq32, vq64, vo32, vo64, ccount, cstart, cfill, cmol, cq32, gq, rq, eq;
+    DevBuf scell, sq32, sq64, so32, so64, vcell, vq32, vq64, vo32, vo64, ccount, cstart, cfill, cmol, cq32, gq, rq, rq2, eq;
     int gq_cap = 0, rq_cap = 0;
     int flat_ctas = 0;  // resident CTAs per SM of k_pairs_flat32
     int tile_ctas = 0;  // resident CTAs per SM of k_pairs_tile32 / k_pairs_direct32 (self mode)
     int images_ctas = 1;  // ... of k_pairs_images32
-    int guard_ctas = 1, edge_ctas = 1, rand_ctas = 1, real_ctas = 1;  // ... of the guard, edge, random and generic kernels
+    int guard_ctas = 1, edge_ctas = 1, rand_ctas = 1, fast_ctas = 1, records_ctas = 1,
+        real_ctas = 1;  // ... of the guard, edge, random and generic kernels
     // group tables
     DevBuf g_soff, g_sidx, g_voff, g_vidx;
     // ATOMS
@@ -641,6 +642,8 @@ int flat_setup(cm_handle *h) {
                                   kGuardWarps * 32, hsm);
     h->edge_ctas = resident_ctas(self ? (const void *)k_pairs_edge<true> : (const void *)k_pairs_edge<false>, 128, hsm);
     h->rand_ctas = resident_ctas(fp32 ? (const void *)k_random_eval<true> : (const void *)k_random_eval<false>, 128, hsm);
+    h->fast_ctas = resident_ctas((const void *)k_random_fast, 128, hsm);
+    h->records_ctas = resident_ctas((const void *)k_random_records, kGuardWarps * 32, hsm);
     const void *real = fp32 ? (self ? (const void *)k_pairs_real<true, true> : (const void *)k_pairs_real<true, false>)
                             : (self ? (const void *)k_pairs_real<false, true> : (const void *)k_pairs_real<false, false>);
     h->real_ctas = resident_ctas(real, kWarps * 32, hsm + (size_t)kWarps * kMaxSmallMol * 16 + (size_t)kWarps * kQueue * 8);
@@ -701,6 +704,8 @@ void kernel_smem_limits(int device) {
     raise((const void *)k_pairs_real<false, true>);
     raise((const void *)k_pairs_real<false, false>);
     raise((const void *)k_random_eval<true>);
+    raise((const void *)k_random_fast);
+    raise((const void *)k_random_records);
     raise((const void *)k_random_eval<false>);
     for (const AtomsKernels &k : {atoms_kernels_of<true, kSchedCell>(), atoms_kernels_of<true, kSchedBalanced>(),
                                   atoms_kernels_of<false, kSchedCell>(), atoms_kernels_of<false, kSchedThread>()}) {
@@ -868,15 +873,20 @@ void plan(cm_handle *h, const cm_frames *f) {
     if (h->regime == CM_REGIME_PAIRS) {
         dev_alloc(h, h->scell, fc * ms * 4);
         dev_alloc(h, h->sq32, fc * ms * 16);
-        dev_alloc(h, h->sq64, fc * ms * 32);
         dev_alloc(h, h->so32, fc * h->Ns * 16);
-        dev_alloc(h, h->so64, fc * h->Ns * 32);
+        const bool fp64 = d.precision != CM_PRECISION_FP32_GUARD;  // the FP64 search's molecules
+        if (fp64) {
+            dev_alloc(h, h->sq64, fc * ms * 32);
+            dev_alloc(h, h->so64, fc * h->Ns * 32);
+        }
         if (!d.autocorrelation) {
             dev_alloc(h, h->vcell, fc * mv * 4);
             dev_alloc(h, h->vq32, fc * mv * 16);
-            dev_alloc(h, h->vq64, fc * mv * 32);
             dev_alloc(h, h->vo32, fc * h->Nv * 16);
-            dev_alloc(h, h->vo64, fc * h->Nv * 32);
+            if (fp64) {
+                dev_alloc(h, h->vq64, fc * mv * 32);
+                dev_alloc(h, h->vo64, fc * h->Nv * 32);
+            }
         }
         dev_alloc(h, h->cmol, fc * mv * 4);
         dev_alloc(h, h->cq32, fc * mv * 16);
@@ -894,6 +904,7 @@ void plan(cm_handle *h, const cm_frames *f) {
             const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>((int64_t)fc * d.n_random_samples, (1 << 23) / mv));
             h->rq_cap = (int)(chunk * mv);
             dev_alloc(h, h->rq, (size_t)h->rq_cap * sizeof(int2));
+            if (d.precision == CM_PRECISION_FP32_GUARD) dev_alloc(h, h->rq2, (size_t)h->rq_cap * sizeof(int2));
         }
     } else {
         dev_alloc(h, h->akey, fc * h->Ns * 4);
@@ -1121,6 +1132,7 @@ Bufs chunk_bufs(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample 
         B.eq = P<int4>(h->eq);
         B.eq_cap = h->gq_cap;
         B.rq = P<int2>(h->rq);
+        B.rq2 = P<int2>(h->rq2);
         B.rq_cap = h->rq_cap;
     } else {
         B.akey = P<int>(h->akey);
@@ -1181,6 +1193,8 @@ void launch_one(int kid, dim3 g, size_t smem, cudaStream_t st, const MArgs &a) {
     case MK_PREP_SOLUTE_F32: k_prep_atoms_solute<float><<<g, t, smem, st>>>(a.B, (const float *)a.p, a.i0); break;
     case MK_PREP_SOLUTE_F64: k_prep_atoms_solute<double><<<g, t, smem, st>>>(a.B, (const double *)a.p, a.i0); break;
     case MK_FRAME_CONSTS: k_frame_consts<<<g, t, smem, st>>>(a.S, a.B, a.a0); break;
+    case MK_ATOMS_U64_F32: k_atoms_u64<float><<<g, t, smem, st>>>(a.B, (const float *)a.p, a.i0, a.a0); break;
+    case MK_ATOMS_U64_F64: k_atoms_u64<double><<<g, t, smem, st>>>(a.B, (const double *)a.p, a.i0, a.a0); break;
     case MK_SCAN: k_scan<<<g, t, smem, st>>>(a.B, a.a0); break;
     case MK_SCATTER_ATOMS: k_scatter_atoms<<<g, t, smem, st>>>(a.B); break;
     case MK_ATOMS_NEAR: k_atoms_near<<<g, t, smem, st>>>(a.B); break;
@@ -1301,6 +1315,9 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
     em.kernel(f32 ? MK_PREP_SOLUTE_F32 : MK_PREP_SOLUTE_F64, dim3(grid_for(h->Ns, 256), nf), 0, CM_K_PREP,
               args(xs, xs_stride, 0, 0, 0));
     em.kernel(MK_FRAME_CONSTS, dim3(nf), 0, CM_K_PREP, args(nullptr, 0, 0, 0, 0));
+    if (rnd && d.precision == CM_PRECISION_FP32_GUARD)
+        em.kernel(f32 ? MK_ATOMS_U64_F32 : MK_ATOMS_U64_F64, dim3(grid_for(mv, 128), nf), 0, CM_K_PREP,
+                  args(xsolv, self ? xs_stride : xv_stride, 0, iref, 0));
     em.kernel(MK_SCAN, dim3(nf), 0, CM_K_CELLS, args(nullptr, 0, 0, 1, 0));
     em.kernel(MK_SCATTER_ATOMS, dim3(grid_for(h->Ns, 256), nf), 0, CM_K_CELLS, base);
     if (rnd) em.zero(B.flags, (size_t)nf * B.ndist * mv);
@@ -1399,9 +1416,12 @@ void run_chunk(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample *
         if (rnd) CM_CUDA(cudaMemsetAsync(B.flags, 0, (size_t)nf * B.ndist * mv, st));
         CM_CUDA(cudaMemsetAsync(B.ccount, 0, (size_t)nf * B.cs * 4, st));
         // solute molecules (in self mode they also fill the cell counts)
-        CM_LAUNCH(CM_K_PREP, k_prep_pairs<T><<<dim3(grid_for(ms, 128), nf), 128, 0, st>>>(B, xs, xs_stride, 0, self ? 1 : 0));
-        if (!self)
-            CM_LAUNCH(CM_K_PREP, k_prep_pairs<T><<<dim3(grid_for(mv, 128), nf), 128, 0, st>>>(B, xv, xv_stride, 1, 1));
+        auto prep = [&](const T *x, int64_t stride, int64_t n, int side, int count) {
+            if (fp32) CM_LAUNCH(CM_K_PREP, k_prep_pairs32<T><<<dim3(grid_for(n, 128), nf), 128, 0, st>>>(B, x, stride, side, count));
+            else CM_LAUNCH(CM_K_PREP, k_prep_pairs<T><<<dim3(grid_for(n, 128), nf), 128, 0, st>>>(B, x, stride, side, count));
+        };
+        prep(xs, xs_stride, ms, 0, self ? 1 : 0);
+        if (!self) prep(xv, xv_stride, mv, 1, 1);
         CM_LAUNCH(CM_K_PREP, k_frame_consts<<<nf, 128, 0, st>>>(S, B, 1));
         CM_LAUNCH(CM_K_CELLS, k_scan<<<nf, 1024, 0, st>>>(B, 0));
         CM_LAUNCH(CM_K_CELLS, k_scatter_mols<<<dim3(grid_for(mv, 256), nf), 256, 0, st>>>(B, self ? 1 : 0));
@@ -1456,9 +1476,16 @@ void run_chunk(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample *
             const int piece = (int)std::max<int64_t>(1, h->rq_cap / mv);
             for (int s0 = 0; s0 < c.nsmp; s0 += piece) {
                 const int ny = std::min(piece, c.nsmp - s0);
-                if (s0 > 0) CM_CUDA(cudaMemsetAsync(B.counters + 1, 0, sizeof(int), st));
+                if (s0 > 0) {
+                    CM_CUDA(cudaMemsetAsync(B.counters + 1, 0, sizeof(int), st));
+                    if (B.rq2) CM_CUDA(cudaMemsetAsync(B.counters + 10, 0, sizeof(int), st));
+                }
                 CM_LAUNCH(CM_K_RANDOM, k_random_filter<<<grid_for((int64_t)ny * mv, 128), 128, 0, st>>>(S, B, c.smp0 + s0, ny));
-                if (fp32) CM_LAUNCH(CM_K_RANDOM, k_random_eval<true><<<sms * h->rand_ctas, 128, hsm, st>>>(S, B));
+                if (B.rq2) {
+                    const int fgrid = (int)std::min<int64_t>(grid_for((int64_t)ny * mv, 128), (int64_t)sms * h->fast_ctas);
+                    CM_LAUNCH(CM_K_RANDOM, k_random_fast<<<fgrid, 128, hsm, st>>>(S, B));
+                    CM_LAUNCH(CM_K_RANDOM, k_random_records<<<sms * h->records_ctas, kGuardWarps * 32, hsm, st>>>(S, B));
+                } else if (fp32) CM_LAUNCH(CM_K_RANDOM, k_random_eval<true><<<sms * h->rand_ctas, 128, hsm, st>>>(S, B));
                 else CM_LAUNCH(CM_K_RANDOM, k_random_eval<false><<<sms * h->rand_ctas, 128, hsm, st>>>(S, B));
             }
         }
@@ -1847,7 +1874,7 @@ void free_all(cm_handle *h) {
     DevBuf *all[] = {&h->geoms, &h->samples, &h->fscratch, &h->off64, &h->off32, &h->hist, &h->sums, &h->stats, &h->errflag, &h->hist_snap, &h->stats_snap,
                      &h->slot, &h->flags, &h->bulk, &h->nbulk, &h->tabs, &h->counters, &h->stage_s[0], &h->stage_s[1], &h->stage_v[0],
                      &h->stage_v[1], &h->scell, &h->sq32, &h->sq64, &h->so32, &h->so64, &h->vcell, &h->vq32, &h->vq64,
-                     &h->vo32, &h->vo64, &h->u64, &h->u32, &h->rc, &h->ccount, &h->cstart, &h->cfill, &h->cmol, &h->cq32, &h->gq, &h->eq, &h->rq, &h->akey, &h->atq32,
+                     &h->vo32, &h->vo64, &h->u64, &h->u32, &h->rc, &h->ccount, &h->cstart, &h->cfill, &h->cmol, &h->cq32, &h->gq, &h->eq, &h->rq, &h->rq2, &h->akey, &h->atq32,
                      &h->atq64, &h->asq32, &h->asq64, &h->acount, &h->astart, &h->afill, &h->avcell, &h->avq32, &h->avq64,
                      &h->pcell, &h->pq32, &h->pq64, &h->anear, &h->aq, &h->g_soff, &h->g_sidx, &h->g_voff, &h->g_vidx,
                      &h->aslot, &h->skey, &h->adefer, &h->sslot, &h->scount, &h->gstart, &h->gedge, &h->gpool, &h->gent, &h->dcd_sidx, &h->dcd_vidx, &h->dcd_raw[0], &h->dcd_raw[1], &h->final_out, &h->final_job,
@@ -2218,6 +2245,8 @@ void launch_multi(int kid, unsigned grid, size_t smem, cudaStream_t st, const MT
         CM_MK(MK_PREP_SOLUTE_F32)
         CM_MK(MK_PREP_SOLUTE_F64)
         CM_MK(MK_FRAME_CONSTS)
+        CM_MK(MK_ATOMS_U64_F32)
+        CM_MK(MK_ATOMS_U64_F64)
         CM_MK(MK_SCAN)
         CM_MK(MK_SCATTER_ATOMS)
         CM_MK(MK_ATOMS_NEAR)

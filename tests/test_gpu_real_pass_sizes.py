@@ -49,3 +49,27 @@ def test_crowded_cells(cm, orc, gpu_ready, apm):
     got, ref, st = compare(cm, orc, ms=n, aps=apm, mv=n, apv=apm, xs=xs, xv=None, cells=cells, self_mode=True,
                            precision="fp32", regime="pairs", irefatom=1, dbulk=4.0, usecutoff=False, **OPT)
     assert ref["md"].sum() > 0
+
+
+@pytest.mark.parametrize("apm", [1, 3, 14, 32])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_random_insertion_and_prep(cm, orc, gpu_ready, apm, dtype):
+    """Many random samples on fine bins (slots inside the FP32 placement's band
+    decided apart), molecules split over the periodic boundary, coordinates far
+    outside the cell, and one molecule that the integer positions leave to the
+    FP64 chain (beyond 2^22 A)."""
+    rng = np.random.default_rng(44)
+    n = 500 // apm + 8
+    xs, _, cells = make_system(rng, TRICLINIC, n, apm, n, apm, 2, True, spread=0.5)
+    H = TRICLINIC
+    shift = rng.integers(-3, 4, size=(n, 3)) @ H.T
+    xs = xs + np.repeat(shift, apm, axis=0)[None]
+    frac = xs @ np.linalg.inv(H).T
+    split = np.arange(n * apm) % (2 * apm) < apm
+    xs[:, split] = ((frac - np.floor(frac)) @ H.T)[:, split]
+    if dtype == np.float64:
+        xs[1, -apm:] += 2.0**19 * H[:, 0]
+    got, ref, st = compare(cm, orc, ms=n, aps=apm, mv=n, apv=apm, xs=xs, xv=None, cells=cells, self_mode=True,
+                           precision="fp32", regime="pairs", irefatom=1, cutoff=5.0, dbulk=5.0, usecutoff=False, binstep=0.01,
+                           nbins=500, n_random_samples=40, seed=72, dtype=dtype)
+    assert ref["md_random"].sum() > 0 and st["guard_reevaluations"] > 0
