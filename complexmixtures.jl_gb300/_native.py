@@ -405,11 +405,8 @@ def raise_for(status: int, handle, server=None, batch=None) -> None:
 def csr(rows, nrows: int):
     """(offsets int64[nrows+1], values int32[]) from a list of int sequences."""
     off = np.zeros(nrows + 1, dtype=np.int64)
-    vals = []
-    for i in range(nrows):
-        r = rows[i]
-        off[i + 1] = off[i] + len(r)
-        vals.extend(int(g) for g in r)
+    np.cumsum([len(rows[i]) for i in range(nrows)], out=off[1:])
+    vals = [int(g) for i in range(nrows) for g in rows[i]]
     return off, np.asarray(vals if vals else [0], dtype=np.int32)
 
 

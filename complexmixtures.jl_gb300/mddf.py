@@ -151,7 +151,7 @@ def mddf(trajectory, solute=None, solvent=None, options: Optional[Options] = Non
         return _device_result(R, res, options, coordination_number_only)
     for k in ("md_count", "md_count_random", "rdf_count", "rdf_count_random", "solute_group_count",
               "solute_group_count_random", "solvent_group_count", "solvent_group_count_random"):
-        setattr(R, k, c[k].copy())
+        setattr(R, k, c[k])
     R.volume.total = c["volume_total"]
     return finalresults(R, options, coordination_number_only=coordination_number_only)
 

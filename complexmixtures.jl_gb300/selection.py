@@ -108,6 +108,18 @@ class AtomSelection:
                 out.append(g)
         return out
 
+    def _credit_rows(self, atoms: Sequence[int]) -> List[List[int]]:
+        """``groups_of_index`` of each atom, for sorted groups from one pass over
+        the groups: one search per atom and group takes 30 ms for a 4,000-atom
+        solute with a group per residue."""
+        if any(inds[k] > inds[k + 1] for inds in self.group_atom_indices for k in range(len(inds) - 1)):
+            return [self.groups_of_index(i) for i in atoms]
+        groups = {}
+        for g, inds in enumerate(self.group_atom_indices):
+            for i in dict.fromkeys(inds):
+                groups.setdefault(i, []).append(g)
+        return [list(groups.get(i, ())) for i in atoms]
+
     def solute_credit_table(self):
         """Per local atom of one molecule, the groups credited when that atom is
         the solute side of a minimum-distance pair, or None for default groups.
@@ -118,14 +130,14 @@ class AtomSelection:
         atoms of the selection's first molecule."""
         if not self.custom_groups:
             return None
-        return [self.groups_of_index(self.indices[a]) for a in range(self.natomspermol)]
+        return self._credit_rows(self.indices[: self.natomspermol])
 
     def solvent_credit_table(self):
         """Per atom of the whole selection, the groups credited when that atom
         is the solvent side of a pair (``md.j`` is global), or None."""
         if not self.custom_groups:
             return None
-        return [self.groups_of_index(i) for i in self.indices]
+        return self._credit_rows(self.indices)
 
     def __eq__(self, other):
         if not isinstance(other, AtomSelection):

@@ -98,7 +98,11 @@ class ArrayTrajectory(Trajectory):
 
     # bulk access used by the driver to hand many frames to the GPU at once
     def frame_arrays(self, idx: Sequence[int]):
+        """Coordinates and cells of the given frames (0-based); views of the
+        stored arrays when the frames are consecutive."""
         idx = np.asarray(idx, dtype=np.int64)
+        if idx.ndim == 1 and idx.size and idx[0] >= 0 and idx[-1] < self.nframes and np.all(np.diff(idx) == 1):
+            idx = slice(int(idx[0]), int(idx[-1]) + 1)
         return self._xs[idx], self._xv[idx], self._cells[idx]
 
 
