@@ -23,19 +23,20 @@
 // the guard test only asks that) and the reference site's smallest distance
 // are then the values a walk over every stencil cell gives, and every decision
 // follows the FP32 + guard rules of atoms_decide.  A query whose record lies
-// inside the guard band is decided in place from exact distances
-// (agrid_record), its exact scans reading the same lists, so the counts stay
-// the oracle's.
+// inside the guard band is listed for k_agrid_records, which decides it from
+// exact distances (agrid_record), its exact scans reading the same lists, so
+// the counts stay the oracle's.
 //
 // A list entry is the atom's FP32 position from the fine cell's search-cell
 // origin, q_a + off(cell_a - cell), which is the displacement form of the
 // ATOMS walks (the guard band's error bound covers it), and the atom's index
 // in the molecule.
 //
-// Kernels: k_agrid_build (the lists of every frame, one CTA per search cell,
-// space reserved in a per-frame pool; a frame whose pool runs out loses its
+// Kernels: k_agrid_build (the lists of every frame, one search cell near the
+// solute at a time per CTA, space reserved in a per-frame pool; a frame whose pool runs out loses its
 // grid), k_agrid_real (real pass) and k_agrid_random (random insertion: the
-// queries of the slots k_slot_filter listed and k_atoms_place placed).
+// queries of the slots k_slot_filter listed and k_atoms_place placed), each
+// followed by k_agrid_records.
 // Frames without a grid take the walk path: k_agrid_real queues their
 // molecule pairs for k_atoms_eval as k_atoms_filter does, and k_atoms_place
 // queues their slots.
@@ -46,9 +47,11 @@ namespace cmk {
 
 constexpr int kAgridMaxK = 6;          // fine cells per search-cell axis
 constexpr int kAgridBuckets = 8;       // each list ordered by bucket of the atom's smallest distance to the fine cell
-constexpr int kAgridStage = 3072;      // stencil atoms staged in shared memory at a time (48 KB, dynamic)
-constexpr int kAgridRound = 4;         // stencil atoms each thread loads per staging round
+static_assert(kAgridStarts == kAgridBuckets + 1, "starts of a list");
+constexpr int kAgridStage = 2560;      // stencil atoms staged in shared memory at a time (40 KB, dynamic)
+constexpr int kAgridRound = 2;         // stencil atoms each thread loads per staging round
 constexpr int kAgridBuildThreads = 256;
+constexpr int kAgridBuildCtas = 4;     // resident CTAs per SM (40 KB of stage and 12 KB more each, 61 registers a thread)
 constexpr int kAgridRecThreads = 32;   // k_agrid_records: a few records per SM,
 constexpr int kAgridRecLanes = 4;      // each on a group of lanes
 
@@ -76,14 +79,33 @@ __device__ __forceinline__ float fine_near2(const FineCells &fc, const float *c,
     return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
 
-// Lists of the fine cells of one search cell (grid: x = search cell, y =
-// frame), in one pass.  The CTA stages the cell's stencil atoms in shared
-// memory; each warp takes fine cells in turn and its lanes split the staged
-// atoms (warp reductions, and ballots for the compacted writes).  The CTA
-// counts its lists by bucket, reserves their room in the frame's entry pool
-// with one atomic, writes each fine cell's bucket starts and end to gstart and
-// its bucket edges to gedge, then the entries.  A frame whose pool runs out
-// loses its grid (its queries take the walk).
+// A square root for bucket numbers: its error (2 ulp) lies within the lists' slack.
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Lists of the fine cells of one search cell at a time, claimed by a resident
+// grid from the list of cells near the solute (k_atoms_near).  The CTA stages
+// the cell's stencil atoms in shared memory; each warp takes fine cells in
+// turn and its lanes split the staged atoms (warp reductions, and ballots for
+// the compacted writes).  The CTA counts its lists by bucket, reserves their
+// room in the frame's entry pool with one atomic, writes each fine cell's
+// bucket starts and end to gstart and its bucket edges to gedge, then the
+// entries.  A frame whose pool runs out loses its grid (its queries take the
+// walk).
+// Bound by instruction issue: each fine cell tests every staged atom three
+// times.  So (a) the grid holds only the near cells, one CTA per cell of the
+// box spent most of a sparse frame on cells with nothing to do; (b) stencil
+// cells farther than the own atoms' bound are dropped before their atoms are
+// loaded; (c) bucket positions stay in lanes 0 .. 7 and ballots find a
+// bucket's lanes, where match_any and a shared-memory update did.  us, before
+// and after: 20,000-atom chain in water 656 and 513, in 14-site cosolvent
+// 1,105 and 824, 24 systems of up to 10,000 atoms 3,234 and 1,741, 50 frames
+// of 2,150 atoms 723 and 568.  Four CTAs of 256 threads with 40 KB of stage
+// (rounds of two atoms a thread); three with 48 KB and rounds of four: 498,
+// 835, 1,955 and 617; four with 32 KB: 553, 901, 1,805 and 580.
 __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const dim3 gridDim, const DevSys &S, const Bufs &B) {
     extern __shared__ float4 s_at[];  // kAgridStage entries
     __shared__ int s_pre[kAgridMaxStencil + 1];
@@ -94,24 +116,24 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
     __shared__ int s_wsum[kAgridBuildThreads / 32];
     __shared__ int s_base;
     __shared__ float s_tmax;
-    const int f = blockIdx.y;
-    const int c = blockIdx.x;
-    const FrameGeom &G = B.G[f];
-    const FrameScratch &F = B.FS[f];
-    if (c >= G.ncell) return;
+    __shared__ FineCells s_fc;
+    __shared__ int s_item, s_cells;
     const int K = B.agk, K3 = K * K * K;
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
     const unsigned below = (1u << lane) - 1u;
+    const int nitems = B.counters[11], per_frame = (int)(B.gfs / K3);
+    for (;;) {
+    __syncthreads();  // the previous cell's shared arrays are read no more
+    if (t == 0) s_item = atomicAdd(B.counters + 12, 1);
+    __syncthreads();
+    if (s_item >= nitems) return;
+    const int item = B.galist[s_item];
+    const int f = item / per_frame, c = item - f * per_frame;
+    const FrameGeom &G = B.G[f];
+    const FrameScratch &F = B.FS[f];
     const int64_t gbase = ((int64_t)f * B.gfs + (int64_t)c * K3) * (kAgridBuckets + 1);  // bucket starts and end
     const int64_t ebase = (int64_t)f * B.gfs + (int64_t)c * K3;                            // fine-cell bucket edges
-    const bool active = F.agrid && B.anear[(int64_t)f * B.as + c];
-    if (!active) {
-        // no solute atom within a stencil of this cell: empty lists
-        for (int g = t; g < K3 * (kAgridBuckets + 1); g += blockDim.x) B.gstart[gbase + g] = 0;
-        for (int g = t; g < K3; g += blockDim.x) B.gedge[ebase + g] = make_float2(0.f, 0.f);
-        return;
-    }
     const int La0 = F.La[0], La1 = F.La[1], La2 = F.La[2];
     const int nx = 2 * La0 + 1, ny = 2 * La1 + 1, nst = nx * ny * (2 * La2 + 1);
     const int cx = c % G.n[0], cy = (c / G.n[0]) % G.n[1], cz = c / (G.n[0] * G.n[1]);
@@ -124,44 +146,33 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
         s_pre[i] = cs[cell + 1] - cs[cell];
         s_oi[i] = (short)off_index(dx, dy, dz);
     }
-    __syncthreads();
-    if (t < 32) {
-        // exclusive scan of the stencil cells' atom counts
-        int run = 0;
-        for (int i0 = 0; i0 < nst; i0 += 32) {
-            const int i = i0 + t;
-            const int v = i < nst ? s_pre[i] : 0;
-            int incl = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                if (t >= o) incl += u;
-            }
-            if (i < nst) s_pre[i] = run + incl - v;
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (t == 0) s_pre[nst] = run;
-    }
-    __syncthreads();
-    const int N = s_pre[nst];
     const float4 *aq = B.asq32 + (int64_t)f * B.Ns;
     const float4 *off = B.off32 + (int64_t)f * kOffEntries;
+    if (t == 0) {
+        s_fc = F.fcells;  // the frame's fine-cell geometry (k_frame_consts)
+        s_tmax = 0.f;
+    }
+    for (int g = t; g < K3; g += blockDim.x) {
+        s_far[g] = INFINITY;
+        s_near[g] = INFINITY;
+    }
+    __syncthreads();
+    int N = 0, ncells = 0;  // atoms and cells of the stencil that are kept (below)
     // stencil atom kk: its position from this cell's origin
+    auto atom_of = [&](int cell, int k) {
+        const float4 q = aq[s_beg[cell] + k];
+        const float4 o = off[s_oi[cell]];
+        return make_float4(q.x + o.x, q.y + o.y, q.z + o.z, q.w);
+    };
     auto atom_at = [&](int kk) {
-        int lo = 0, hi = nst - 1;
+        int lo = 0, hi = ncells - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
             if (s_pre[mid] <= kk) lo = mid;
             else hi = mid - 1;
         }
-        const float4 q = aq[s_beg[lo] + (kk - s_pre[lo])];
-        const float4 o = off[s_oi[lo]];
-        return make_float4(q.x + o.x, q.y + o.y, q.z + o.z, q.w);
+        return atom_of(lo, kk - s_pre[lo]);
     };
-    // the frame's fine-cell geometry (k_frame_consts), shared
-    __shared__ FineCells s_fc;
-    if (t == 0) s_fc = F.fcells;
-    __syncthreads();
     const FineCells fc = s_fc;
     auto centre = [&](int g, float *cen) {
         const float u0 = ((float)(g % K) + 0.5f), u1 = ((float)((g / K) % K) + 0.5f), u2 = ((float)(g / (K * K)) + 0.5f);
@@ -240,22 +251,16 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
     // the list threshold and bucket edges of fine cell g from its bounds
     auto thresh = [&](int g) { return fminf(fc.ortho ? sqrtf(s_far[g]) : sqrtf(s_far[g]) + fc.R, cut) + margin; };
     auto lowest = [&](int g) { return fc.ortho ? sqrtf(s_near[g]) : fmaxf(sqrtf(s_near[g]) - fc.R, 0.f); };
-    if (t == 0) s_tmax = 0.f;
     int kept = -1;  // atoms of pass 1 still staged (-1 none yet, -2 several stages)
     {
-        for (int g = t; g < K3; g += blockDim.x) {
-            s_far[g] = INFINITY;
-            s_near[g] = INFINITY;
-        }
         // the search cell's own atoms first: each fine cell's bound from them
         // limits the stencil atoms that can matter to those within the
         // largest bound of the cell (dense solutes: a few Angstrom)
-        const int own = (La2 * ny + La1) * nx + La0;
-        const int own_beg = s_pre[own], own_n = s_pre[own + 1] - s_pre[own];
+        const int own = (La2 * ny + La1) * nx + La0, own_n = s_pre[own];
         for (int k0 = 0; k0 < own_n; k0 += kAgridStage) {
             const int nb = min(kAgridStage, own_n - k0);
             __syncthreads();
-            for (int k = t; k < nb; k += blockDim.x) s_at[k] = atom_at(own_beg + k0 + k);
+            for (int k = t; k < nb; k += blockDim.x) s_at[k] = atom_of(own, k0 + k);
             __syncthreads();
             for (int g = warp; g < K3; g += nwarps) {
                 float cen[3];
@@ -270,6 +275,46 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
         for (int g = t; g < K3; g += blockDim.x) atomicMax((int *)&s_tmax, __float_as_int(thresh(g)));
         __syncthreads();
         const float thr1 = s_tmax + slack;
+        // the stencil cells that hold atoms and (orthogonal cells) reach
+        // within thr1 of this one, moved to the front; s_pre becomes the
+        // exclusive scan of their counts
+        if (t < 32) {
+            int run = 0, cells = 0;
+            for (int i0 = 0; i0 < nst; i0 += 32) {
+                const int i = i0 + t;
+                int v = i < nst ? s_pre[i] : 0;
+                const int beg = i < nst ? s_beg[i] : 0;
+                const short oi = i < nst ? s_oi[i] : (short)0;
+                if (v > 0 && fc.ortho) {
+                    const int dx = i % nx - La0, dy = (i / nx) % ny - La1, dz = i / (nx * ny) - La2;
+                    const float gx = fmaxf((float)abs(dx) - 1.f, 0.f) * fabsf(fc.e[0]), gy = fmaxf((float)abs(dy) - 1.f, 0.f) * fabsf(fc.e[4]),
+                                gz = fmaxf((float)abs(dz) - 1.f, 0.f) * fabsf(fc.e[8]);
+                    if (sqrtf(fmaf(gz, gz, fmaf(gy, gy, gx * gx))) * (float)K > thr1 + slack) v = 0;
+                }
+                int incl = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (t >= o) incl += u;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, v > 0);
+                if (v > 0) {
+                    const int at = cells + __popc(m & below);  // at most i: read above
+                    s_pre[at] = run + incl - v;
+                    s_beg[at] = beg;
+                    s_oi[at] = oi;
+                }
+                cells += __popc(m);
+                run += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            if (t == 0) {
+                s_pre[cells] = run;
+                s_cells = cells;
+            }
+        }
+        __syncthreads();
+        ncells = s_cells;
+        N = s_pre[ncells];
         // pass 1: an upper bound of the nearest atom's distance over each fine
         // cell, and the smallest distance of any atom to it
         int cursor = 0;
@@ -317,7 +362,9 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
     float4 *ent = B.gent + (int64_t)f * B.gcap;
     // one stage of atoms through every fine cell: lane k of a group of 32
     // tests atom k; counting sums the buckets, filling writes each bucket's
-    // atoms in stage order after its start
+    // atoms in stage order after its start.  Lane b < 8 keeps the position of
+    // bucket b, and three ballots of the bucket's bits give every lane the
+    // lanes of any bucket.
     auto pass2 = [&](int nb, bool fill) {
         for (int g = warp; g < K3; g += nwarps) {
             float cen[3];
@@ -326,32 +373,27 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
             LT(g, L, T);
             const float lim2 = fc.ortho ? T * T : (T + fc.R) * (T + fc.R);
             const float inv = T > L ? (float)kAgridBuckets / (T - L) : 0.f;
+            int pos = s_pos[g][lane & (kAgridBuckets - 1)];
             for (int k0 = 0; k0 < nb; k0 += 32) {
                 const int k = k0 + lane;
-                int bk = -1;
-                float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (k < nb) {
-                    p = s_at[k];
-                    const float d2 = fine_near2(fc, cen, p);
-                    if (d2 <= lim2) {
-                        const float dmin = fc.ortho ? sqrtf(d2) : fmaxf(sqrtf(d2) - fc.R, 0.f);
-                        bk = min(kAgridBuckets - 1, max(0, (int)((dmin - L) * inv)));
-                    }
+                const float4 p = s_at[min(k, nb - 1)];
+                const float d2 = fine_near2(fc, cen, p);
+                const bool in = k < nb && d2 <= lim2;
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                if (m == 0u) continue;
+                const float d = sqrt_approx(d2);
+                const int bk = min(kAgridBuckets - 1, max(0, (int)(((fc.ortho ? d : fmaxf(d - fc.R, 0.f)) - L) * inv)));
+                const unsigned b0 = __ballot_sync(0xffffffffu, bk & 1), b1 = __ballot_sync(0xffffffffu, bk & 2),
+                               b2 = __ballot_sync(0xffffffffu, bk & 4);
+                auto of = [&](int q) { return m & (q & 1 ? b0 : ~b0) & (q & 2 ? b1 : ~b1) & (q & 4 ? b2 : ~b2); };
+                if (fill) {
+                    const int at = __shfl_sync(0xffffffffu, pos, bk) + __popc(of(bk) & below);
+                    if (in) ent[at] = p;
                 }
-                if (!__any_sync(0xffffffffu, bk >= 0)) continue;
-                // the lanes of each bucket: the lowest one advances the
-                // bucket's position, the others write after it in lane order
-                const unsigned m = __match_any_sync(0xffffffffu, bk);
-                const int leader = __ffs(m) - 1;
-                int at = 0;
-                if (bk >= 0 && lane == leader) {
-                    at = s_pos[g][bk];
-                    s_pos[g][bk] = at + __popc(m);
-                }
-                at = __shfl_sync(0xffffffffu, at, leader);
-                if (fill && bk >= 0) ent[at + __popc(m & below)] = p;
-                __syncwarp();
+                pos += __popc(of(lane));
             }
+            __syncwarp();
+            if (lane < kAgridBuckets) s_pos[g][lane] = pos;
         }
     };
     // pass 1's single stage holds every atom that passes thr2 (thr2 <= thr1),
@@ -406,7 +448,7 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
         }
     }
     __syncthreads();
-    if (s_base < 0) return;
+    if (s_base < 0) continue;
     if (t < K3) {
         const int start = s_base + wbefore + incl - tot;
         int *st = B.gstart + gbase + (int64_t)t * (kAgridBuckets + 1);
@@ -419,9 +461,10 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
     }
     __syncthreads();
     sweep(true);
+    }
 }
 
-__global__ void __launch_bounds__(kAgridBuildThreads, 3) k_agrid_build(DevSys S, Bufs B) {
+__global__ void __launch_bounds__(kAgridBuildThreads, kAgridBuildCtas) k_agrid_build(DevSys S, Bufs B) {
     k_agrid_build_body(blockIdx, gridDim, S, B);
 }
 

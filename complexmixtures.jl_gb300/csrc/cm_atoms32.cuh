@@ -43,22 +43,37 @@ __device__ __forceinline__ void k_atoms_near_body(const uint3 blockIdx, const di
     const FrameGeom &G = B.G[f];
     const FrameScratch &F = B.FS[f];
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)B.ms * G.ncell) return;
-    const int s = (int)(t / G.ncell), cell = (int)(t - (int64_t)s * G.ncell);
-    const int *cs = B.astart + (int64_t)f * B.as + (int64_t)s * G.ncell;
-    const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
-    const int cx = cell % n0, cy = (cell / n0) % n1, cz = cell / (n0 * n1);
+    const int64_t n = (int64_t)B.ms * G.ncell;
     unsigned char near = 0;
-    for (int dz = -F.La[2]; dz <= F.La[2] && !near; ++dz)
-        for (int dy = -F.La[1]; dy <= F.La[1] && !near; ++dy)
-            for (int dx = -F.La[0]; dx <= F.La[0]; ++dx) {
-                const int c = (wrap_cell(cz + dz, n2) * n1 + wrap_cell(cy + dy, n1)) * n0 + wrap_cell(cx + dx, n0);
-                if (cs[c + 1] > cs[c]) {
-                    near = 1;
-                    break;
+    if (t < n) {
+        const int s = (int)(t / G.ncell), cell = (int)(t - (int64_t)s * G.ncell);
+        const int *cs = B.astart + (int64_t)f * B.as + (int64_t)s * G.ncell;
+        const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
+        const int cx = cell % n0, cy = (cell / n0) % n1, cz = cell / (n0 * n1);
+        for (int dz = -F.La[2]; dz <= F.La[2] && !near; ++dz)
+            for (int dy = -F.La[1]; dy <= F.La[1] && !near; ++dy)
+                for (int dx = -F.La[0]; dx <= F.La[0]; ++dx) {
+                    const int c = (wrap_cell(cz + dz, n2) * n1 + wrap_cell(cy + dy, n1)) * n0 + wrap_cell(cx + dx, n0);
+                    if (cs[c + 1] > cs[c]) {
+                        near = 1;
+                        break;
+                    }
                 }
-            }
-    B.anear[(int64_t)f * B.as + t] = near;
+        B.anear[(int64_t)f * B.as + t] = near;
+    }
+    if (B.agk == 0) return;
+    // candidate grid (one solute molecule: t is the cell): the near cells are
+    // listed for k_agrid_build, and the warp clears the lists of its cells
+    const int lane = threadIdx.x & 31, K3 = B.agk * B.agk * B.agk;
+    const unsigned m = __ballot_sync(0xffffffffu, near && F.agrid);
+    int at = 0;
+    if (lane == 0 && m) at = atomicAdd(B.counters + 11, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if ((m >> lane) & 1u) B.galist[at + __popc(m & ((1u << lane) - 1u))] = f * (int)(B.gfs / K3) + (int)t;
+    const int64_t t0 = t - lane;
+    const int starts = K3 * kAgridStarts * (int)max((int64_t)0, min((int64_t)32, n - t0));
+    int *st = B.gstart + ((int64_t)f * B.gfs + t0 * K3) * kAgridStarts;
+    for (int i = lane; i < starts; i += 32) st[i] = 0;
 }
 
 __global__ void k_atoms_near(Bufs B) {

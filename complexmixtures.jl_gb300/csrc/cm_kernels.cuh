@@ -48,6 +48,7 @@ constexpr int kMaxSmallMol = 32;  // PAIRS regime: atoms per molecule on either 
 constexpr int kWarps = 8;         // warps per CTA of the PAIRS real-pass kernels
 constexpr int kQueue = 64;        // per-warp candidate queue
 constexpr int kTileCells = 128;   // half-stencil cells the tiled real pass stages per home cell
+constexpr int kAgridStarts = 9;        // a candidate-grid list's bucket starts and its end
 constexpr int kAgridMaxStencil = 343;  // ATOMS stencil cells the candidate-grid build stages (half-widths up to 3)
 
 enum : int { ERR_STENCIL = 1, ERR_BIN = 2, ERR_QUEUE = 4, ERR_SIZE = 8 };
@@ -132,7 +133,7 @@ struct FrameScratch {
     int La[3];      // ATOMS stencil half-widths
     float xmax;     // largest |coordinate component| of the frame's input atoms (rounded up)
     int tile;       // self mode, one image per pair, half stencil within kTileCells: the tiled real pass takes the frame
-    int agrid;      // ATOMS, one solute molecule: the frame's candidate grid is complete (k_agrid_scan clears it on overflow)
+    int agrid;      // ATOMS, one solute molecule: the frame's candidate grid is complete (k_agrid_build clears it on overflow)
     FineCells fcells;  // the candidate grid's fine cells (when agrid)
     int place32;    // ATOMS, FP32 search: random-insertion slots placed in FP32 (placed_store32), the band widened to match
     FixedGeom fx;   // integer positions of the FP32 search's prep (k_offtable)
@@ -440,6 +441,7 @@ struct Bufs {
     int64_t gfs;                    // fine cells per frame (ncell_cap * agk^3)
     int64_t gcap;                   // entries per frame
     int *gstart;                    // [nf][gfs][buckets + 1]: each fine cell's bucket starts and its end
+    int *galist;                    // search cells near the solute (frame * ncell_cap + cell); count in counters[11]
     int *gpool;                     // [nf]: entries reserved in the frame's pool
     float2 *gedge;                  // [nf][gfs]: smallest distance of a listed atom to the fine cell, list threshold
     float4 *gent;                   // [nf][gcap]: position from the fine cell's search-cell origin, solute atom index

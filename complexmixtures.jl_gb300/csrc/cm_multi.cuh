@@ -125,11 +125,11 @@ __device__ __forceinline__ void mk_body(const uint3 vb, const dim3 vg, const MAr
 }
 
 // Two resident CTAs per SM for the stages of up to 256 threads (four for the
-// candidate-grid queries, as their stand-alone kernels): the arguments now
+// candidate-grid queries and lists, as their stand-alone kernels): the arguments now
 // come from the work table instead of the parameter space, and the register
 // budget of the stand-alone kernels is kept.
 __host__ __device__ constexpr int mk_min_ctas(int kid) {
-    return mk_query(kid) ? 4 : mk_threads(kid) <= 256 ? 2 : 1;
+    return mk_query(kid) ? 4 : kid == MK_AGRID_BUILD ? kAgridBuildCtas : mk_threads(kid) <= 256 ? 2 : 1;
 }
 
 template <int KID>

@@ -165,7 +165,7 @@ BlockCache &blocks() {
     return *c;
 }
 
-constexpr int kCounters = 12;  // ints of Bufs::counters
+constexpr int kCounters = 14;  // ints of Bufs::counters
 constexpr size_t kOutChunk = size_t(512) << 10;  // bytes of a pinned read-out buffer
 
 // Random samples placed per launch in the ATOMS layout.  FP64, or under an HBM
@@ -236,7 +236,7 @@ struct cm_handle {
     int atoms_piece = 0;   // samples placed per random-insertion launch
     // candidate grid of a single solute molecule (FP32): agk fine cells per
     // search-cell axis (0: none), gcap entries per frame
-    DevBuf gstart, gedge, gpool, gent;
+    DevBuf gstart, gedge, gpool, galist, gent;
     int agk = 0;
     int64_t gcap = 0;
     int agrid_real_ctas = 1, agrid_rand_ctas = 1;  // resident CTAs per SM of k_agrid_real / k_agrid_random
@@ -807,6 +807,7 @@ void ensure_cells(cm_handle *h, int64_t ncell) {
             dev_alloc(h, h->gstart, (size_t)h->fc * ncell * k3 * (kAgridBuckets + 1) * 4);
             dev_alloc(h, h->gedge, (size_t)h->fc * ncell * k3 * sizeof(float2));
             dev_alloc(h, h->gpool, (size_t)h->fc * 4);
+            dev_alloc(h, h->galist, (size_t)h->fc * ncell * 4);
             if (h->mddf) dev_alloc(h, h->scount, (size_t)h->fc * ncell * k3 * 4);
         }
     }
@@ -977,7 +978,6 @@ void plan(cm_handle *h, const cm_frames *f) {
         const int64_t asked = mv * (1 + (h->mddf ? (int64_t)d.n_random_samples : 0));
         const bool pays = (d.solvent_natomspermol <= 4 && asked >= 4 * h->Ns) ||
                           (d.solvent_natomspermol <= kMaxSmallMol && asked * d.solvent_natomspermol >= 8 * h->Ns);
-        (void)dense;
         const bool want = d.atoms_grid > 0 || (d.atoms_grid == 0 && pays);
         if (want && fp32 && ms == 1 && !d.autocorrelation && (int64_t)fc * mv <= h->aq_cap) {
             int K = d.atoms_grid > 0 ? d.atoms_grid : (int)std::ceil(target_cell(h) / 4.5);
@@ -1166,6 +1166,7 @@ Bufs chunk_bufs(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample 
             B.gcap = h->gcap;
             B.gstart = P<int>(h->gstart);
             B.gpool = P<int>(h->gpool);
+            B.galist = P<int>(h->galist);
             B.gedge = P<float2>(h->gedge);
             B.gent = P<float4>(h->gent);
             B.skey = P<int2>(h->skey);
@@ -1343,8 +1344,10 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
     };
     if (agrid) {
         // the single solute molecule's candidate lists of every frame
+        // (counters[11 .. 12]: the near cells, the next one)
         em.zero(B.gpool, (size_t)nf * sizeof(int));
-        em.kernel(MK_AGRID_BUILD, dim3(c.ncell_max, nf), (size_t)kAgridStage * sizeof(float4), CM_K_CELLS, base);
+        em.kernel(MK_AGRID_BUILD, dim3((unsigned)std::min<int64_t>((int64_t)c.ncell_max * nf, (int64_t)sms * kAgridBuildCtas)),
+                  (size_t)kAgridStage * sizeof(float4), CM_K_CELLS, base);
         // real pass: every solvent molecule queried (records inside the band
         // decided in place); frames without a grid go to the evaluation queue.
         // counters[6 .. 7]: the queries' next molecule (zeroed with the chunk's counters)
@@ -1964,7 +1967,7 @@ void free_all(cm_handle *h) {
                      &h->vo32, &h->vo64, &h->u64, &h->u32, &h->rc, &h->ccount, &h->cstart, &h->cfill, &h->cmol, &h->cq32, &h->gq, &h->eq, &h->rq, &h->rq2, &h->akey, &h->atq32,
                      &h->atq64, &h->asq32, &h->asq64, &h->acount, &h->astart, &h->afill, &h->avcell, &h->avq32, &h->avq64,
                      &h->pcell, &h->pq32, &h->pq64, &h->anear, &h->aq, &h->g_soff, &h->g_sidx, &h->g_voff, &h->g_vidx,
-                     &h->aslot, &h->skey, &h->adefer, &h->sslot, &h->scount, &h->gstart, &h->gedge, &h->gpool, &h->gent, &h->dcd_sidx, &h->dcd_vidx, &h->dcd_raw[0], &h->dcd_raw[1], &h->final_out, &h->final_job,
+                     &h->aslot, &h->skey, &h->adefer, &h->sslot, &h->scount, &h->gstart, &h->gedge, &h->gpool, &h->galist, &h->gent, &h->dcd_sidx, &h->dcd_vidx, &h->dcd_raw[0], &h->dcd_raw[1], &h->final_out, &h->final_job,
                      &h->contrib_q, &h->contrib_g, &h->contrib_out};
     for (DevBuf *b : all) {
         blocks().put(h->device, false, b->p, b->bytes);
