@@ -892,9 +892,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, CM_TILE_MIN_CTAS) k_pairs_til
 // staged table changes.  The test of a home molecule against the staged
 // table is |w - q|^2 <= R^2 as |w|^2 / 2 - w q <= (R^2 - |q|^2) / 2, three
 // multiply-adds on a staged (w, |w|^2 / 2), R the reach of the largest
-// molecule of the frame; its rounding (4 u (|w|^2 / 2 + |w| |q|), under 2e-3
-// A^2 for cells of 25 A) is far inside the margin of cut_pre (R times 1e-3 (1 +
-// range), 0.15 A^2 for water).  A lane keeps its hits of up to 32 rounds in a
+// molecule of the frame; its rounding (under 2e-3 A^2 for cells of 25 A) is far
+// inside the margin of cut_pre (R times 1e-3 (1 + range), 0.15 A^2 for water),
+// and a frame of much wider cells is left to k_pairs_flat32 (FrameScratch::tile).  A lane keeps its hits of up to 32 rounds in a
 // bit mask; the masks are compacted into the queue afterwards.  The distances
 // are formed as in flat_flush, so the records and the queues are the same.
 // 19,338 waters, cutoff 10 A, 16 frames: 1,979 us in k_pairs_tile32, 746 here

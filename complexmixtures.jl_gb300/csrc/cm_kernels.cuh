@@ -132,7 +132,8 @@ struct FrameScratch {
     int multi;      // PAIRS axes with several images (bit k set for axis k)
     int La[3];      // ATOMS stencil half-widths
     float xmax;     // largest |coordinate component| of the frame's input atoms (rounded up)
-    int tile;       // self mode, one image per pair, half stencil within kTileCells: the tiled real pass takes the frame
+    int tile;       // self mode, one image per pair, half stencil within kTileCells, cells not far wider than the search
+                    // range: the tiled real pass takes the frame
     int agrid;      // ATOMS, one solute molecule: the frame's candidate grid is complete (k_agrid_build clears it on overflow)
     FineCells fcells;  // the candidate grid's fine cells (when agrid)
     int place32;    // ATOMS, FP32 search: random-insertion slots placed in FP32 (placed_store32), the band widened to match
@@ -1883,6 +1884,9 @@ __device__ __forceinline__ void k_frame_consts_body(const uint3 blockIdx, const 
         F.gr = g;
         return;
     }
+    // the tiled kernels test |w|^2 / 2 - w q for a staged position w (at most Q + OFF long) and a home position q
+    // (at most Q): with the threshold it is within 16 u (Q + OFF)^2, which half the margin of cut_pre has to cover
+    if (16.0 * u * (Q + OFF) * (Q + OFF) > 0.5 * range * (1e-3 * (1.0 + range) - g.delta)) F.tile = 0;
     F.g = g;
     // the FP64 search: the same rules with band eps
     Guard64 g64;
