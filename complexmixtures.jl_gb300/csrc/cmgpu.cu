@@ -175,11 +175,12 @@ constexpr size_t kOutChunk = size_t(512) << 10;  // bytes of a pinned read-out b
 // end on their slowest warps and on the latency of its few exact records, so
 // fewer and larger pieces are faster.
 constexpr int64_t kPieceSlots = 1 << 22;
+constexpr int64_t kPieceSamples = 65535;  // a piece's samples are the y axis of k_slot_filter's grid
 int chunk_samples(const cm_system_desc &d) {
     if (d.precision != CM_PRECISION_FP32_GUARD) return 32;
     const int64_t apv = d.solvent_natomspermol;
     const int64_t fit = 32 * (52 * apv + 20) / (20 * apv + 36);
-    return (int)(d.hbm_budget_bytes > 0 ? fit : std::max(fit, kPieceSlots / d.solvent_nmols));
+    return (int)(d.hbm_budget_bytes > 0 ? fit : std::max(fit, std::min(kPieceSlots / d.solvent_nmols, kPieceSamples)));
 }
 
 // Lanes per candidate-grid query (k_agrid_real, k_agrid_random).
