@@ -941,13 +941,14 @@ __device__ __forceinline__ void warp_max_pos(float *addr, float v) {
 }
 
 // PAIRS prep, one thread per molecule (grid y = frame).  The molecule is made
-// whole around its first atom (minimum image of each atom's displacement), its
-// centroid c = x_0 + mean(d) is binned, and its atoms are stored as FP64 and
+// whole around atom ref (minimum image of each atom's displacement; the solvent
+// reference atom, as exact_unwrapped does for the random insertion), its
+// centroid c = x_ref + mean(d) is binned, and its atoms are stored as FP64 and
 // FP32 offsets from the centroid; the radius is the largest offset (rounded
 // up).  Displacements shorter than 0.45 of the narrowest cell width are their
 // own minimum image, so the FP64 unwrap runs only for longer ones.
 template <typename T>
-__global__ void k_prep_pairs(Bufs B, const T *__restrict__ xyz, int64_t xyz_stride, int solvent_side, int count_cells) {
+__global__ void k_prep_pairs(Bufs B, const T *__restrict__ xyz, int64_t xyz_stride, int solvent_side, int count_cells, int ref) {
     const int f = blockIdx.y;
     const int nmol = (int)(solvent_side ? B.mv : B.ms);
     const int64_t Nmol_atoms = solvent_side ? B.Nv : B.Ns;
@@ -964,7 +965,7 @@ __global__ void k_prep_pairs(Bufs B, const T *__restrict__ xyz, int64_t xyz_stri
     const T *x = xyz + (int64_t)f * xyz_stride + (int64_t)m * apm * 3;
     const int64_t base = (int64_t)m * apm;
     double x0[3];
-    load_xyz(x, x0);
+    load_xyz(x + 3 * ref, x0);
     const float wlim = (float)(0.45 * fmin(G.w[0], fmin(G.w[1], G.w[2])));
     double sx = 0.0, sy = 0.0, sz = 0.0, xm = 0.0;
     for (int a = 0; a < apm; ++a) {
@@ -1012,7 +1013,7 @@ __global__ void k_prep_pairs(Bufs B, const T *__restrict__ xyz, int64_t xyz_stri
 // frames: 547 us with the FP64 chain, 198 here.
 template <typename T>
 __global__ void __launch_bounds__(128) k_prep_pairs32(Bufs B, const T *__restrict__ xyz, int64_t xyz_stride, int solvent_side,
-                                                      int count_cells) {
+                                                      int count_cells, int ref) {
     const int f = blockIdx.y;
     const int nmol = (int)(solvent_side ? B.mv : B.ms);
     const int64_t Nmol_atoms = solvent_side ? B.Nv : B.Ns;
@@ -1029,8 +1030,8 @@ __global__ void __launch_bounds__(128) k_prep_pairs32(Bufs B, const T *__restric
     bool ok = X.set && !X.bad;
     int64_t x0[3] = {0, 0, 0}, sum[3] = {0, 0, 0};
     if (ok)
-        for (int k = 0; k < 3; ++k) ok = fixed_of(x[k], x0[k]) && ok;
-    // displacement of atom a from the first one, made its minimum image
+        for (int k = 0; k < 3; ++k) ok = fixed_of(x[3 * ref + k], x0[k]) && ok;
+    // displacement of atom a from atom ref, made its minimum image
     auto displacement = [&](int a, int64_t *d) {
         bool good = true;
         for (int k = 0; k < 3; ++k) {
@@ -1059,7 +1060,7 @@ __global__ void __launch_bounds__(128) k_prep_pairs32(Bufs B, const T *__restric
         }
     } else {
         double xd0[3], s[3] = {0.0, 0.0, 0.0}, qd[3];
-        load_xyz(x, xd0);
+        load_xyz(x + 3 * ref, xd0);
         auto disp = [&](int a, double *d) {
             double xa[3];
             load_xyz(x + 3 * a, xa);

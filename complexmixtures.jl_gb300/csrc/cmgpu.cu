@@ -1427,8 +1427,9 @@ void run_chunk(cm_handle *h, const Chunk &c, const FrameGeom *dG, const Sample *
         CM_CUDA(cudaMemsetAsync(B.ccount, 0, (size_t)nf * B.cs * 4, st));
         // solute molecules (in self mode they also fill the cell counts)
         auto prep = [&](const T *x, int64_t stride, int64_t n, int side, int count) {
-            if (fp32) CM_LAUNCH(CM_K_PREP, k_prep_pairs32<T><<<dim3(grid_for(n, 128), nf), 128, 0, st>>>(B, x, stride, side, count));
-            else CM_LAUNCH(CM_K_PREP, k_prep_pairs<T><<<dim3(grid_for(n, 128), nf), 128, 0, st>>>(B, x, stride, side, count));
+            const int ref = self || side == 1 ? S.iref : 0;
+            if (fp32) CM_LAUNCH(CM_K_PREP, k_prep_pairs32<T><<<dim3(grid_for(n, 128), nf), 128, 0, st>>>(B, x, stride, side, count, ref));
+            else CM_LAUNCH(CM_K_PREP, k_prep_pairs<T><<<dim3(grid_for(n, 128), nf), 128, 0, st>>>(B, x, stride, side, count, ref));
         };
         prep(xs, xs_stride, ms, 0, self ? 1 : 0);
         if (!self) prep(xv, xv_stride, mv, 1, 1);
@@ -2154,8 +2155,8 @@ void noalloc_run(cm_handle *h, const cm_frames *f, cudaStream_t stream) {
         Chunk one;
         one.nf = 1;
         const Bufs B = chunk_bufs(h, one, dG, nullptr);
-        k_prep_pairs<T><<<grid_for(d.solute_nmols, 128), 128, 0, stream>>>(B, xs, h->Ns * 3, 0, 0);
-        if (!d.autocorrelation) k_prep_pairs<T><<<grid_for(d.solvent_nmols, 128), 128, 0, stream>>>(B, xv, h->Nv * 3, 1, 0);
+        k_prep_pairs<T><<<grid_for(d.solute_nmols, 128), 128, 0, stream>>>(B, xs, h->Ns * 3, 0, 0, d.autocorrelation ? d.irefatom - 1 : 0);
+        if (!d.autocorrelation) k_prep_pairs<T><<<grid_for(d.solvent_nmols, 128), 128, 0, stream>>>(B, xv, h->Nv * 3, 1, 0, d.irefatom - 1);
         CM_CUDA(cudaGetLastError());
     }
     FrameScratch F;
