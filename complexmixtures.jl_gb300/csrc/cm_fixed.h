@@ -173,4 +173,14 @@ CM_HD int64_t fixed_mean(int64_t sum, int n) {
     return sum < 0 ? v - (int64_t)r : v;
 }
 
+// Bounds of the FP32 search's displacement components in units of u = 2^-24
+// (k_frame_consts): of an atom pair of the search, and what a slot of the
+// random insertion adds when it is placed in FP32 (r: the molecule radius) or
+// in FP64 from the molecule's FP32 offsets (their rounding, rotated).
+CM_HD double fp32_pair_units(double Q, double OFF, double rs, double rv, double cut) {
+    return (5.0 * Q + 4.0 * OFF + 2.0 * rv + rs + cut + 1.0) * (1.0 + 0x1.0p-19);
+}
+CM_HD double fp32_slot_units(double Q, double r) { return 5.0 * Q + 44.0 * r; }
+CM_HD double fp32_offset_units(double r) { return r * (1.0 + 0x1.0p-19); }
+
 }  // namespace cmgeom

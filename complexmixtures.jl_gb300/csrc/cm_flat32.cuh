@@ -1356,8 +1356,7 @@ __global__ void __launch_bounds__(kGuardWarps * 32) k_pairs_guard(DevSys S, Bufs
 }
 
 // The random-insertion slots inside k_random_fast's band (rq2), one warp per
-// slot: placed in FP64 (the narrow band: k_random_eval's argument for the FP32
-// offsets), the pairs and the molecule's atoms split over the lanes, and
+// slot: placed in FP64 from the FP32 offsets (the narrow band gp), the pairs and the molecule's atoms split over the lanes, and
 // decided by decide_warp.  One thread per slot waited 360 us for its chain of
 // FP64 operations (14-atom molecules), whatever the number of slots.
 __global__ void __launch_bounds__(kGuardWarps * 32) k_random_records(DevSys S, Bufs B) {
@@ -1421,7 +1420,7 @@ __global__ void __launch_bounds__(kGuardWarps * 32) k_random_records(DevSys S, B
         Pass32 P;
         pass32_warp<false>(S, Pf.off32, im, qs32, qv32, s_os[warp], s_ov[warp], pi, total, lane, P);
         DirRec r1, r2;
-        decide_warp<false>(S, G, B, X, F.g, P, Pf.off32, im, qs32, qv32, s_os[warp], s_ov[warp], s, k, pi, total, lane, r1, r2,
+        decide_warp<false>(S, G, B, X, F.gp, P, Pf.off32, im, qs32, qv32, s_os[warp], s_ov[warp], s, k, pi, total, lane, r1, r2,
                            st);
         if (lane == 0 && r1.within) {
             apply_hit_local(S, h, true, r1.bin, r1.i_local, r1.j, (int)(r1.j - (int64_t)k * apv), r1.ref, r1.rbin);

@@ -140,6 +140,7 @@ struct FrameScratch {
     FixedGeom fx;   // integer positions of the FP32 search's prep (k_offtable)
     Guard g;        // FP32 search
     Guard gr;       // FP32 random insertion of the PAIRS layout: slots placed in FP32 (k_random_fast)
+    Guard gp;       // ... and slots placed in FP64 from the FP32 offsets (k_random_records, k_random_eval)
     Guard64 g64;    // FP64 search
 };
 
@@ -1688,8 +1689,7 @@ __global__ void __launch_bounds__(128) k_random_eval(DevSys S, Bufs B) {
         st.molpairs++;
         st.atompairs += (unsigned long long)S.aps * S.apv * image_count(im);
         if (FP32) {
-            // the FP32 offsets, rotated in FP64: each coordinate within 2 u r_v of the rotated FP64 offset,
-            // u r_v more than the band's bound counts and well inside its 25 % (E is at least 6 u r_v)
+            // the FP32 offsets, rotated in FP64: each coordinate within 2 u r_v of the rotated FP64 offset (band gp)
             float4 ov32[kMaxSmallMol];
             const float4 *o = Pf.vo32 + (int64_t)P.jmol * S.apv;
             for (int b = 0; b < S.apv; ++b) {
@@ -1703,7 +1703,7 @@ __global__ void __launch_bounds__(128) k_random_eval(DevSys S, Bufs B) {
             const float4 *os32 = Pf.so32 + (int64_t)s * S.aps;
             Pass32 Q;
             pairs_pass<false>(S, Pf.off32, im, qs32, qp32, os32, (const float4 *)ov32, Q);
-            pairs_decide<false>(S, G, B, X, F.g, Q, Pf.off32, im, qs32, qp32, os32, (const float4 *)ov32, s, k, r1, r2, st);
+            pairs_decide<false>(S, G, B, X, F.gp, Q, Pf.off32, im, qs32, qp32, os32, (const float4 *)ov32, s, k, r1, r2, st);
         } else {
             d4 ov64[kMaxSmallMol];
             const d4 *o = Pf.vo64 + (int64_t)P.jmol * S.apv;
@@ -1761,7 +1761,11 @@ __device__ __forceinline__ FineCells fine_cells(const FrameGeom &G, const FrameS
 // atom of the random insertion is no rounding of an FP64 value: placed_store32
 // forms it in FP32 within u (5Q + 41 r_c) of the FP64 placement (r_c the
 // largest centroid radius), and E adds u (5Q + 44 r_c) in the frames that
-// place in FP32 (F.place32).  The distance is within
+// place in FP32 (F.place32).  In the molecule layout k_random_fast's slots add
+// u (5Q + 44 r_v), and slots placed in FP64 from the FP32 offsets add u r_v: the
+// rotation carries the offset's rounding on, before the placed offset is
+// rounded (fp32_offset_units).  The FP32 positions are within (1 + 2^-19) u
+// (cm_fixed.h), which the whole bound is widened by.  The distance is within
 // sqrt(3) E plus 2.5 u d (three roundings of d^2, one of the square root).  The
 // atom-cell layout's displacement (q_a - (q_b - off)) is bounded by the same
 // expression with r = 0.  delta adds 25 % to the bound.
@@ -1835,7 +1839,7 @@ __device__ __forceinline__ void k_frame_consts_body(const uint3 blockIdx, const 
         cn[lane] = norm3d(v[0], v[1], v[2]);
     }
     __syncthreads();
-    if (lane > 1) return;  // lane 0: the search's constants; lane 1: the band of k_random_fast, beside it
+    if (lane > 2) return;  // lane 0: the search's constants; lanes 1 and 2: the bands gr and gp, beside it
     double Q = 0.0, OFF = 0.0;
     for (int k = 0; k < 8; ++k) {
         Q = fmax(Q, cn[k]);
@@ -1854,11 +1858,11 @@ __device__ __forceinline__ void k_frame_consts_body(const uint3 blockIdx, const 
                      2.0 * ((double)F.rmax_s + rc + (double)F.rcmax) + 1.0;
     const double eps = 0x1.0p-53 * (512.0 + 4.0 * (double)(S.apv + (pairs ? S.aps : 0))) * M;
     const double u = 0x1.0p-24;
-    const double E0 = u * (5.0 * Q + 4.0 * OFF + 2.0 * rv + rs + S.cut + 1.0);
+    const double E0 = u * fp32_pair_units(Q, OFF, rs, rv, S.cut);
     // ATOMS frames: the random insertion's slots are placed in FP32 (placed_store32) when
     // that widens the band by at most 60 % (small molecules); larger molecules have few
     // slots per atom and more records per slot in a wider band, and keep the FP64 placement
-    const double P = u * (5.0 * Q + 44.0 * (double)F.rcmax);
+    const double P = u * fp32_slot_units(Q, (double)F.rcmax);
     const bool place32 = !pairs && S.fp32 && P <= 0.6 * E0;
     if (lane == 0) F.place32 = place32 ? 1 : 0;
     // the band of displacements within E of the exact ones
@@ -1879,10 +1883,12 @@ __device__ __forceinline__ void k_frame_consts_body(const uint3 blockIdx, const 
         g.list_band = g.two_delta + 1e-3f * (1.0f + (float)S.cut);
         return g;
     };
-    // lane 1: the slots that k_random_fast places in FP32 (r_c: the solvent molecules' radius)
-    const Guard g = band(E0 + (lane == 1 ? u * (5.0 * Q + 44.0 * rv) : place32 ? P : 0.0));
-    if (lane == 1) {
-        F.gr = g;
+    // lane 1: the slots that k_random_fast places in FP32 (r_c: the solvent molecules' radius); lane 2: those placed
+    // in FP64 from the FP32 offsets
+    const Guard g = band(E0 + (lane == 1 ? u * fp32_slot_units(Q, rv) : lane == 2 ? u * fp32_offset_units(rv) : place32 ? P : 0.0));
+    if (lane > 0) {
+        if (lane == 1) F.gr = g;
+        else F.gp = g;
         return;
     }
     // the tiled kernels test |w|^2 / 2 - w q for a staged position w (at most Q + OFF long) and a home position q
