@@ -165,6 +165,14 @@ CM_HD bool fixed_unwrap(const FixedGeom &X, int64_t *d) {
     return true;
 }
 
+// sum += d for |d| below 2^51; false once the sum leaves (-2^62, 2^62), which a
+// few thousand atoms far from their molecule's reference atom can make it do
+// (2^62 units are 4.2 10^6 A).
+CM_HD bool fixed_add(int64_t &sum, int64_t d) {
+    sum = (int64_t)((uint64_t)sum + (uint64_t)d);
+    return sum < (int64_t(1) << 62) && sum > -(int64_t(1) << 62);
+}
+
 // sum / n for n >= 1, within one unit.
 CM_HD int64_t fixed_mean(int64_t sum, int n) {
     if (n == 1) return sum;

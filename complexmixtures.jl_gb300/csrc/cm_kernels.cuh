@@ -1989,7 +1989,7 @@ __device__ __forceinline__ void k_prep_atoms_solvent_body(const uint3 blockIdx, 
             if (centroids) {
                 int64_t d[3] = {p[0] - xr[0], p[1] - xr[1], p[2] - xr[2]};
                 ok = fixed_unwrap(X, d) && ok;
-                for (int k = 0; k < 3; ++k) sum[k] += d[k];
+                for (int k = 0; k < 3; ++k) ok = fixed_add(sum[k], d[k]) && ok;
             }
         }
         if (ok && centroids) {
