@@ -298,12 +298,14 @@ __device__ __forceinline__ void k_agrid_build_body(const uint3 blockIdx, const d
                     if (t >= o) incl += u;
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, v > 0);
+                __syncwarp();  // every lane has read its cell: the stores go to cells of this group or before it
                 if (v > 0) {
-                    const int at = cells + __popc(m & below);  // at most i: read above
+                    const int at = cells + __popc(m & below);
                     s_pre[at] = run + incl - v;
                     s_beg[at] = beg;
                     s_oi[at] = oi;
                 }
+                __syncwarp();
                 cells += __popc(m);
                 run += __shfl_sync(0xffffffffu, incl, 31);
             }
