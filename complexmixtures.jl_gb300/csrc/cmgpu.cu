@@ -171,16 +171,21 @@ constexpr size_t kOutChunk = size_t(512) << 10;  // bytes of a pinned read-out b
 // Random samples placed per launch in the ATOMS layout.  FP64, or under an HBM
 // budget: 32 samples' worth of FP64 slots (52 bytes a site and 20 more); FP32
 // slots are smaller (20 a site and 36 more), so 41 to 76 samples fit the same
-// memory.  FP32 without a budget: up to kPieceSlots slots.  A piece's launches
-// end on their slowest warps and on the latency of its few exact records, so
-// fewer and larger pieces are faster.
+// memory.  FP32 without a budget: up to kPieceSlots slots of up to kPieceSites
+// sites in all, 335 MB of placement buffers and 151 MB of slot lists and queue
+// at the most.  A piece's launches end on their slowest warps and on the
+// latency of its few exact records, so fewer and larger pieces are faster: 4 M
+// slots of three sites are within both bounds, and so are the slots of
+// molecules of up to four sites.
 constexpr int64_t kPieceSlots = 1 << 22;
+constexpr int64_t kPieceSites = 1 << 24;
 constexpr int64_t kPieceSamples = 65535;  // a piece's samples are the y axis of k_slot_filter's grid
 int chunk_samples(const cm_system_desc &d) {
     if (d.precision != CM_PRECISION_FP32_GUARD) return 32;
-    const int64_t apv = d.solvent_natomspermol;
+    const int64_t apv = d.solvent_natomspermol, mv = d.solvent_nmols;
     const int64_t fit = 32 * (52 * apv + 20) / (20 * apv + 36);
-    return (int)(d.hbm_budget_bytes > 0 ? fit : std::max(fit, std::min(kPieceSlots / d.solvent_nmols, kPieceSamples)));
+    if (d.hbm_budget_bytes > 0) return (int)fit;
+    return (int)std::max(fit, std::min({kPieceSlots / mv, kPieceSites / (mv * apv), kPieceSamples}));
 }
 
 // Lanes per candidate-grid query (k_agrid_real, k_agrid_random).
@@ -933,8 +938,9 @@ void plan(cm_handle *h, const cm_frames *f) {
             // the work queue holds every slot of the samples placed in one launch
             const int64_t cs = chunk_samples(d);
             const int64_t want = std::min<int64_t>(cs * mv, std::max<int64_t>(1 << 22, mv));
-            h->atoms_piece = (int)std::max<int64_t>(1, std::min<int64_t>(cs, want / mv));
-            const int chunk = std::min(h->atoms_piece, std::max(1, fc * d.n_random_samples));
+            // (a chunk has fc n_random_samples of them at the most)
+            h->atoms_piece = (int)std::max<int64_t>(1, std::min<int64_t>({cs, want / mv, (int64_t)fc * d.n_random_samples}));
+            const int chunk = h->atoms_piece;
             dev_alloc(h, h->pcell, (size_t)chunk * h->Nv * 4);
             h->aslot_cap = (int)std::min<int64_t>((int64_t)chunk * mv, (int64_t)INT32_MAX);
             dev_alloc(h, h->aslot, (size_t)h->aslot_cap * 4);
