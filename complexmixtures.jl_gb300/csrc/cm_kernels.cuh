@@ -419,7 +419,7 @@ struct Bufs {
     float4 *avq32;
     d4 *avq64;
     d4 *u64;                        // [nf][Nv]
-    float4 *u32;                    // [nf][Nv] FP32 copies of u64 (the FP32 placement)
+    float4 *u32;                    // [nf][Nv] FP32 copies of u64 (the FP32 placement; nullptr in FP64)
     float *rc;                      // [nf][mv]
     int *pcell;                     // [placed samples][Nv]
     float4 *pq32;
@@ -2026,7 +2026,7 @@ __device__ __forceinline__ void k_prep_atoms_solvent_body(const uint3 blockIdx, 
         }
         if (centroids) {
             centroid_data(G, x, apm, iref, B.u64 + at, r);
-            for (int b = 0; b < apm; ++b) {
+            for (int b = 0; b < apm && B.u32; ++b) {
                 const d4 w = B.u64[at + b];
                 B.u32[at + b] = make_float4((float)w.x, (float)w.y, (float)w.z, 0.f);
             }

@@ -309,25 +309,61 @@ void quiesce(cm_handle *h) {
     if (h->copy_stream) CM_CUDA(cudaStreamSynchronize(h->copy_stream));
 }
 
-void dev_alloc(cm_handle *h, DevBuf &b, size_t bytes) {
-    if (b.bytes >= bytes && b.p) return;
+// Give a device buffer back (the handle's queued work is done with it).
+void dev_free(cm_handle *h, DevBuf &b) {
+    if (!b.p) return;
+    blocks().put(h->device, false, b.p, b.bytes);
+    h->device_bytes -= (int64_t)b.charged;
+    b.p = nullptr;
+    b.bytes = b.charged = 0;
+}
+
+// A device buffer of at least `bytes`; false when it does not fit the budget
+// or the device (the old block is then given back).
+bool dev_try_alloc(cm_handle *h, DevBuf &b, size_t bytes) {
+    if (b.bytes >= bytes && b.p) return true;
     if (b.p) {
         quiesce(h);  // queued kernels of this handle may still read the old block
-        blocks().put(h->device, false, b.p, b.bytes);
-        h->device_bytes -= (int64_t)b.charged;
-        b.p = nullptr;
-        b.bytes = b.charged = 0;
+        dev_free(h, b);
+    }
+    const size_t want = BlockCache::round_up(bytes);
+    if (h->d.hbm_budget_bytes > 0 && h->device_bytes + (int64_t)want > h->d.hbm_budget_bytes) return false;
+    size_t got = 0;
+    b.p = blocks().get(h->device, false, bytes, &got);
+    if (!b.p) return false;
+    b.bytes = got;
+    b.charged = want;  // independent of which cached block was reused
+    h->device_bytes += (int64_t)want;
+    return true;
+}
+
+// The candidate grid given up (later chunks walk the stencil): its lists are
+// the one thing on the device that a handle can do without.
+void agrid_drop(cm_handle *h) {
+    quiesce(h);
+    h->agk = 0;
+    for (DevBuf *b : {&h->gent, &h->gstart, &h->gedge, &h->gpool, &h->galist, &h->scount, &h->skey, &h->sslot, &h->adefer})
+        dev_free(h, *b);
+}
+
+// A buffer of the candidate grid; false (and the grid dropped) when it does not fit.
+bool agrid_alloc(cm_handle *h, DevBuf &b, size_t bytes) {
+    if (h->agk > 0 && dev_try_alloc(h, b, bytes)) return true;
+    if (h->agk > 0) agrid_drop(h);
+    return false;
+}
+
+void dev_alloc(cm_handle *h, DevBuf &b, size_t bytes) {
+    if (dev_try_alloc(h, b, bytes)) return;
+    if (h->agk > 0) {
+        agrid_drop(h);
+        if (dev_try_alloc(h, b, bytes)) return;
     }
     const size_t want = BlockCache::round_up(bytes);
     if (h->d.hbm_budget_bytes > 0 && h->device_bytes + (int64_t)want > h->d.hbm_budget_bytes)
         throw cm_error(CM_ENOMEM, "device memory budget exceeded (" + std::to_string(h->device_bytes + (int64_t)want) +
                                       " > " + std::to_string(h->d.hbm_budget_bytes) + " bytes)");
-    size_t got = 0;
-    b.p = blocks().get(h->device, false, bytes, &got);
-    if (!b.p) throw cm_error(CM_ENOMEM, "cudaMalloc(" + std::to_string(want) + "): out of device memory");
-    b.bytes = got;
-    b.charged = want;  // independent of which cached block was reused
-    h->device_bytes += (int64_t)want;
+    throw cm_error(CM_ENOMEM, "cudaMalloc(" + std::to_string(want) + "): out of device memory");
 }
 
 // Pinned host staging from the block cache.
@@ -810,11 +846,10 @@ void ensure_cells(cm_handle *h, int64_t ncell) {
         dev_alloc(h, h->anear, n);
         if (h->agk > 0) {
             const int64_t k3 = (int64_t)h->agk * h->agk * h->agk;
-            dev_alloc(h, h->gstart, (size_t)h->fc * ncell * k3 * (kAgridBuckets + 1) * 4);
-            dev_alloc(h, h->gedge, (size_t)h->fc * ncell * k3 * sizeof(float2));
-            dev_alloc(h, h->gpool, (size_t)h->fc * 4);
-            dev_alloc(h, h->galist, (size_t)h->fc * ncell * 4);
-            if (h->mddf) dev_alloc(h, h->scount, (size_t)h->fc * ncell * k3 * 4);
+            (void)(agrid_alloc(h, h->gstart, (size_t)h->fc * ncell * k3 * (kAgridBuckets + 1) * 4) &&
+                   agrid_alloc(h, h->gedge, (size_t)h->fc * ncell * k3 * sizeof(float2)) &&
+                   agrid_alloc(h, h->gpool, (size_t)h->fc * 4) && agrid_alloc(h, h->galist, (size_t)h->fc * ncell * 4) &&
+                   (!h->mddf || agrid_alloc(h, h->scount, (size_t)h->fc * ncell * k3 * 4)));
         }
     }
 }
@@ -905,19 +940,32 @@ void plan(cm_handle *h, const cm_frames *f) {
         dev_alloc(h, h->cq32, fc * mv * 16);
         // guard queue of a chunk: every candidate fits when the system is small
         // (candidates <= ms * mv per frame); otherwise 64 per solute molecule and
-        // frame, far above the guard-band rate
-        const int64_t bound = ms * mv * fc;
-        h->gq_cap = (int)(bound <= (1LL << 24) ? std::max<int64_t>(bound, 1024)
-                                               : std::min<int64_t>(std::max<int64_t>(1 << 20, 64 * ms * fc), 1LL << 25));
-        if (d.guard_queue_capacity > 0) h->gq_cap = d.guard_queue_capacity;
-        dev_alloc(h, h->gq, (size_t)h->gq_cap * sizeof(int4));
-        dev_alloc(h, h->eq, (size_t)h->gq_cap * 3 * sizeof(int4));
+        // frame, far above the guard-band rate.  (The FP64 search decides every
+        // record where it is found.)
+        if (!fp64) {
+            const int64_t bound = ms * mv * fc;
+            h->gq_cap = (int)(bound <= (1LL << 24) ? std::max<int64_t>(bound, 1024)
+                                                   : std::min<int64_t>(std::max<int64_t>(1 << 20, 64 * ms * fc), 1LL << 25));
+            if (d.guard_queue_capacity > 0) h->gq_cap = d.guard_queue_capacity;
+            dev_alloc(h, h->gq, (size_t)h->gq_cap * sizeof(int4));
+            dev_alloc(h, h->eq, (size_t)h->gq_cap * 3 * sizeof(int4));
+        }
         if (h->mddf) {
-            // random-insertion queue: every slot of `chunk` samples fits
-            const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>((int64_t)fc * d.n_random_samples, (1 << 23) / mv));
+            // random-insertion queue: every slot of `chunk` samples fits.  Under an
+            // HBM budget the two queues of the FP32 search take no more than its one
+            // queue and the FP64 molecules that it left out: fewer samples a launch
+            int64_t chunk = std::max<int64_t>(1, std::min<int64_t>((int64_t)fc * d.n_random_samples, (1 << 23) / mv));
+            if (!fp64 && d.hbm_budget_bytes > 0) {
+                auto size = [](int64_t bytes) { return (int64_t)BlockCache::round_up((size_t)bytes); };
+                auto queue = [&](int64_t samples) { return size(samples * mv * (int64_t)sizeof(int2)); };
+                const int64_t molecules = size(fc * ms * 32) + size(fc * h->Ns * 32) +
+                                          (d.autocorrelation ? 0 : size(fc * mv * 32) + size(fc * h->Nv * 32));
+                const int64_t room = queue(chunk) + molecules;
+                while (chunk > 1 && 2 * queue(chunk) > room) chunk -= std::max<int64_t>(1, chunk / 32);
+            }
             h->rq_cap = (int)(chunk * mv);
             dev_alloc(h, h->rq, (size_t)h->rq_cap * sizeof(int2));
-            if (d.precision == CM_PRECISION_FP32_GUARD) dev_alloc(h, h->rq2, (size_t)h->rq_cap * sizeof(int2));
+            if (!fp64) dev_alloc(h, h->rq2, (size_t)h->rq_cap * sizeof(int2));
         }
     } else {
         dev_alloc(h, h->akey, fc * h->Ns * 4);
@@ -933,7 +981,7 @@ void plan(cm_handle *h, const cm_frames *f) {
         }
         if (h->mddf) {
             dev_alloc(h, h->u64, fc * h->Nv * 32);
-            dev_alloc(h, h->u32, fc * h->Nv * 16);
+            if (d.precision == CM_PRECISION_FP32_GUARD) dev_alloc(h, h->u32, fc * h->Nv * 16);  // the FP32 placement's
             dev_alloc(h, h->rc, fc * mv * 4);
             // the work queue holds every slot of the samples placed in one launch
             const int64_t cs = chunk_samples(d);
@@ -996,12 +1044,10 @@ void plan(cm_handle *h, const cm_frames *f) {
             if (d.hbm_budget_bytes <= 0 || h->device_bytes + bytes <= d.hbm_budget_bytes / 4) {
                 h->agk = K;
                 h->gcap = gcap;
-                dev_alloc(h, h->gent, (size_t)bytes);
-                dev_alloc(h, h->adefer, (size_t)std::max<int64_t>(fc * mv, h->aslot_cap) * 4);
-                if (h->mddf) {
-                    dev_alloc(h, h->skey, (size_t)h->aslot_cap * 8);
-                    dev_alloc(h, h->sslot, (size_t)h->aslot_cap * 4);
-                }
+                (void)(agrid_alloc(h, h->gent, (size_t)bytes) &&
+                       agrid_alloc(h, h->adefer, (size_t)std::max<int64_t>(fc * mv, h->aslot_cap) * 4) &&
+                       (!h->mddf || (agrid_alloc(h, h->skey, (size_t)h->aslot_cap * 8) &&
+                                     agrid_alloc(h, h->sslot, (size_t)h->aslot_cap * 4))));
             }
         }
         if (h->agk > 0) {
@@ -1827,7 +1873,7 @@ void agrid_grow(cm_handle *h) {
     const int64_t bytes = (int64_t)h->fc * gcap * 16;
     const int64_t now = (int64_t)h->gent.charged;
     if (h->d.hbm_budget_bytes > 0 && h->device_bytes - now + bytes > h->d.hbm_budget_bytes / 4) return;
-    dev_alloc(h, h->gent, (size_t)bytes);
+    if (!agrid_alloc(h, h->gent, (size_t)bytes)) return;
     h->gcap = gcap;
     CM_CUDA(cudaMemsetAsync(P<unsigned long long>(h->stats) + ST_AGRID_OVF, 0, sizeof(ovf), h->stream));
 }
