@@ -2127,24 +2127,31 @@ void noalloc_fixed(cm_handle *h, Carve &c) {
         c.take(h->bulk, (size_t)nd * mv * 4);
         c.take(h->nbulk, (size_t)nd * 4);
     }
+    const bool fp64 = d.precision != CM_PRECISION_FP32_GUARD;
     c.take(h->scell, ms * 4);
     c.take(h->sq32, ms * 16);
-    c.take(h->sq64, ms * 32);
     c.take(h->so32, h->Ns * 16);
-    c.take(h->so64, h->Ns * 32);
+    if (fp64) {
+        c.take(h->sq64, ms * 32);
+        c.take(h->so64, h->Ns * 32);
+    }
     if (!d.autocorrelation) {
         c.take(h->vcell, mv * 4);
         c.take(h->vq32, mv * 16);
-        c.take(h->vq64, mv * 32);
         c.take(h->vo32, h->Nv * 16);
-        c.take(h->vo64, h->Nv * 32);
+        if (fp64) {
+            c.take(h->vq64, mv * 32);
+            c.take(h->vo64, h->Nv * 32);
+        }
     }
     c.take(h->cmol, mv * 4);
     c.take(h->cq32, mv * 16);
-    h->gq_cap = (int)std::min<int64_t>(std::max<int64_t>(ms * mv, 1024), 1 << 17);
-    if (d.guard_queue_capacity > 0) h->gq_cap = std::min(h->gq_cap, d.guard_queue_capacity);
-    c.take(h->gq, (size_t)h->gq_cap * sizeof(int4));
-    c.take(h->eq, (size_t)h->gq_cap * 3 * sizeof(int4));
+    if (!fp64) {
+        h->gq_cap = (int)std::min<int64_t>(std::max<int64_t>(ms * mv, 1024), 1 << 17);
+        if (d.guard_queue_capacity > 0) h->gq_cap = std::min(h->gq_cap, d.guard_queue_capacity);
+        c.take(h->gq, (size_t)h->gq_cap * sizeof(int4));
+        c.take(h->eq, (size_t)h->gq_cap * 3 * sizeof(int4));
+    }
     if (h->mddf) {
         h->rq_cap = (int)std::min<int64_t>(std::max<int64_t>((int64_t)d.n_random_samples * mv, mv), std::max<int64_t>(mv, 1 << 18));
         c.take(h->rq, (size_t)h->rq_cap * sizeof(int2));
@@ -2207,8 +2214,13 @@ void noalloc_run(cm_handle *h, const cm_frames *f, cudaStream_t stream) {
         Chunk one;
         one.nf = 1;
         const Bufs B = chunk_bufs(h, one, dG, nullptr);
-        k_prep_pairs<T><<<grid_for(d.solute_nmols, 128), 128, 0, stream>>>(B, xs, h->Ns * 3, 0, 0, d.autocorrelation ? d.irefatom - 1 : 0);
-        if (!d.autocorrelation) k_prep_pairs<T><<<grid_for(d.solvent_nmols, 128), 128, 0, stream>>>(B, xv, h->Nv * 3, 1, 0, d.irefatom - 1);
+        auto prep = [&](const T *x, int64_t n, int64_t atoms, int side, int ref) {
+            if (d.precision == CM_PRECISION_FP32_GUARD) k_prep_pairs32<T><<<grid_for(n, 128), 128, 0, stream>>>(B, x, atoms * 3, side, 0, ref);
+            else k_prep_pairs<T><<<grid_for(n, 128), 128, 0, stream>>>(B, x, atoms * 3, side, 0, ref);
+        };
+        k_offtable<<<dim3(grid_for(cmgeom::kOffEntries, 256), 1), 256, 0, stream>>>(B);
+        prep(xs, d.solute_nmols, h->Ns, 0, d.autocorrelation ? d.irefatom - 1 : 0);
+        if (!d.autocorrelation) prep(xv, d.solvent_nmols, h->Nv, 1, d.irefatom - 1);
         CM_CUDA(cudaGetLastError());
     }
     FrameScratch F;
