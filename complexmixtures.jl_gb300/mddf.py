@@ -189,7 +189,7 @@ def _run_frames(eng: Engine, trajectory: Trajectory, to_compute, fw, batch_frame
             if os.path.isfile(STOP_FILE):
                 break
             ids = to_compute[b0 : b0 + batch_frames]
-            xs, xv, cells = trajectory.frame_arrays([i - 1 for i in ids])
+            xs, xv, cells = trajectory._frames_to_submit([i - 1 for i in ids])
             eng.submit(xs, None if eng.autocorrelation else xv, cells, weights=[fw[i - 1] for i in ids], frame_ids=ids)
         return
     if isinstance(trajectory, NamdDCD):

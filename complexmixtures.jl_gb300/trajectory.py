@@ -98,12 +98,20 @@ class ArrayTrajectory(Trajectory):
 
     # bulk access used by the driver to hand many frames to the GPU at once
     def frame_arrays(self, idx: Sequence[int]):
-        """Coordinates and cells of the given frames (0-based); views of the
+        """Coordinates and cells of the given frames (0-based), copies."""
+        idx = np.asarray(idx, dtype=np.int64)
+        return self._xs[idx], self._xv[idx], self._cells[idx]
+
+    def _frames_to_submit(self, idx: Sequence[int]):
+        """``frame_arrays`` for the driver, which only reads them: views of the
         stored arrays when the frames are consecutive."""
+        if type(self).frame_arrays is not ArrayTrajectory.frame_arrays:
+            return self.frame_arrays(idx)
         idx = np.asarray(idx, dtype=np.int64)
         if idx.ndim == 1 and idx.size and idx[0] >= 0 and idx[-1] < self.nframes and np.all(np.diff(idx) == 1):
-            idx = slice(int(idx[0]), int(idx[-1]) + 1)
-        return self._xs[idx], self._xv[idx], self._cells[idx]
+            run = slice(int(idx[0]), int(idx[-1]) + 1)
+            return self._xs[run], self._xv[run], self._cells[run]
+        return self.frame_arrays(idx)
 
 
 def unitcell_from_lengths_angles(a: float, b: float, c: float, alpha: float, beta: float, gamma: float) -> np.ndarray:
