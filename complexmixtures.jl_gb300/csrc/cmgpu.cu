@@ -2453,13 +2453,62 @@ void record_chunk(cm_handle *h, const Staged &S, const Chunk &c, std::vector<Ste
     else atoms_chain<double>(h, c, D, B, S.dT, (const double *)xs, (const double *)xv, ss, vs, em);
 }
 
-// A fused staging round: every system's chunk j goes through the same chain
-// of stages, and each stage runs once for all of them (k_multi, k_multi_zero)
-// in one captured graph on the batch stream; where the systems' kernels of a
+// The stage of a chain's step: kernels that differ only in the system's data
+// type, lanes or schedule are one stage (a launch per kernel).
+int stage_of(const Step &s) {
+    if (!s.kernel) return -1;
+    switch (s.kid) {
+    case MK_PREP_SOLVENT_F64: return MK_PREP_SOLVENT_F32;
+    case MK_PREP_SOLUTE_F64: return MK_PREP_SOLUTE_F32;
+    case MK_ATOMS_U64_F64: return MK_ATOMS_U64_F32;
+    case MK_AGRID_REAL4: return MK_AGRID_REAL;
+    case MK_AGRID_RANDOM4: return MK_AGRID_RANDOM;
+    case MK_EVAL_REAL_BALANCED: return MK_EVAL_REAL_CELL;
+    case MK_EVAL_RANDOM_BALANCED: return MK_EVAL_RANDOM_CELL;
+    default: return s.kid;
+    }
+}
+
+// A sequence of stages that holds both chains' in their order: a shortest one
+// (the chains' longest common subsequence merged once) when their middles,
+// between the common ends, are of ordinary length, else one middle after the other.
+std::vector<int> merge_stages(const std::vector<int> &a, const std::vector<int> &b) {
+    size_t lo = 0, ea = a.size(), eb = b.size();
+    while (lo < ea && lo < eb && a[lo] == b[lo]) ++lo;
+    while (ea > lo && eb > lo && a[ea - 1] == b[eb - 1]) --ea, --eb;
+    std::vector<int> z(a.begin(), a.begin() + lo);
+    const size_t na = ea - lo, nb = eb - lo;
+    size_t i = 0, j = 0;
+    if (na > 0 && nb > 0 && na * nb <= (size_t(1) << 20)) {
+        // len[i][j]: the longest common subsequence of the middles from i and j on
+        std::vector<int> len((na + 1) * (nb + 1), 0);
+        auto at = [&](size_t x, size_t y) -> int & { return len[x * (nb + 1) + y]; };
+        for (size_t x = na; x-- > 0;)
+            for (size_t y = nb; y-- > 0;)
+                at(x, y) = a[lo + x] == b[lo + y] ? at(x + 1, y + 1) + 1 : std::max(at(x + 1, y), at(x, y + 1));
+        while (i < na && j < nb) {
+            if (a[lo + i] == b[lo + j]) z.push_back(a[lo + i]), ++i, ++j;
+            else if (at(i + 1, j) >= at(i, j + 1)) z.push_back(a[lo + i++]);
+            else z.push_back(b[lo + j++]);
+        }
+    }
+    z.insert(z.end(), a.begin() + lo + i, a.begin() + ea);
+    z.insert(z.end(), b.begin() + lo + j, b.begin() + eb);
+    z.insert(z.end(), a.begin() + ea, a.end());
+    return z;
+}
+
+// A fused staging round: the systems' chunks j go through one sequence of
+// stages, and each stage runs once for all of them (k_multi, k_multi_zero) in
+// one captured graph on the batch stream; where the systems' kernels of a
 // stage differ (the ATOMS evaluation schedule follows each solute's density)
-// the stage takes one launch per kernel.  False (nothing launched) when the
-// systems cannot share the launches: another layout or precision, a weight
-// class change inside the round, or chains of different stages.
+// the stage takes one launch per kernel.  Systems with the candidate grid and
+// without it, and with different numbers of random-insertion pieces, have
+// different chains: the sequence holds the stages of all of them, and a
+// system has no part in those that are not its own.  24 small systems, half of
+// them on the stencil walk: 2,586 us a round, on their own streams 3,231.
+// False (nothing launched) when the systems cannot share the launches:
+// another layout or precision, or a weight class change inside the round.
 bool batch_round_fused(cm_batch *bt, std::vector<Staged> &st, const std::vector<char> &active) {
     const size_t n = bt->hs.size();
     size_t nchunks = 0;
@@ -2477,20 +2526,30 @@ bool batch_round_fused(cm_batch *bt, std::vector<Staged> &st, const std::vector<
     // stage need not be split by shared-memory class
     for (size_t i = 0; i < n; ++i)
         if (active[i]) bt->hs[i]->smem_groups = 0;
-    // rec[j][i]: the stages of system i's chunk j
+    // rec[j][i]: the steps of system i's chunk j; pos[j][i]: their stages' positions in seq[j]
     std::vector<std::vector<std::vector<Step>>> rec(nchunks, std::vector<std::vector<Step>>(n));
+    std::vector<std::vector<std::vector<int>>> pos(nchunks, std::vector<std::vector<int>>(n));
+    std::vector<std::vector<int>> seq(nchunks);
     for (size_t j = 0; j < nchunks; ++j) {
-        const std::vector<Step> *shape = nullptr;
+        std::vector<std::vector<int>> chains;  // the different ones
+        std::vector<size_t> chain(n, 0);
         for (size_t i = 0; i < n; ++i) {
             if (!active[i] || j >= st[i].chunks.size()) continue;
             record_chunk(bt->hs[i], st[i], st[i].chunks[j], rec[j][i]);
-            const std::vector<Step> &r = rec[j][i];
-            if (!shape) shape = &r;
-            else {
-                // a system of fewer random-insertion pieces has the shorter chain; its steps are the first ones
-                for (size_t k = 0; k < std::min(r.size(), shape->size()); ++k)
-                    if (r[k].kernel != (*shape)[k].kernel) return false;
-                if (r.size() > shape->size()) shape = &r;
+            std::vector<int> c;
+            for (const Step &s : rec[j][i]) c.push_back(stage_of(s));
+            chain[i] = std::find(chains.begin(), chains.end(), c) - chains.begin();
+            if (chain[i] == chains.size()) {
+                seq[j] = chains.empty() ? c : merge_stages(seq[j], c);
+                chains.push_back(std::move(c));
+            }
+        }
+        for (size_t i = 0; i < n; ++i) {
+            if (rec[j][i].empty()) continue;
+            int at = 0;
+            for (int stage : chains[chain[i]]) {
+                while (seq[j][at] != stage) ++at;
+                pos[j][i].push_back(at++);
             }
         }
     }
@@ -2519,35 +2578,36 @@ bool batch_round_fused(cm_batch *bt, std::vector<Staged> &st, const std::vector<
         memcpy(host.data() + off, p, bytes);
         return off;
     };
+    std::vector<size_t> next(n);
+    std::vector<const Step *> step(n);  // each system's step of the stage, nullptr if it has none
     for (size_t j = 0; j < nchunks; ++j) {
-        size_t nsteps = 0;
-        for (size_t i = 0; i < n; ++i) nsteps = std::max(nsteps, rec[j][i].size());
-        for (size_t k = 0; k < nsteps; ++k) {
+        std::fill(next.begin(), next.end(), 0);
+        for (size_t k = 0; k < seq[j].size(); ++k) {
+            for (size_t i = 0; i < n; ++i) {
+                const bool own = next[i] < pos[j][i].size() && pos[j][i][next[i]] == (int)k;
+                step[i] = own ? &rec[j][i][next[i]++] : nullptr;
+            }
             // the kernels of this stage across the systems, in order of first
             // appearance, each with the systems' shared memory in 32 KB classes:
             // a launch asks for its largest class, and a system with a small
             // histogram does not lower the occupancy of those with none
             auto smem_class = [](size_t b) { return (int)((b + 32767) / 32768); };
-            std::vector<std::pair<int, int>> kids;
-            bool zero = false;
-            for (size_t i = 0; i < n; ++i) {
-                if (rec[j][i].size() <= k) continue;
-                const Step &s = rec[j][i][k];
-                if (!s.kernel) zero = true;
-                else {
-                    const std::pair<int, int> key(s.kid, smem_class(s.smem));
-                    if (std::find(kids.begin(), kids.end(), key) == kids.end()) kids.push_back(key);
-                }
-            }
-            if (zero) {
+            if (seq[j][k] < 0) {
                 std::vector<MZero> zs;
                 for (size_t i : order)
-                    if (rec[j][i].size() > k) zs.push_back({rec[j][i][k].zp, (long long)rec[j][i][k].zbytes});
+                    if (step[i]) zs.push_back({step[i]->zp, (long long)step[i]->zbytes});
+                if (zs.empty()) continue;  // every chain found the stage earlier in the sequence
                 Launch L{};
                 L.n = (int)zs.size();
                 L.off = put(zs.data(), zs.size() * sizeof(MZero));
                 plan.push_back(L);
                 continue;
+            }
+            std::vector<std::pair<int, int>> kids;
+            for (size_t i = 0; i < n; ++i) {
+                if (!step[i]) continue;
+                const std::pair<int, int> key(step[i]->kid, smem_class(step[i]->smem));
+                if (std::find(kids.begin(), kids.end(), key) == kids.end()) kids.push_back(key);
             }
             for (const auto &key : kids) {
                 Launch L{};
@@ -2556,10 +2616,8 @@ bool batch_round_fused(cm_batch *bt, std::vector<Staged> &st, const std::vector<
                 std::vector<MTask> ts;
                 long long blocks = 0;
                 for (size_t i : order) {
-                    if (rec[j][i].size() <= k || rec[j][i][k].kid != key.first ||
-                        smem_class(rec[j][i][k].smem) != key.second)
-                        continue;
-                    const Step &s = rec[j][i][k];
+                    if (!step[i] || step[i]->kid != key.first || smem_class(step[i]->smem) != key.second) continue;
+                    const Step &s = *step[i];
                     MTask t;
                     t.a = s.a;
                     t.grid = make_uint3(s.grid.x, s.grid.y, s.grid.z);
