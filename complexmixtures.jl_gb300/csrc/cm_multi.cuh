@@ -160,6 +160,11 @@ __global__ void __launch_bounds__(mk_threads(KID), mk_min_ctas(KID))
 }
 
 // Zero-fill of (pointer, bytes) ranges: CTA r takes range r, r + gridDim.x, ...
+// The table holds ranges of at most kZeroPiece bytes, so that the slot counts
+// of a large system's fine cells (megabytes) are not one CTA's: two systems of
+// 200,000 atoms among six small ones 8,356 us a round whole, 8,266 in pieces.
+constexpr size_t kZeroPiece = size_t(64) << 10;
+
 struct MZero {
     void *p;
     long long bytes;

@@ -2595,7 +2595,9 @@ bool batch_round_fused(cm_batch *bt, std::vector<Staged> &st, const std::vector<
             if (seq[j][k] < 0) {
                 std::vector<MZero> zs;
                 for (size_t i : order)
-                    if (step[i]) zs.push_back({step[i]->zp, (long long)step[i]->zbytes});
+                    if (step[i])
+                        for (size_t at = 0; at < step[i]->zbytes; at += kZeroPiece)
+                            zs.push_back({(char *)step[i]->zp + at, (long long)std::min(kZeroPiece, step[i]->zbytes - at)});
                 if (zs.empty()) continue;  // every chain found the stage earlier in the sequence
                 Launch L{};
                 L.n = (int)zs.size();

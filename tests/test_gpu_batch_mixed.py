@@ -58,3 +58,29 @@ def test_mixed_chains(cm, gpu_ready, names):
         assert ref["md"].sum() > 0
         for k in KEYS:
             assert np.array_equal(got[k], ref[k]), (name, k)
+
+
+@pytest.mark.parametrize("edge", [47.0, 95.0])
+def test_zero_ranges_of_many_pieces(cm, gpu_ready, edge):
+    """Boxes of 343 and 3,375 search cells (8 fine cells each, two frames): slot
+    counts of 22 KB, less than one zero-fill range, and of 216 KB, four, the
+    last one partial, beside another system's and over three rounds."""
+    rng = np.random.default_rng(68)
+    H = np.diag([edge] * 3)
+    kw = dict(solute_nmols=1, solute_natomspermol=120, solvent_nmols=400, solvent_natomspermol=3, autocorrelation=False,
+              n_random_samples=6, **OPT)
+    frames = [chain_system(rng, H, n=120, nframes=2, mv=400, apv=3), chain_system(rng, ORTHO, n=120, nframes=2, mv=400, apv=3)]
+    engines = [cm.Engine(**kw) for _ in frames]
+    with cm.Batch(engines) as b:
+        for _ in range(3):
+            b.submit(frames)
+        assert b.graph_stats()["fused_rounds"] == 3
+    for e, (xs, xv, cells) in zip(engines, frames):
+        with cm.Engine(**kw) as alone:
+            for _ in range(3):
+                alone.submit(xs, xv, cells)
+            want = alone.raw_counts()
+        got = e.raw_counts()
+        e.close()
+        assert want["md_random"].sum() > 0
+        assert all(np.array_equal(got[k], want[k]) for k in KEYS)
