@@ -55,7 +55,6 @@ constexpr int kAgridBuildCtas = 4;     // resident CTAs per SM (40 KB of stage a
 constexpr int kAgridRecThreads = 32;   // k_agrid_records: a few records per SM,
 constexpr int kAgridRecLanes = 4;      // each on a group of lanes
 
-// The fine cells of a search cell: edge vectors and bounds, FP32.
 // Largest distance from p to a point of the fine cell centred at c: squared
 // for orthogonal cells, the distance to the centre squared otherwise (the
 // bound is then that distance + R).
@@ -852,8 +851,8 @@ __global__ void __launch_bounds__(256, 4) k_agrid_real(DevSys S, Bufs B) {
 
 // Random insertion of a single solute molecule, last pass: GL lanes per
 // slot that k_atoms_place placed, in the order of the slots' fine cells;
-// persistent grid.  The slot's sites are queried and the record is decided
-// (agrid_record inside the band).  k_atoms_place has
+// persistent grid.  The slot's sites are queried and the record is decided, or
+// listed for k_agrid_records when it lies inside the band.  k_atoms_place has
 // queued the near slots of the frames without a grid for k_atoms_eval.
 //
 // The loads of the lists bound it: a 16-byte load of 32 lanes from 32 lists

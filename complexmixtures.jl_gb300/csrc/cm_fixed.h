@@ -5,8 +5,8 @@
 // instruction occupies a quarter of an SM for 64 cycles on this GPU: the prep
 // kernels ran with the FP64 pipe 84 % busy and nothing else above 10 %.  Here
 // a coordinate is an integer in units of 2^-40 Angstrom (exact for FP32 inputs
-// above 2^-17 A and FP64 inputs above 2^11 A, truncated by less than 2^-40 A
-// otherwise), H^-1 an integer in units of 2^-64, and the fractional coordinate
+// above 2^-17 A and FP64 inputs above 2^12 A, truncated by less than 2^-40 A
+// otherwise; below 2^22 A), H^-1 an integer in units of 2^-64, and the fractional coordinate
 // their product modulo 1 in units of 2^-64: its upper bits times the cell count
 // are the cell, the rest the position in it.  A position is within
 //   3 (2^-40 A + |x| 2^-64 |H|) + |H| 2^-62
@@ -23,8 +23,7 @@
 
 namespace cmgeom {
 
-constexpr int kFixBits = 40;            // position unit 2^-40 Angstrom
-constexpr float kFixLimit = 4194304.f;  // |x| below 2^22 Angstrom
+constexpr int kFixBits = 40;  // position unit 2^-40 Angstrom
 
 struct FixedGeom {
     int64_t A[9];         // row-major H^-1 in units of 2^-64

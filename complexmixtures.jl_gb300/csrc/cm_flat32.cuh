@@ -361,7 +361,8 @@ __device__ __forceinline__ void image_at(const Images &im, int img, int &dx, int
 // slot, so the slots end with the values over all images.  (The generic
 // kernel evaluates every atom pair of every image, one lane per molecule: 300
 // 9-atom molecules in a 30 A box, cutoff 9 A, 16 frames: 5,473 us a pass with the
-// generic kernel, 1,048 with this one.)
+// generic kernel, 1,048 with this one, which spills 76 to 160 bytes at the 80
+// registers of two CTAs per SM.)
 template <bool SELF, int APS>
 __device__ __forceinline__ void flat_images(const DevSys &S, const Bufs &B, const SHist &h, FlatWarpSmem &W,
                                             const PairsFrame &Pf, const Guard &g, int f, int s, int sslot, const float4 qs,
@@ -749,6 +750,28 @@ __device__ __forceinline__ int tile_molecule(const TileCellTab &T, int K, int m,
     return T.cbeg[lo] + (m - T.nbeg[lo]);
 }
 
+// Stage n molecules of the half stencil from position m0 on, up to the next
+// multiple of 32 with entries that are no candidates; the CTA's threads share them.
+template <typename TILE>
+__device__ __forceinline__ void tile_stage(TILE &T, const PairsFrame &Pf, const FrameScratch &F, const float4 *cq32, int K, int m0,
+                                           int n) {
+    for (int i = threadIdx.x; i < ((n + 31) & ~31); i += blockDim.x) {
+        if (i >= n) {
+            T.w[i] = make_float4(0.f, 0.f, 0.f, INFINITY);
+            continue;
+        }
+        int k, dx, dy, dz;
+        const int p = tile_molecule(T.c, K, m0 + i, k);
+        half_stencil_cell(k, F.L, dx, dy, dz);
+        const float4 of = Pf.off32[off_index(dx, dy, dz)];
+        const float4 q = cq32[p];
+        const float x = q.x + of.x, y = q.y + of.y, z = q.z + of.z;
+        T.w[i] = make_float4(x, y, z, 0.5f * fmaf(z, z, fmaf(y, y, x * x)));
+        const int v = Pf.cmol[p];
+        T.v[i] = v | (k << 24) | (Pf.slot && Pf.slot[v] >= 0 ? 0x80000000 : 0);
+    }
+}
+
 template <int APS>
 __global__ void __launch_bounds__(kTileWarps * 32, CM_TILE_MIN_CTAS) k_pairs_tile32(DevSys S, Bufs B) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -792,21 +815,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, CM_TILE_MIN_CTAS) k_pairs_til
         for (int m0 = 0; m0 < M; m0 += kTileStage) {
             const int n = min(kTileStage, M - m0), nr = (n + 31) & ~31;
             if (m0 > 0) __syncthreads();  // the previous pass's table is no longer read
-            for (int i = tid; i < nr; i += blockDim.x) {
-                if (i >= n) {
-                    T.w[i] = make_float4(0.f, 0.f, 0.f, INFINITY);  // never a candidate
-                    continue;
-                }
-                int k, dx, dy, dz;
-                const int p = tile_molecule(T.c, K, m0 + i, k);
-                half_stencil_cell(k, F.L, dx, dy, dz);
-                const float4 of = Pf.off32[off_index(dx, dy, dz)];
-                const float4 q = cq32[p];
-                const float x = q.x + of.x, y = q.y + of.y, z = q.z + of.z;
-                T.w[i] = make_float4(x, y, z, 0.5f * fmaf(z, z, fmaf(y, y, x * x)));
-                const int v = Pf.cmol[p];
-                T.v[i] = v | (k << 24) | (Pf.slot && Pf.slot[v] >= 0 ? 0x80000000 : 0);
-            }
+            tile_stage(T, Pf, F, cq32, K, m0, n);
             if (tid == 0) T.next = 0;
             __syncthreads();
             // the home molecules, claimed one at a time
@@ -899,7 +908,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, CM_TILE_MIN_CTAS) k_pairs_til
 // are formed as in flat_flush, so the records and the queues are the same.
 // 19,338 waters, cutoff 10 A, 16 frames: 1,979 us in k_pairs_tile32, 746 here
 // (12 or 20 warps per CTA: 801, 825); the candidates' decisions and the gathers
-// of their atoms bound it (73 % issue, 69 % of the L1 port).
+// of their atoms bound it (73 % issue, 69 % of the L1 port).  At 64 registers
+// molecules of 3, 4 and 5 atoms spill 32, 96 and 180 bytes.
 #ifndef CM_DIRECT_WARPS
 #define CM_DIRECT_WARPS 16
 #endif
@@ -1001,21 +1011,7 @@ __global__ void __launch_bounds__(kDirectWarps * 32, 2) k_pairs_direct32(DevSys 
                 const int nh = min(kDirectHome, nH - h0), n = min(kDirectStage, M - m0);
                 const int nr = (n + 31) & ~31;
                 __syncthreads();  // the previous pass's tables are no longer read
-                for (int i = tid; i < nr; i += blockDim.x) {
-                    if (i >= n) {
-                        T.w[i] = make_float4(0.f, 0.f, 0.f, INFINITY);  // never a candidate
-                        continue;
-                    }
-                    int k, dx, dy, dz;
-                    const int p = tile_molecule(T.c, K, m0 + i, k);
-                    half_stencil_cell(k, F.L, dx, dy, dz);
-                    const float4 of = Pf.off32[off_index(dx, dy, dz)];
-                    const float4 q = cq32[p];
-                    const float x = q.x + of.x, y = q.y + of.y, z = q.z + of.z;
-                    T.w[i] = make_float4(x, y, z, 0.5f * fmaf(z, z, fmaf(y, y, x * x)));
-                    const int v = Pf.cmol[p];
-                    T.v[i] = v | (k << 24) | (Pf.slot && Pf.slot[v] >= 0 ? 0x80000000 : 0);
-                }
+                tile_stage(T, Pf, F, cq32, K, m0, n);
                 for (int i = tid; i < nh; i += blockDim.x) {
                     const float4 q = cq32[hbeg + h0 + i];
                     const float R = (g.cut_pre + q.w) + rmax;
@@ -1093,7 +1089,8 @@ __global__ void __launch_bounds__(kDirectWarps * 32, 2) k_pairs_direct32(DevSys 
 // pairs_decide.
 
 // Atom pair i of a molecule pair: image i / (aps apv), then solvent atom b and
-// solute atom a; the quotients from FP32 reciprocals are exact for i < 2^16.
+// solute atom a; the quotients from FP32 reciprocals are exact for every pair
+// of up to 32 atoms a side and up to 16^3 images.
 struct PairIndex {
     float inv_pi, inv_aps;
     int per_img, aps;

@@ -2248,7 +2248,7 @@ __device__ __forceinline__ bool placed_store32(const Bufs &B, const FrameScratch
 // work): a slot whose molecule cannot reach a cell near its solute molecule
 // (placed_maybe_near on a box widened to cover the FP32 rounding of the
 // centre's cell) can hold no pair within the cutoff and is dropped; the others
-// go to the slot list (y * mv + slot, count in counters[5]), so that the FP64
+// go to the slot list (y * mv + slot, count in counters[5]), so that the
 // placement runs on full warps.  With the candidate grid a listed slot also
 // counts itself at the fine cell of its centre (frames from frame0 on), for
 // the queries' order (k_slot_scan).
@@ -2359,7 +2359,8 @@ __global__ void __launch_bounds__(1024) k_slot_scan(Bufs B, int frame0) {
     k_slot_scan_body(blockIdx, gridDim, B, frame0);
 }
 
-// Second pass: the listed slots placed (FP64, the same draws, on full warps),
+// Second pass: the listed slots placed on full warps (the same draws; in FP32
+// where FrameScratch::place32, else in FP64),
 // written to the placement buffers, and -- in frames without a candidate grid
 // -- queued for k_atoms_eval when one of their atoms lies in a near cell of
 // the solute molecule: (slot, placed sample, sample, 1).  The grid's frames

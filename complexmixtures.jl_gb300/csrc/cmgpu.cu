@@ -1401,8 +1401,8 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
         em.zero(B.gpool, (size_t)nf * sizeof(int));
         em.kernel(MK_AGRID_BUILD, dim3((unsigned)std::min<int64_t>((int64_t)c.ncell_max * nf, (int64_t)sms * kAgridBuildCtas)),
                   (size_t)kAgridStage * sizeof(float4), CM_K_CELLS, base);
-        // real pass: every solvent molecule queried (records inside the band
-        // decided in place); frames without a grid go to the evaluation queue.
+        // real pass: every solvent molecule queried, the records inside the band
+        // decided by k_agrid_records; frames without a grid go to the evaluation queue.
         // counters[6 .. 7]: the queries' next molecule (zeroed with the chunk's counters)
         em.zero(B.counters + 2, sizeof(int));
         em.kernel(agrid_lanes(d) == 4 ? MK_AGRID_REAL4 : MK_AGRID_REAL, dim3(agrid_grid((int64_t)nf * mv, h->agrid_real_ctas)), hsm, CM_K_REAL, base);
@@ -1439,7 +1439,7 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
                       0, CM_K_RANDOM, args(nullptr, 0, 0, c.smp0 + s0, f0));
             if (agrid) {
                 em.kernel(agrid_lanes(d) == 4 ? MK_AGRID_RANDOM4 : MK_AGRID_RANDOM, dim3(agrid_grid((int64_t)ny * mv, h->agrid_rand_ctas)), hsm, CM_K_RANDOM,
-                          args(nullptr, 0, 0, c.smp0 + s0, ny));
+                          args(nullptr, 0, 0, c.smp0 + s0, 0));
                 em.kernel(MK_AGRID_REC_RANDOM, dim3(rec_grid((int64_t)ny * mv)), hsm, CM_K_RANDOM,
                           args(nullptr, 0, 0, c.smp0 + s0, 0));
             }

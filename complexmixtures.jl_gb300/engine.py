@@ -76,8 +76,9 @@ def system_desc(
     real-pass schedule of the molecule layout (speed only); ``atoms_grid``
     (ATOMS layout, one solute molecule, FP32) sets the fine cells per
     search-cell axis of the per-frame candidate grid (1-6; 0 = fine cells of
-    about 4.5 A when at least 8 solvent sites are asked per solute atom and
-    frame, the walk otherwise; -1 = no grid, every query walks the stencil;
+    about 4.5 A when a frame asks for at least 4 solvent molecules or slots per
+    solute atom (molecules of up to 4 sites) or 8 sites per solute atom (up to
+    32 sites), the walk otherwise; -1 = no grid, every query walks the stencil;
     speed only) and
     ``atoms_grid_capacity`` its list entries per frame (0 = sized by the
     engine; a frame whose lists do not fit walks the stencil)."""

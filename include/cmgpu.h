@@ -136,9 +136,13 @@ typedef struct cm_system_desc {
                                          not depend on it */
     int32_t atoms_grid;               /* ATOMS layout with one solute molecule, FP32 search: fine cells per
                                          search-cell axis of the per-frame candidate grid (1-6; 0 = a grid of
-                                         fine cells of about 4.5 A when at least 8 solvent sites are asked per
-                                         solute atom and frame, the stencil walk otherwise; -1 = no grid, every
-                                         query walks the stencil).  The counts do not depend on it */
+                                         fine cells of about 4.5 A when a frame asks for enough queries, the
+                                         stencil walk otherwise; -1 = no grid, every query walks the stencil).
+                                         Queries: a frame's solvent molecules, each once and n_random_samples
+                                         times in MDDF mode; enough: 4 per solute atom for molecules of up to 4
+                                         sites, or 8 sites per solute atom for up to 32; larger molecules walk.
+                                         The grid is given up when the HBM budget or the device has no room for
+                                         it.  The counts do not depend on it */
     int32_t atoms_grid_capacity;      /* list entries per frame of that grid; 0 = sized by the engine.  A frame
                                          whose lists do not fit walks the stencil instead, so the counts do
                                          not depend on it (a small value only exercises that path) */
