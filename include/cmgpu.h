@@ -122,7 +122,9 @@ typedef struct cm_system_desc {
     const int32_t *solvent_groups;
     int32_t device;                   /* CUDA device ordinal */
     int32_t max_frames_per_batch;     /* frames staged on the device per submit chunk; 0 = 64 */
-    int64_t hbm_budget_bytes;         /* 0 = no limit; cm_create fails with CM_ENOMEM above it */
+    int64_t hbm_budget_bytes;         /* device memory of the handle; 0 = no limit.  Calls that need more fail
+                                         with CM_ENOMEM, after the engine has taken smaller random-insertion
+                                         pieces and given up the candidate grid */
     int32_t kernel_timing;            /* 1: time every launch with CUDA events (cm_get_kernel_times) */
     int32_t cell_scale_pct;           /* search-cell size in percent of the default (0 = 100, range 30-300);
                                          the counts do not depend on it, only the speed (cm_autotune) */
