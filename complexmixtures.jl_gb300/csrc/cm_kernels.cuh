@@ -2312,17 +2312,23 @@ __global__ void k_slot_filter(DevSys S, Bufs B, int sample0, int frame0) {
 }
 
 // First position of each fine cell's slots in the sorted slot list: an
-// exclusive scan of a frame's counts by one CTA of 1024 threads (frame frame0
-// + block), from a base that the frame takes off counters[8] (the order of
-// the frames in the list does not matter).  A few microseconds; the sorted
-// order is what it buys (k_agrid_random).
+// exclusive scan of kScanCells counts of a frame by one CTA of 1024 threads
+// (grid x: the frame's pieces, grid y: frames from frame0 on), from a base that
+// the CTA takes off counters[8] (the order of the pieces and frames in the list
+// does not matter).  A few microseconds; the sorted order is what it buys
+// (k_agrid_random).  A sparse box of 373,000 fine cells: 9 us, 311 with one CTA
+// for all of the frame's cells.
+constexpr int kScanCells = 8192;
+
 __device__ __forceinline__ void k_slot_scan_body(const uint3 blockIdx, const dim3 gridDim, const Bufs &B, int frame0) {
     __shared__ int wsum[32];
     __shared__ int s_base;
-    const int f = frame0 + blockIdx.x;
+    const int f = frame0 + blockIdx.y;
     if (!B.FS[f].agrid) return;  // no slot of the frame was counted
-    int *c = B.scount + (int64_t)blockIdx.x * B.gfs;
-    const int n = B.G[f].ncell * B.agk * B.agk * B.agk;
+    const int64_t first = (int64_t)blockIdx.x * kScanCells;
+    const int n = (int)min((int64_t)kScanCells, (int64_t)B.G[f].ncell * B.agk * B.agk * B.agk - first);
+    if (n <= 0) return;
+    int *c = B.scount + (int64_t)blockIdx.y * B.gfs + first;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const int per = (n + 1023) / 1024;
     const int lo = min(n, t * per), hi = min(n, lo + per);

@@ -1434,7 +1434,9 @@ void atoms_chain(cm_handle *h, const Chunk &c, const DevSys &S, const Bufs &B, c
             // slots that can reach the solute, their placement on full warps,
             // then (candidate grid) their queries in fine-cell order
             em.kernel(MK_SLOT_FILTER, dim3(grid_for(mv, 128), ny), 0, CM_K_RANDOM, args(nullptr, 0, 0, c.smp0 + s0, f0));
-            if (agrid) em.kernel(MK_SLOT_SCAN, dim3(f1 - f0 + 1), 0, CM_K_RANDOM, args(nullptr, 0, 0, f0, 0));
+            if (agrid)
+                em.kernel(MK_SLOT_SCAN, dim3(grid_for((int64_t)c.ncell_max * h->agk * h->agk * h->agk, kScanCells), f1 - f0 + 1), 0,
+                          CM_K_RANDOM, args(nullptr, 0, 0, f0, 0));
             em.kernel(MK_ATOMS_PLACE, dim3((unsigned)std::min<int64_t>(grid_for((int64_t)ny * mv, 128), (int64_t)sms * 16)),
                       0, CM_K_RANDOM, args(nullptr, 0, 0, c.smp0 + s0, f0));
             if (agrid) {
